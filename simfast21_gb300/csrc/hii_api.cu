@@ -111,6 +111,8 @@ struct sf21_hii_ctx {
     cudaStream_t st;
   } gkey = {0, -1, nullptr, nullptr, nullptr, nullptr};
   PipeMaps pmaps;
+  const PairOps* pair = nullptr;  // passes over pairs of radii, when the context may use them
+  float2* d_twp = nullptr;        // plain twiddle table of the pair passes (powers of two)
   int* d_err = nullptr;
   int* d_ctl = nullptr;     // work-queue control block of pipeline 8
   unsigned int* d_rc32 = nullptr;  // pipeline 8: 32-bit first-hit box (atomicMin), folded into d_rc per set
@@ -196,7 +198,7 @@ static void span(sf21_hii_ctx* c, int kind, int a, int b) {
 static std::string g_create_err;
 
 // ---- autotuner cache --------------------------------------------------------
-// One JSON object per line, {"key": "<device>|N=<N>|K=<K>", "ms": [t1, ..., t7]}
+// One JSON object per line, {"key": "<device> rev <kernels>|N=<N>|K=<K>", "ms": [t1, ..., t7]}
 // (milliseconds of one batch per radius pipeline, 0 = not available), in
 // $SF21_TUNE_CACHE, else $XDG_CACHE_HOME/simfast21_gb300/tune.jsonl, else
 // ~/.cache/simfast21_gb300/tune.jsonl.  SF21_RETUNE=1 ignores the cache (and
@@ -210,11 +212,15 @@ static std::string tune_cache_path() {
   return dir + "/simfast21_gb300/tune.jsonl";
 }
 
+// Revision of the pipelines' kernels: timings stored for other kernels are
+// not reused.
+constexpr int kTuneRev = 2;
+
 static std::string tune_key(int device, long N, int K) {
   cudaDeviceProp pr;
   char b[512];
   if (cudaGetDeviceProperties(&pr, device) != cudaSuccess) return "";
-  snprintf(b, sizeof b, "%s sm_%d%d x%d|N=%ld|K=%d", pr.name, pr.major, pr.minor, pr.multiProcessorCount, N, K);
+  snprintf(b, sizeof b, "%s sm_%d%d x%d rev %d|N=%ld|K=%d", pr.name, pr.major, pr.minor, pr.multiProcessorCount, kTuneRev, N, K);
   for (char* q = b; *q; ++q)
     if (*q == '"' || *q == '\\') *q = '_';
   return b;
@@ -322,7 +328,7 @@ static void free_ctx(sf21_hii_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   void* ptrs[] = {c->d_delta, c->d_src, c->d_rec0, c->d_fres, c->d_partials, c->d_alpha,
-                  c->d_xhii, c->d_spec, c->d_tw, c->d_rc, c->d_mask, c->d_flag, c->d_box2,
+                  c->d_xhii, c->d_spec, c->d_tw, c->d_twp, c->d_rc, c->d_mask, c->d_flag, c->d_box2,
                   c->d_C, c->d_A, c->d_acc, c->d_zpart, c->d_g, c->d_gd, c->d_gs, c->d_halos, c->d_fine,
                   c->d_hscratch, c->d_chain, c->d_om, c->d_xhii2, c->d_pk, c->d_pk_w, c->d_pk_part,
                   c->d_pk_cnt, c->d_t21, c->d_t21_part};
@@ -375,6 +381,15 @@ static int prologue_args(sf21_hii_ctx* c, double z, int kind, PrologueArgs* pa) 
   pa->pf_resid = prod_fast_prepare(resid, 3);
   pa->pf_src = prod_fast_prepare(pa->src_mul, pa->n_src_mul);
   return SF21_OK;
+}
+
+// The passes over radius pairs read slot K of a batch with an odd number K of
+// radii: the last radius again, with the next work box.
+static void pad_pair(const sf21_hii_ctx* c, Batch& bt) {
+  if ((bt.K & 1) && bt.K < (int)c->d_work.size()) {
+    bt.r[bt.K] = bt.r[bt.K - 1];
+    bt.r[bt.K].work = c->d_work[bt.K];
+  }
 }
 
 static int enqueue_batch(sf21_hii_ctx* c, const Batch& bt, cudaStream_t st);
@@ -462,9 +477,18 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
   CREATE_CUDA(dev_malloc(&c->d_xhii, box_f));
   CREATE_CUDA(dev_malloc(&c->d_spec, box_c));
   CREATE_CUDA(dev_malloc(&c->d_rc, c->n3));
-  c->d_work.assign(K, nullptr);
-  CREATE_CUDA(dev_malloc(&c->d_work_base, box_c * K));
-  for (int k = 0; k < K; ++k) c->d_work[k] = c->d_work_base + (size_t)k * c->n3;
+  // passes over pairs of radii (pipeline 5, and the one of the sides that are
+  // not powers of two): an even number of boxes.  Sides that are not powers
+  // of two take one radius at a time when only one box is asked for.
+  const PairOps* po = pair_ops((int)N);
+  if (c->gen ? (po && K > 1) : (cfg->path == 0 || cfg->path == 5)) {
+    c->pair = po;
+    CREATE_CUDA(po->setup());
+  }
+  const int Kw = c->pair ? K + (K & 1) : K;
+  c->d_work.assign(Kw, nullptr);
+  CREATE_CUDA(dev_malloc(&c->d_work_base, box_c * Kw));
+  for (int k = 0; k < Kw; ++k) c->d_work[k] = c->d_work_base + (size_t)k * c->n3;
   CREATE_CUDA(dev_malloc(&c->d_err, sizeof(int)));
   CREATE_CUDA(cudaMemset(c->d_err, 0, sizeof(int)));
   CREATE_CUDA(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device));
@@ -486,6 +510,14 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
   }
   CREATE_CUDA(dev_malloc(&c->d_tw, sizeof(float2) * N));
   CREATE_CUDA(cudaMemcpy(c->d_tw, tw.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
+  if (c->pair && !c->gen) {  // the plain table as well
+    for (long t = 0; t < N; ++t) {
+      const double ang = -2.0 * kPI * t / N;
+      tw[t] = make_float2((float)cos(ang), (float)sin(ang));
+    }
+    CREATE_CUDA(dev_malloc(&c->d_twp, sizeof(float2) * N));
+    CREATE_CUDA(cudaMemcpy(c->d_twp, tw.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
+  }
   for (SetInfo& s : c->sets) {
     CREATE_CUDA(dev_malloc(&s.d_nmax, sizeof(int) * s.nmax.size()));
     CREATE_CUDA(cudaMemcpy(s.d_nmax, s.nmax.data(), sizeof(int) * s.nmax.size(), cudaMemcpyHostToDevice));
@@ -553,6 +585,7 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
           bt.r[k].ridx = k;
           bt.r[k].work = c->d_work[k];
         }
+        pad_pair(c, bt);
         for (int p = 1; p <= NPATH; ++p) {
           if (!available(p)) continue;
           c->path = p;
@@ -626,6 +659,22 @@ extern "C" int sf21_hii_radii(const sf21_hii_ctx* ctx, int set, double* R, int c
   if (n_fft) *n_fft = s.n_fft;
   return (int)s.R.size();
 }
+
+namespace sf21 {
+const PairOps* pair_ops_a(int);
+const PairOps* pair_ops_b(int);
+const PairOps* pair_ops_c(int);
+const PairOps* pair_ops_d(int);
+const PairOps* pair_ops_e(int);
+const PairOps* pair_ops_f(int);
+const PairOps* pair_ops_g(int);
+const PairOps* pair_ops_h(int);
+const PairOps* pair_ops(int N) {
+  for (auto f : {pair_ops_a, pair_ops_b, pair_ops_c, pair_ops_d, pair_ops_e, pair_ops_f, pair_ops_g, pair_ops_h})
+    if (const PairOps* p = f(N)) return p;
+  return nullptr;
+}
+}  // namespace sf21
 
 // ---- transform passes: register kernels (power-of-two sides) or shared-memory
 // kernels (other sides), same arguments ------------------------------------
@@ -719,14 +768,25 @@ static int enqueue_batch(sf21_hii_ctx* c, const Batch& bt, cudaStream_t st) {
     span(c, KD_FUSED, e1, e2);
     return SF21_OK;
   }
-  if (c->path >= 5) {  // column-block-major work boxes
+  if (c->pair && (c->gen || c->path == 5)) {  // three axis passes over pairs of radii
+    const float2* tw = c->gen ? c->d_tw : c->d_twp;
+    int e0 = mark(c, st);
+    CTX_CUDA(c, c->pair->rows_filter(c->d_spec, bt, tw, c->nsm, st));
+    int e1 = mark(c, st);
+    CTX_CUDA(c, c->pair->cols_b(bt, tw, c->nsm, st));
+    int e2 = mark(c, st);
+    CTX_CUDA(c, c->pair->cols_a_test(bt, c->d_rc, c->d_alpha, tw, c->nsm, st));
+    int e3 = mark(c, st);
+    span(c, KD_IROWS, e0, e1);
+    span(c, KD_ICB, e1, e2);
+    span(c, KD_ICA, e2, e3);
+    return SF21_OK;
+  }
+  if (c->path >= 6) {  // column-block-major work boxes, TMA-pipelined passes
     int e0 = mark(c, st);
     CTX_CUDA(c, launch_rows_filter_cb(N, c->d_spec, bt, c->d_tw, st));
     int e1 = mark(c, st);
-    if (c->path == 5)
-      CTX_CUDA(c, launch_cols_b_cb(N, bt, c->d_tw, st));
-    else
-      CTX_CUDA(c, launch_pipe(N, 0, 1, c->pmaps, bt, c->d_work_base, c->d_rc, c->d_alpha, c->d_tw, c->d_err,
+    CTX_CUDA(c, launch_pipe(N, 0, 1, c->pmaps, bt, c->d_work_base, c->d_rc, c->d_alpha, c->d_tw, c->d_err,
                               c->nsm, st, c->wait_limit));
     int e2 = mark(c, st);
     if (c->path == 7)
@@ -790,6 +850,7 @@ static int enqueue_radii(sf21_hii_ctx* c, int set, cudaStream_t st) {
       bt.r[k].ridx = k0 + k;
       bt.r[k].work = c->d_work[k];
     }
+    pad_pair(c, bt);
     if ((rc = enqueue_batch(c, bt, st))) return rc;
   }
   if (c->path == 8) CTX_CUDA(c, launch_rc32_to_rc(c->n3, c->d_rc32, c->d_rc, st));

@@ -1,0 +1,340 @@
+// Inverse transform of a batch of radii, two radii at a time: the kernels of
+// one box side (instantiated by the kernels_pair_*.cu units).
+//
+// The work boxes of a batch are private, so a pair of radii shares a box of
+// 16-byte values {rec_2p, rec_2p+1, ion_2p, ion_2p+1}, column-block major with
+// blocks of 8 columns:
+//     index(a, b, c) = ((c / 8) N + a) N + b) 8 + c mod 8,
+// one slab of 8 N^2 values per column block: a b-axis tile (fixed a, one
+// block) is one contiguous run, an a-axis tile (fixed b) reads 128-byte runs
+// inside one slab.  A batch with an odd number of radii carries its last
+// radius twice (the centre test of a radius is idempotent).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "pair_line.cuh"
+#include "sf21_kernels.h"
+
+namespace sf21 {
+
+__host__ __device__ constexpr int pair_min(int a, int b) { return a < b ? a : b; }
+__host__ __device__ constexpr int pair_max(int a, int b) { return a > b ? a : b; }
+
+// Column tiles: 8 columns of one line set, small boxes several tiles per CTA.
+// REGS: registers per thread that the occupancy is planned for.
+template <class L, int REGS>
+struct PairCol {
+  static constexpr int N = L::N;
+  static constexpr int LT = 8 * L::T;
+  static constexpr int TPC = LT >= 128 ? 1 : (N * (N / 8)) % (128 / LT) == 0 ? 128 / LT : 1;
+  static constexpr int THREADS = LT * TPC;
+  static constexpr int NTILES = N * (N / 8);
+  static constexpr size_t SMEM = (size_t)TPC * N * 8 * sizeof(cpair) + L::TW * sizeof(float2);
+  static constexpr int PER_SM = pair_max(1, pair_min(pair_min(32, 65536 / ((THREADS + 31) / 32 * 32 * REGS)),
+                                                     (int)(230000 / (SMEM + 1024))));
+};
+
+// Rows: RW rows per CTA.
+template <class L, int RW_, int REGS>
+struct PairRow {
+  static constexpr int N = L::N;
+  static constexpr int RW = RW_;
+  static constexpr int THREADS = RW * L::T;
+  static constexpr int NW = (N / 2 + L::T) / L::T;  // window values per thread
+  static constexpr int WS = (N / 2 + 2) / 2 * 2;    // float2 of a row's windows
+  static constexpr size_t SMEM =
+      (size_t)RW * (L::XR * sizeof(cpair) + WS * sizeof(float2)) + L::TW * sizeof(float2);
+  static constexpr int PER_SM = pair_max(1, pair_min(pair_min(32, 65536 / ((THREADS + 31) / 32 * 32 * REGS)),
+                                                     (int)(230000 / (SMEM + 1024))));
+  static_assert((N * N) % RW == 0, "rows per CTA");
+};
+
+// ---- c axis: the top-hat filter of the batch's radii, inverse transform -------
+// (get_HIIbubbles.c:305-322.)  Persistent: a CTA takes row groups blockIdx.x,
+// blockIdx.x + gridDim.x, ...; the next group's spectrum rows are asked into
+// L2 while the current one is transformed.  c and N - c share |k|, so per pair
+// the row's threads evaluate the N/2 + 1 distinct windows once into shared
+// memory.
+template <class L, int RW, int REGS>
+__global__ void __launch_bounds__(PairRow<L, RW, REGS>::THREADS, PairRow<L, RW, REGS>::PER_SM)
+k_pair_rows_filter(const float2* __restrict__ spec, Batch bt, const float2* __restrict__ plain) {
+  using R = PairRow<L, RW, REGS>;
+  constexpr int N = L::N;
+  extern __shared__ __align__(16) unsigned char psm[];
+  cpair* exs = reinterpret_cast<cpair*>(psm);
+  float2* ws = reinterpret_cast<float2*>(exs + RW * L::XR);
+  float2* tw = ws + RW * R::WS;
+  constexpr int NG = N * N / RW;  // row groups
+  const int row = threadIdx.x / L::T, t = threadIdx.x % L::T;
+  cpair* ex = exs + row * L::XR;
+  float2* wrow = ws + row * R::WS;
+  auto sync = [] {
+    if constexpr (R::THREADS <= 32) __syncwarp();
+    else __syncthreads();
+  };
+  auto load = [&](float2 (&z)[L::IT1][L::E1], int group) {
+    const float2* src = spec + ((long)group * RW + row) * N;
+#pragma unroll
+    for (int i = 0; i < L::IT1; ++i) {
+      const int q = t + i * L::T;
+      if (L::Q1 % L::T == 0 || q < L::Q1) {
+#pragma unroll
+        for (int m = 0; m < L::E1; ++m) z[i][m] = __ldg(src + q + m * L::Q1);
+      }
+    }
+  };
+  pair_tw_load<L>(tw, plain);
+  __syncthreads();
+  for (int group = blockIdx.x; group < NG; group += gridDim.x) {
+    const int rid = group * RW + row;
+    float kmag[R::NW];
+    {
+      const int a = rid / N, b = rid % N;
+      const int ka = kfreq(a, N), kb = kfreq(b, N);
+      const int kab = ka * ka + kb * kb;
+#pragma unroll
+      for (int i = 0; i < R::NW; ++i) {
+        const int kc = t + i * L::T;
+        kmag[i] = sqrtf((float)(kab + kc * kc));
+      }
+    }
+    float2 z[L::IT1][L::E1];
+    load(z, group);
+    if (group + gridDim.x < NG)  // the next group's rows on their way into L2
+      for (int i = threadIdx.x; i < RW * N / 16; i += R::THREADS)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(spec + (long)(group + gridDim.x) * RW * N + 16 * i));
+    for (int k = 0; k < bt.K; k += 2) {
+      const float d0 = bt.r[k].dkR, d1 = bt.r[k + 1].dkR;
+#pragma unroll
+      for (int i = 0; i < R::NW; ++i) {
+        const int kc = t + i * L::T;
+        if (kc <= N / 2) wrow[kc] = make_float2(w_tophat(d0 * kmag[i]), w_tophat(d1 * kmag[i]));
+      }
+      sync();  // the windows are in; the previous pair's exchange has been read
+      cpair v[L::IT1][L::E1];
+#pragma unroll
+      for (int i = 0; i < L::IT1; ++i) {
+        const int q = t + i * L::T;
+        if (L::Q1 % L::T == 0 || q < L::Q1) {
+#pragma unroll
+          for (int m = 0; m < L::E1; ++m) {
+            const int c = q + m * L::Q1;
+            const float2 x = z[i][m], w = wrow[c <= N / 2 ? c : N - c];
+            // scalar products: a packed product that feeds a packed addition
+            // was seen to be fused with it, which loses the scalar bits
+            v[i][m].re = make_float2(__fmul_rn(x.x, w.x), __fmul_rn(x.x, w.y));
+            v[i][m].im = make_float2(__fmul_rn(x.y, w.x), __fmul_rn(x.y, w.y));
+          }
+        }
+      }
+      cpair* box = reinterpret_cast<cpair*>(bt.r[k].work) + (long)rid * 8;
+      pair_line<L, true, 1>(v, ex, tw, t, sync, [&](int q, int m, int, const cpair& u) {
+        if constexpr (L::QL % 8 == 0) {
+          st_pair(box + (long)(q / 8) * N * N * 8 + q % 8 + (long)m * (L::QL / 8) * N * N * 8, u);
+        } else {
+          const int c = q + m * L::QL;
+          st_pair(box + (long)(c / 8) * N * N * 8 + c % 8, u);
+        }
+      });
+    }
+  }
+}
+
+// ---- strided axes ---------------------------------------------------------------
+// EPI 0: b axis, in place.  EPI 1: a axis, then the centre test and the
+// first-hit update (get_HIIbubbles.c:335-352; is_centre on both lanes).
+// One CTA per tile (group); no prefetch into registers: several CTAs per SM
+// overlap one tile's loads with another's transform, and the next pair's
+// lines are asked into L2 a pair ahead.
+template <class L, int EPI, int REGS>
+__global__ void __launch_bounds__(PairCol<L, REGS>::THREADS, PairCol<L, REGS>::PER_SM)
+k_pair_cols(Batch bt, uint8_t* __restrict__ rc, const float* __restrict__ alpha_ptr,
+            const float2* __restrict__ plain, int ahead) {
+  using C = PairCol<L, REGS>;
+  constexpr int N = L::N;
+  extern __shared__ __align__(16) unsigned char psm[];
+  cpair* exs = reinterpret_cast<cpair*>(psm);
+  float2* tw = reinterpret_cast<float2*>(exs + C::TPC * N * 8);
+  pair_tw_load<L>(tw, plain);
+  const int sub = threadIdx.x / C::LT;
+  const int col = threadIdx.x % 8;
+  const int t = (threadIdx.x % C::LT) / 8;
+  const int tile = blockIdx.x * C::TPC + sub;
+  cpair* ex = exs + sub * N * 8 + col;
+  constexpr long RS = EPI == 1 ? (long)N * 8 : 8;  // from one element of a line to the next
+  const long base = (EPI == 1 ? ((long)(tile / N) * N * N + tile % N) * 8 : (long)tile * N * 8) + col;
+  float alpha = 0.0f;
+  if (EPI == 1) alpha = *alpha_ptr;
+  auto sync = [] { __syncthreads(); };
+  // EPI 1: bit 8 (m & 3) + k of hit[m / 4]: output m is a centre at radius k of
+  // the batch (radius indices increase with k: the lowest bit is the first hit)
+  constexpr int HW = (L::EL + 3) / 4;
+  uint32_t hit[EPI == 1 ? L::ITL : 1][HW];
+#pragma unroll
+  for (int i = 0; i < (EPI == 1 ? L::ITL : 1); ++i)
+#pragma unroll
+    for (int h = 0; h < HW; ++h) hit[i][h] = 0u;
+  for (int k = 0; k < bt.K; k += 2) {
+    cpair* box = reinterpret_cast<cpair*>(bt.r[k].work) + base;
+    cpair v[L::IT1][L::E1];
+#pragma unroll
+    for (int i = 0; i < L::IT1; ++i) {
+      const int q = t + i * L::T;
+      if (L::Q1 % L::T == 0 || q < L::Q1) {
+        const cpair* src = box + q * RS;
+#pragma unroll
+        for (int m = 0; m < L::E1; ++m) v[i][m] = ld_pair(src + m * L::Q1 * RS);
+      }
+    }
+    if (ahead > 0) {  // the next pair's lines on their way into L2 (the last pair: those of a tile that comes later)
+      const bool more = k + 2 < bt.K;
+      const int ntile = tile + (more ? 0 : ahead * C::TPC);
+      if (ntile < C::NTILES) {
+        const cpair* nx = reinterpret_cast<const cpair*>(bt.r[more ? k + 2 : 0].work) +
+                          (EPI == 1 ? ((long)(ntile / N) * N * N + ntile % N) * 8 : (long)ntile * N * 8);
+        for (int r = threadIdx.x % C::LT; r < N; r += C::LT)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + r * RS));
+      }
+    }
+    __syncthreads();  // the previous pair's exchange has been read (k = 0: twiddles)
+    const float2 al2 = dup2(alpha), zm2 = dup2(bt.zmul);
+    const uint32_t bit = 1u << k;
+    pair_line<L, true, 8>(v, ex, tw, t, sync, [&](int q, int m, int i, const cpair& u) {
+      if constexpr (EPI == 0) {
+        st_pair(box + (q + m * L::QL) * RS, u);
+      } else {
+        const float2 y = mul2(u.im, zm2), x = mul2(u.re, al2);
+        if (u.im.x > 0.0f && y.x >= x.x) hit[i][m >> 2] |= bit << (8 * (m & 3));
+        if (u.im.y > 0.0f && y.y >= x.y) hit[i][m >> 2] |= bit << (8 * (m & 3) + 1);
+      }
+    });
+  }
+  if (EPI == 1 && alpha > 0.0f) {  // alpha <= 0: no source anywhere, no centre
+    const int b = tile % N;
+    const int c = (tile / N) * 8 + col;
+#pragma unroll
+    for (int i = 0; i < L::ITL; ++i) {
+      const int q = t + i * L::T;
+      if (L::QL % L::T == 0 || q < L::QL) {
+#pragma unroll
+        for (int m = 0; m < L::EL; ++m) {
+          const uint32_t byte = (hit[i][m >> 2] >> (8 * (m & 3))) & 0xFFu;
+          if (byte) {
+            const uint32_t h = (uint32_t)bt.r[__ffs(byte) - 1].ridx;
+            const long idx = ((long)(q + m * L::QL) * N + b) * N + c;
+            if (h < rc[idx]) rc[idx] = (uint8_t)h;
+          }
+        }
+      }
+    }
+  }
+}
+
+// ---- the lines of each side ----------------------------------------------------------
+// Column tiles: threads per line, codes, planned registers.  Rows: threads per
+// line, rows per CTA, planned registers, codes.  Chosen by timing candidates
+// of each kind on the GPU (8 radii; SM clocks per voxel and radius, where
+// DRAM's copy rate allows 0.42 / 0.74 / 0.37 for the filter / ky / kx pass):
+// tiles want few exchanges as long as two or more CTAs fit an SM (two groups at
+// 256: kx 0.40, three 0.47; at 512 0.53 and 0.53, but ky 0.86 and 0.74), rows
+// want many threads (512: three groups 0.56, two 0.80), and threads per line
+// that fill whole warps (400: 40 threads 0.58, 50 threads 0.76).  Sides whose
+// radices have no such cut (720, 1000, 1080, 1152, 1200, 1280) stay with the
+// shared-memory lines of kernels_gen.cu; 600 has transforms of its own.
+template <int N> struct PairSide;
+#define SF21_SIDE(N_, CT, CREGS, RT, RW_, RREGS, COLS, ROWS)          \
+  template <> struct PairSide<N_> {                                  \
+    using Col = PairLine<N_, CT, SF21_CODES COLS>;                   \
+    using Row = PairLine<N_, RT, SF21_CODES ROWS>;                   \
+    static constexpr int CR = CREGS, RW = RW_, RR = RREGS;           \
+  };
+#define SF21_CODES(...) __VA_ARGS__
+SF21_SIDE(16, 2, 64, 2, 16, 96, (8, CUT, 2), (8, CUT, 2))
+SF21_SIDE(24, 8, 64, 8, 8, 96, (3, CUT, 8), (3, CUT, 8))
+SF21_SIDE(32, 4, 64, 4, 16, 96, (8, CUT, 4), (8, CUT, 4))
+SF21_SIDE(40, 8, 80, 8, 8, 96, (5, CUT, 8), (5, CUT, 8))
+SF21_SIDE(48, 8, 80, 8, 8, 96, (3, S8A2, CUT, S8B4, 2), (3, S8A2, CUT, S8B4, 2))
+SF21_SIDE(64, 8, 64, 8, 8, 96, (8, CUT, 8), (8, CUT, 8))
+SF21_SIDE(72, 9, 80, 9, 8, 112, (3, 3, CUT, 8), (3, 3, CUT, 8))
+SF21_SIDE(80, 10, 96, 10, 8, 112, (5, S8A2, CUT, S8B4, 2), (5, S8A2, CUT, S8B4, 2))
+SF21_SIDE(96, 12, 96, 12, 8, 128, (3, S8A4, CUT, S8B2, 4), (3, S8A4, CUT, S8B2, 4))
+SF21_SIDE(120, 16, 128, 16, 4, 168, (5, 3, CUT, 8), (5, 3, CUT, 8))
+SF21_SIDE(128, 16, 64, 16, 4, 128, (8, CUT, 8, CUT, 2), (8, CUT, 8, CUT, 2))
+SF21_SIDE(144, 16, 112, 16, 4, 128, (3, 3, CUT, 8, 2), (3, 3, CUT, 8, 2))
+SF21_SIDE(160, 16, 112, 16, 4, 128, (5, S8A2, CUT, S8B4, 4), (5, S8A2, CUT, S8B4, 4))
+SF21_SIDE(192, 16, 128, 16, 4, 168, (3, S8A4, CUT, S8B2, 8), (3, S8A4, CUT, S8B2, 8))
+SF21_SIDE(200, 40, 64, 40, 4, 64, (5, CUT, 5, CUT, 8), (5, CUT, 5, CUT, 8))
+SF21_SIDE(216, 24, 128, 24, 4, 168, (3, 3, CUT, 3, 8), (3, 3, CUT, 3, 8))
+SF21_SIDE(240, 16, 128, 16, 2, 168, (5, 3, CUT, 8, 2), (5, 3, CUT, 8, 2))
+SF21_SIDE(256, 16, 128, 32, 2, 96, (8, S8A2, CUT, S8B4, 4), (8, CUT, 8, CUT, 4))
+SF21_SIDE(288, 32, 64, 32, 2, 80, (3, 3, CUT, 8, CUT, 4), (3, 3, CUT, 8, CUT, 4))
+SF21_SIDE(320, 40, 80, 64, 1, 64, (5, CUT, 8, CUT, 8), (5, CUT, 8, CUT, 8))
+SF21_SIDE(360, 24, 128, 48, 2, 128, (5, 3, CUT, 3, 8), (5, CUT, 3, 3, CUT, 8))
+SF21_SIDE(384, 24, 128, 24, 4, 168, (3, 8, CUT, 8, 2), (3, 8, CUT, 8, 2))
+SF21_SIDE(400, 40, 80, 40, 4, 96, (5, CUT, 5, S8A2, CUT, S8B4, 2), (5, CUT, 5, S8A2, CUT, S8B4, 2))
+SF21_SIDE(432, 48, 80, 48, 2, 80, (3, 3, CUT, 3, S8A2, CUT, S8B4, 2), (3, 3, CUT, 3, S8A2, CUT, S8B4, 2))
+SF21_SIDE(480, 32, 128, 64, 1, 128, (5, 3, CUT, 8, 4), (5, 3, CUT, 8, CUT, 4))
+SF21_SIDE(512, 64, 64, 64, 1, 96, (8, CUT, 8, CUT, 8), (8, CUT, 8, CUT, 8))
+SF21_SIDE(576, 64, 64, 64, 1, 80, (3, 3, CUT, 8, CUT, 8), (3, 3, CUT, 8, CUT, 8))
+SF21_SIDE(640, 64, 128, 64, 1, 128, (5, CUT, 8, CUT, 8, 2), (5, CUT, 8, CUT, 8, 2))
+SF21_SIDE(648, 48, 80, 81, 1, 96, (3, 3, CUT, 3, 3, CUT, 8), (3, 3, CUT, 3, 3, CUT, 8))
+SF21_SIDE(768, 64, 128, 64, 1, 128, (3, S8A4, CUT, S8B2, 8, CUT, 4), (3, S8A4, CUT, S8B2, 8, CUT, 4))
+SF21_SIDE(800, 80, 96, 80, 2, 128, (5, CUT, 5, S8A2, CUT, S8B4, 4), (5, CUT, 5, S8A2, CUT, S8B4, 4))
+SF21_SIDE(864, 48, 128, 108, 1, 128, (3, 3, CUT, 3, S8A4, CUT, S8B2, 4), (3, 3, CUT, 3, S8A4, CUT, S8B2, 4))
+SF21_SIDE(960, 64, 128, 64, 1, 128, (5, 3, CUT, 8, CUT, 8), (5, 3, CUT, 8, CUT, 8))
+SF21_SIDE(1024, 64, 128, 128, 1, 128, (8, CUT, 8, CUT, 8, 2), (8, CUT, 8, CUT, 8, 2))
+#undef SF21_CODES
+#undef SF21_SIDE
+
+// ---- host side: the launches of one side ------------------------------------------
+template <class L, int RW, int REGS>
+cudaError_t pair_rows_setup() {
+  return cudaFuncSetAttribute(k_pair_rows_filter<L, RW, REGS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)PairRow<L, RW, REGS>::SMEM);
+}
+template <class L, int RW, int REGS>
+cudaError_t pair_rows_launch(const float2* spec, const Batch& bt, const float2* tw, int nsm, cudaStream_t st) {
+  using R = PairRow<L, RW, REGS>;
+  const int ng = L::N * L::N / RW, most = nsm * R::PER_SM;
+  k_pair_rows_filter<L, RW, REGS><<<pair_min(ng, most), R::THREADS, R::SMEM, st>>>(spec, bt, tw);
+  return cudaGetLastError();
+}
+template <class L, int EPI, int REGS>
+cudaError_t pair_cols_setup() {
+  return cudaFuncSetAttribute(k_pair_cols<L, EPI, REGS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)PairCol<L, REGS>::SMEM);
+}
+template <class L, int EPI, int REGS, bool AHEAD>
+cudaError_t pair_cols_launch(const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw, int nsm,
+                             cudaStream_t st) {
+  using C = PairCol<L, REGS>;
+  k_pair_cols<L, EPI, REGS><<<C::NTILES / C::TPC, C::THREADS, C::SMEM, st>>>(bt, rc, alpha, tw,
+                                                                             AHEAD ? nsm * C::PER_SM : 0);
+  return cudaGetLastError();
+}
+
+template <int N>
+struct PairLaunch {
+  using S = PairSide<N>;
+  using Row = typename S::Row;
+  using Col = typename S::Col;
+  // the next pair's lines asked into L2 ahead: faster in the kx pass at every
+  // side, in the ky pass where an SM holds two CTAs (512: 0.74 against 0.78 clk),
+  // not at the small sides (240: 0.78 against 0.75)
+  static constexpr bool AHEAD_B = N >= 300;
+  static cudaError_t setup() {
+    cudaError_t e = pair_rows_setup<Row, S::RW, S::RR>();
+    if (!e) e = pair_cols_setup<Col, 0, S::CR>();
+    if (!e) e = pair_cols_setup<Col, 1, S::CR>();
+    return e;
+  }
+  static cudaError_t cols_b(const Batch& bt, const float2* tw, int nsm, cudaStream_t st) {
+    return pair_cols_launch<Col, 0, S::CR, AHEAD_B>(bt, nullptr, nullptr, tw, nsm, st);
+  }
+  static constexpr PairOps ops() {
+    return {setup, pair_rows_launch<Row, S::RW, S::RR>, cols_b, pair_cols_launch<Col, 1, S::CR, true>};
+  }
+};
+
+}  // namespace sf21

@@ -1,0 +1,23 @@
+// Radius-pair kernels (kernels_pair.cuh) of the box sides below.
+#include "kernels_pair.cuh"
+
+namespace sf21 {
+
+const PairOps* pair_ops_a(int N) {
+  switch (N) {
+#define SF21_PAIR_SIDE(n)                                \
+  case n: {                                              \
+    static const PairOps ops = PairLaunch<n>::ops();     \
+    return &ops;                                         \
+  }
+    SF21_PAIR_SIDE(16)
+    SF21_PAIR_SIDE(32)
+    SF21_PAIR_SIDE(64)
+    SF21_PAIR_SIDE(128)
+    SF21_PAIR_SIDE(256)
+#undef SF21_PAIR_SIDE
+    default: return nullptr;
+  }
+}
+
+}  // namespace sf21

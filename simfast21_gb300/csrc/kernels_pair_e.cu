@@ -1,0 +1,22 @@
+// Radius-pair kernels (kernels_pair.cuh) of the box sides below.
+#include "kernels_pair.cuh"
+
+namespace sf21 {
+
+const PairOps* pair_ops_e(int N) {
+  switch (N) {
+#define SF21_PAIR_SIDE(n)                                \
+  case n: {                                              \
+    static const PairOps ops = PairLaunch<n>::ops();     \
+    return &ops;                                         \
+  }
+    SF21_PAIR_SIDE(320)
+    SF21_PAIR_SIDE(360)
+    SF21_PAIR_SIDE(384)
+    SF21_PAIR_SIDE(400)
+#undef SF21_PAIR_SIDE
+    default: return nullptr;
+  }
+}
+
+}  // namespace sf21

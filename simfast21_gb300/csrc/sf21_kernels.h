@@ -107,6 +107,19 @@ cudaError_t launch_cols_b_cb(int N, const Batch& bt, const float2* tw, cudaStrea
 cudaError_t launch_cols_a_test_cb(int N, const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw, int nsm,
                                   cudaStream_t st);
 
+// Radius pipeline over pairs of radii (kernels_pair.cuh): the c-axis filter
+// pass, the in-place b-axis pass, the a-axis pass + centre test, on boxes of
+// 16-byte pair values (r[k].work and r[k + 1].work consecutive; slot K holds
+// the last radius again when K is odd).  tw: the plain table exp(-2 pi i t / N).
+struct PairOps {  // the launches of one box side
+  cudaError_t (*setup)();
+  cudaError_t (*rows_filter)(const float2* spec, const Batch& bt, const float2* tw, int nsm, cudaStream_t st);
+  cudaError_t (*cols_b)(const Batch& bt, const float2* tw, int nsm, cudaStream_t st);
+  cudaError_t (*cols_a_test)(const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw, int nsm,
+                             cudaStream_t st);
+};
+const PairOps* pair_ops(int N);  // null: no pair kernels for this side
+
 // b- and a-axis passes of a batch in one persistent launch through L2
 // (kernels_fused.cu, radius pipeline 8; column-block-major work boxes).
 // ctl: fused_ctl_ints(N) ints of device memory (zeroed by the launch).
