@@ -217,14 +217,19 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, const float* __restrict__ alpha_
     for (int i = 0; i < L::ITL; ++i) {
       const int q = t + i * L::T;
       if (L::QL % L::T == 0 || q < L::QL) {
+        // all the reads first (independent), then the updates; the radius
+        // indices of a batch are consecutive
+        uint32_t old[L::EL];
 #pragma unroll
         for (int m = 0; m < L::EL; ++m) {
           const uint32_t byte = (hit[i][m >> 2] >> (8 * (m & 3))) & 0xFFu;
-          if (byte) {
-            const uint32_t h = (uint32_t)bt.r[__ffs(byte) - 1].ridx;
-            const long idx = ((long)(q + m * L::QL) * N + b) * N + c;
-            if (h < rc[idx]) rc[idx] = (uint8_t)h;
-          }
+          old[m] = byte ? rc[((long)(q + m * L::QL) * N + b) * N + c] : 0u;
+        }
+#pragma unroll
+        for (int m = 0; m < L::EL; ++m) {
+          const uint32_t byte = (hit[i][m >> 2] >> (8 * (m & 3))) & 0xFFu;
+          const uint32_t h = (uint32_t)(bt.r[0].ridx + __ffs(byte) - 1);
+          if (byte && h < old[m]) rc[((long)(q + m * L::QL) * N + b) * N + c] = (uint8_t)h;
         }
       }
     }
@@ -241,7 +246,7 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, const float* __restrict__ alpha_
 // want many threads (512: three groups 0.56, two 0.80), and threads per line
 // that fill whole warps (400: 40 threads 0.58, 50 threads 0.76).  Sides whose
 // radices have no such cut (720, 1000, 1080, 1152, 1200, 1280) stay with the
-// shared-memory lines of kernels_gen.cu; 600 has transforms of its own.
+// shared-memory lines of kernels_gen.cu; 600 follows kernels_gen600.cu.
 template <int N> struct PairSide;
 #define SF21_SIDE(N_, CT, CREGS, RT, RW_, RREGS, COLS, ROWS)          \
   template <> struct PairSide<N_> {                                  \
@@ -277,6 +282,7 @@ SF21_SIDE(432, 48, 80, 48, 2, 80, (3, 3, CUT, 3, S8A2, CUT, S8B4, 2), (3, 3, CUT
 SF21_SIDE(480, 32, 128, 64, 1, 128, (5, 3, CUT, 8, 4), (5, 3, CUT, 8, CUT, 4))
 SF21_SIDE(512, 64, 64, 64, 1, 96, (8, CUT, 8, CUT, 8), (8, CUT, 8, CUT, 8))
 SF21_SIDE(576, 64, 64, 64, 1, 80, (3, 3, CUT, 8, CUT, 8), (3, 3, CUT, 8, CUT, 8))
+SF21_SIDE(600, 24, 128, 60, 1, 128, (5, 5, CUT, 8, 3), (5, CUT, 5, S8A2, CUT, S8B4, 3))
 SF21_SIDE(640, 64, 128, 64, 1, 128, (5, CUT, 8, CUT, 8, 2), (5, CUT, 8, CUT, 8, 2))
 SF21_SIDE(648, 48, 80, 81, 1, 96, (3, 3, CUT, 3, 3, CUT, 8), (3, 3, CUT, 3, 3, CUT, 8))
 SF21_SIDE(768, 64, 128, 64, 1, 128, (3, S8A4, CUT, S8B2, 8, CUT, 4), (3, S8A4, CUT, S8B2, 8, CUT, 4))

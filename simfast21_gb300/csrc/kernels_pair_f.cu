@@ -13,6 +13,7 @@ const PairOps* pair_ops_f(int N) {
     SF21_PAIR_SIDE(432)
     SF21_PAIR_SIDE(480)
     SF21_PAIR_SIDE(576)
+    SF21_PAIR_SIDE(600)
 #undef SF21_PAIR_SIDE
     default: return nullptr;
   }

@@ -164,23 +164,28 @@ __device__ __forceinline__ void pdft8(cpair* v) {
 }
 
 // dft3 and dft5 of kernels_gen.cu with the fused multiply-adds that the
-// compiler forms there, written out.
-#ifndef SF21_D5B1
-#define SF21_D5B1 0
-#define SF21_D5B2 0
-#endif
-template <bool INV>
+// compiler forms there, written out; G600: those of kernels_gen600.cu, whose
+// source fixes other roundings (the products of dft3 are scalar, so that they
+// are not fused with the additions that they feed).
+template <bool INV, bool G600>
 __device__ __forceinline__ void pdft3(cpair& x0, cpair& x1, cpair& x2) {
   const float s = INV ? -0.86602540378443864676f : 0.86602540378443864676f;
   const float2 s2 = dup2(s), sn = dup2(-s), mh = dup2(-0.5f);
   const cpair t1 = padd(x1, x2), t2 = psub(x1, x2);
   const cpair m = {fma2(mh, t1.re, x0.re), fma2(mh, t1.im, x0.im)};
   x0 = padd(x0, t1);
-  x1 = {fma2(s2, t2.im, m.re), fma2(sn, t2.re, m.im)};
-  x2 = {fma2(sn, t2.im, m.re), fma2(s2, t2.re, m.im)};
+  if constexpr (G600) {
+    const cpair b = {make_float2(__fmul_rn(s, t2.re.x), __fmul_rn(s, t2.re.y)),
+                     make_float2(__fmul_rn(s, t2.im.x), __fmul_rn(s, t2.im.y))};
+    x1 = padd_mi<false>(m, b);  // the sign of the direction is in s
+    x2 = psub_mi<false>(m, b);
+  } else {
+    x1 = {fma2(s2, t2.im, m.re), fma2(sn, t2.re, m.im)};
+    x2 = {fma2(sn, t2.im, m.re), fma2(s2, t2.re, m.im)};
+  }
 }
 
-template <bool INV>
+template <bool INV, bool G600>
 __device__ __forceinline__ void pdft5(cpair& x0, cpair& x1, cpair& x2, cpair& x3, cpair& x4) {
   const float2 c1 = dup2(0.30901699437494742410f), c2 = dup2(-0.80901699437494742410f);
   const float f1 = INV ? -0.95105651629515357212f : 0.95105651629515357212f;
@@ -190,14 +195,13 @@ __device__ __forceinline__ void pdft5(cpair& x0, cpair& x1, cpair& x2, cpair& x3
   const cpair a1 = {fma2(c2, p2.re, fma2(c1, p1.re, x0.re)), fma2(c2, p2.im, fma2(c1, p1.im, x0.im))};
   const cpair a2 = {fma2(c1, p2.re, fma2(c2, p1.re, x0.re)), fma2(c1, p2.im, fma2(c2, p1.im, x0.im))};
   cpair b1, b2;
-  if (SF21_D5B1 == 0)
-    b1 = {fma2(s1, m1.re, mul2(s2, m2.re)), fma2(s1, m1.im, mul2(s2, m2.im))};
-  else
+  if constexpr (G600) {
     b1 = {fma2(s2, m2.re, mul2(s1, m1.re)), fma2(s2, m2.im, mul2(s1, m1.im))};
-  if (SF21_D5B2 == 0)
-    b2 = {fma2(s2, m1.re, mul2(s1n, m2.re)), fma2(s2, m1.im, mul2(s1n, m2.im))};
-  else
     b2 = {fma2(s1n, m2.re, mul2(s2, m1.re)), fma2(s1n, m2.im, mul2(s2, m1.im))};
+  } else {
+    b1 = {fma2(s1, m1.re, mul2(s2, m2.re)), fma2(s1, m1.im, mul2(s2, m2.im))};
+    b2 = {fma2(s2, m1.re, mul2(s1n, m2.re)), fma2(s2, m1.im, mul2(s1n, m2.im))};
+  }
   x0 = padd(x0, padd(p1, p2));
   x1 = padd_mi<false>(a1, b1);  // the sign of the direction is in s1, s2
   x4 = psub_mi<false>(a1, b1);
@@ -250,7 +254,7 @@ struct PairLine {
   static constexpr int EL = GROUPS == 3 ? E3 : E2;             // last group
   static constexpr int Q1 = N / E1, Q2 = N / E2, QL = N / EL;  // subsets of the groups
   static constexpr int IT1 = (Q1 + T - 1) / T, IT2 = (Q2 + T - 1) / T, ITL = (QL + T - 1) / T;
-  static constexpr int TW = N + 8 * cut_span();                // twiddle entries in shared memory
+  static constexpr int TW = N + (N == 600 ? 600 : 8 * cut_span());  // twiddle entries in shared memory
   // cpairs of a row's exchange: padded by one in eight when group 1 writes with an even stride
   static constexpr int XR = E1 % 2 == 0 ? N + N / 8 : N;
   static_assert(E1 * E2 * E3 == N, "the codes do not cover the line");
@@ -261,12 +265,20 @@ struct PairLine {
 // (consecutive k on consecutive banks; the stages' tables [Ns, Ns R) follow one
 // another).  A radix-8 stage that is cut has them for r = 0 too (ones), at
 // N + r Ns + k.
+// N = 600 follows kernels_gen600.cu, 600 = 25 x 24: radices 5, 5, 8, 3, where
+// the values that enter the radix-8 stage take the whole twiddle w^(n1 k) of
+// their position k + 25 n1 (at N + 25 n1 + k) and the radix-3 stage only
+// w24^(r (k / 25)).
 // plain: w^t = exp(-2 pi i t / N), t < N
 template <class L, int I = 0, int NS = 1>
 __device__ __forceinline__ void pair_tw_load(float2* st, const float2* __restrict__ plain) {
   if constexpr (I < L::n) {
     constexpr int N = L::N, C = L::code(I), R = stage_radix(C);
-    if constexpr (C == S8A2 || C == S8A4) {
+    if constexpr (N == 600 && NS == 25 && C != CUT) {
+      for (int i = threadIdx.x; i < 600; i += blockDim.x) st[N + i] = plain[(i % 25) * (i / 25)];
+    } else if constexpr (N == 600 && C == 3) {
+      for (int i = threadIdx.x; i < 400; i += blockDim.x) st[NS + i] = plain[25 * (1 + i / 200) * (i % 200 / 25)];
+    } else if constexpr (C == S8A2 || C == S8A4) {
       for (int i = threadIdx.x; i < 8 * NS; i += blockDim.x) st[N + i] = plain[(i % NS) * (i / NS) * (N / (8 * NS))];
     } else if constexpr (C != CUT && C < 10 && NS > 1) {
       for (int i = threadIdx.x; i < NS * (R - 1); i += blockDim.x)
@@ -304,7 +316,12 @@ __device__ __forceinline__ void pair_stages(cpair (&v)[E], const float2* tw, int
         cpair u[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) u[r] = v[ka + NSL * (mu + r * MU)];
-        if constexpr (C == S8A2 || C == S8A4) {
+        if constexpr (N == 600 && NS == 25) {
+          const int pos = (q / NS0) * NS0 * NSL + k0 + NS0 * ka + NSL * (N / E) * mu;
+          const float2* t = tw + N + (pos / 25) * 25 + k0 + NS0 * ka;
+#pragma unroll
+          for (int r = 0; r < R; ++r) u[r] = pcmul(u[r], twid<INV>(t, r * NSL * (N / E) * MU));
+        } else if constexpr (C == S8A2 || C == S8A4) {
           // index in the radix-8 stage: the position divided by N/8
           const int pos = (q / NS0) * NS0 * NSL + k0 + NS0 * ka + NSL * (N / E) * mu;
           const float2* t = tw + N + (pos / (N / 8)) * NS + k0 + NS0 * ka;
@@ -316,9 +333,9 @@ __device__ __forceinline__ void pair_stages(cpair (&v)[E], const float2* tw, int
           for (int r = 1; r < R; ++r) u[r] = pcmul(u[r], twid<INV>(t, (r - 1) * NS));
         }
         if constexpr (C == 8) pdft8<INV>(u);
-        if constexpr (C == 5) pdft5<INV>(u[0], u[1], u[2], u[3], u[4]);
+        if constexpr (C == 5) pdft5<INV, N == 600>(u[0], u[1], u[2], u[3], u[4]);
         if constexpr (C == 4 || C == S8A4) pdft4<INV>(u[0], u[1], u[2], u[3]);
-        if constexpr (C == 3) pdft3<INV>(u[0], u[1], u[2]);
+        if constexpr (C == 3) pdft3<INV, N == 600>(u[0], u[1], u[2]);
         if constexpr (C == 2 || C == S8A2) pdft2<INV>(u[0], u[1]);
         if constexpr (C == S8B4) {
           if (digit == 0) pdft4<INV>(u[0], u[1], u[2], u[3]);

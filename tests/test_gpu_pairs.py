@@ -10,7 +10,7 @@ from simfast21_gb300 import synth
 pytestmark = pytest.mark.gpu
 
 POW2 = [16, 32, 64, 128, 256]
-RAGGED = [24, 40, 48, 72, 80, 96, 120, 144, 160, 192, 200, 216, 240, 288, 320, 360, 384, 400, 432, 480, 576]
+RAGGED = [24, 40, 48, 72, 80, 96, 120, 144, 160, 192, 200, 216, 240, 288, 320, 360, 384, 400, 432, 480, 576, 600]
 
 
 @pytest.mark.parametrize("N", POW2 + RAGGED)
