@@ -392,6 +392,9 @@ static void pad_pair(const sf21_hii_ctx* c, Batch& bt) {
   }
 }
 
+// The plain twiddle table of the pair passes.
+static const float2* pair_tw(const sf21_hii_ctx* c) { return c->gen ? c->d_tw : c->d_twp; }
+
 static int enqueue_batch(sf21_hii_ctx* c, const Batch& bt, cudaStream_t st);
 static int check_device_flag(sf21_hii_ctx* c);
 
@@ -769,11 +772,11 @@ static int enqueue_batch(sf21_hii_ctx* c, const Batch& bt, cudaStream_t st) {
     return SF21_OK;
   }
   if (c->pair && (c->gen || c->path == 5)) {  // three axis passes over pairs of radii
-    const float2* tw = c->gen ? c->d_tw : c->d_twp;
+    const float2* tw = pair_tw(c);
     int e0 = mark(c, st);
     CTX_CUDA(c, c->pair->rows_filter(c->d_spec, bt, tw, c->nsm, st));
     int e1 = mark(c, st);
-    CTX_CUDA(c, c->pair->cols_b(bt, tw, c->nsm, st));
+    CTX_CUDA(c, c->pair->cols_b(bt, true, tw, c->nsm, st));
     int e2 = mark(c, st);
     CTX_CUDA(c, c->pair->cols_a_test(bt, c->d_rc, c->d_alpha, tw, c->nsm, st));
     int e3 = mark(c, st);
@@ -1244,7 +1247,14 @@ static int ensure_adj_buffers(sf21_hii_ctx* c) {
 // recompute the filtered fields of a batch up to (not including) the kx pass
 static int enqueue_recompute(sf21_hii_ctx* c, const Batch& bt, cudaStream_t st) {
   const int N = (int)c->N;
-  if (c->path == 2) {
+  if (c->pair) {
+    int e0 = mark(c, st);
+    CTX_CUDA(c, c->pair->rows_filter(c->d_spec, bt, pair_tw(c), c->nsm, st));
+    int e1 = mark(c, st);
+    CTX_CUDA(c, c->pair->cols_b(bt, true, pair_tw(c), c->nsm, st));
+    span(c, KD_IROWS, e0, e1);
+    span(c, KD_ICB, e1, mark(c, st));
+  } else if (c->path == 2) {
     int e0 = mark(c, st);
     CTX_CUDA(c, launch_plane_filter(N, c->d_spec, bt, c->d_tw, st));
     span(c, KD_PLANE, e0, mark(c, st));
@@ -1271,6 +1281,7 @@ static Batch make_batch(const sf21_hii_ctx* c, int set, int k0, int nr) {
     bt.r[k].ridx = k0 + k;
     bt.r[k].work = c->d_work[k];
   }
+  pad_pair(c, bt);
   return bt;
 }
 
@@ -1291,7 +1302,9 @@ extern "C" int sf21_hii_criterion_device(sf21_hii_ctx* c, double z, int kind, co
     Batch bt = make_batch(c, set, k0, nr);
     if ((rc = enqueue_recompute(c, bt, st))) return rc;
     int e0 = mark(c, st);
-    if (c->gen) {  // shared-memory transforms: whole a-axis pass, then the per-element rule
+    if (c->pair) {
+      CTX_CUDA(c, c->pair->cols_a_crit(bt, c->d_C, c->d_A, c->d_alpha, pair_tw(c), c->nsm, st));
+    } else if (c->gen) {  // shared-memory transforms: whole a-axis pass, then the per-element rule
       CTX_CUDA(c, x_cols(c, nullptr, bt, bt.K, 0, true, st));
       CTX_CUDA(c, launch_crit_elem(c->n3, bt, c->d_C, c->d_A, c->d_alpha, st));
     } else {
@@ -1320,7 +1333,7 @@ extern "C" int sf21_hii_vjp_device(sf21_hii_ctx* c, double z, int kind, const fl
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   const int N = (int)c->N;
   const long n3 = c->n3;
-  const int nzp = c->gen ? adj_elem_blocks() : adj_zpart_blocks(N);
+  const int nzp = c->pair ? c->pair->adj_blocks : c->gen ? adj_elem_blocks() : adj_zpart_blocks(N);
   if (!c->d_acc) CTX_CUDA(c, dev_malloc(&c->d_acc, sizeof(float2) * n3));
   if (!c->d_zpart) CTX_CUDA(c, dev_malloc(&c->d_zpart, sizeof(float) * nzp));
   // recompute the spectrum (the checkpoint holds only the argmax index)
@@ -1334,6 +1347,18 @@ extern "C" int sf21_hii_vjp_device(sf21_hii_ctx* c, double z, int kind, const fl
     Batch bt = make_batch(c, set, k0, nr);
     if ((rc = enqueue_recompute(c, bt, st))) return rc;
     int e0 = mark(c, st);
+    if (c->pair) {
+      if (bt.K & 1) bt.r[bt.K].ridx = -1;  // the slot that fills the last pair takes no voxel
+      CTX_CUDA(c, c->pair->cols_a_adj(bt, dC_dev, c->d_A, c->d_alpha, c->d_zpart, pair_tw(c), st));
+      int e1 = mark(c, st);
+      CTX_CUDA(c, c->pair->cols_b(bt, false, pair_tw(c), c->nsm, st));
+      int e2 = mark(c, st);
+      CTX_CUDA(c, c->pair->rows_adj(bt, c->d_acc, pair_tw(c), c->nsm, st));
+      span(c, KD_ADJA, e0, e1);
+      span(c, KD_ADJB, e1, e2);
+      span(c, KD_ADJR, e2, mark(c, st));
+      continue;
+    }
     if (c->gen) {  // a-axis inverse, cotangents, a-axis forward as whole-box passes
       CTX_CUDA(c, x_cols(c, nullptr, bt, bt.K, 0, true, st));
       CTX_CUDA(c, launch_adj_elem(n3, bt, dC_dev, c->d_A, c->d_alpha, c->d_zpart, st));

@@ -144,12 +144,14 @@ k_pair_rows_filter(const float2* __restrict__ spec, Batch bt, const float2* __re
 // ---- strided axes ---------------------------------------------------------------
 // EPI 0: b axis, in place.  EPI 1: a axis, then the centre test and the
 // first-hit update (get_HIIbubbles.c:335-352; is_centre on both lanes).
+// EPI 2: a axis, then the running maximum of ion_R / rec_R and its radius (the
+// rule of k_cols_a_crit, in the order of the radii).
 // One CTA per tile (group); no prefetch into registers: several CTAs per SM
 // overlap one tile's loads with another's transform, and the next pair's
 // lines are asked into L2 a pair ahead.
-template <class L, int EPI, int REGS>
+template <class L, bool INV, int EPI, int REGS>
 __global__ void __launch_bounds__(PairCol<L, REGS>::THREADS, PairCol<L, REGS>::PER_SM)
-k_pair_cols(Batch bt, uint8_t* __restrict__ rc, const float* __restrict__ alpha_ptr,
+k_pair_cols(Batch bt, uint8_t* __restrict__ rc, float* __restrict__ Cbuf, const float* __restrict__ alpha_ptr,
             const float2* __restrict__ plain, int ahead) {
   using C = PairCol<L, REGS>;
   constexpr int N = L::N;
@@ -162,19 +164,27 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, const float* __restrict__ alpha_
   const int t = (threadIdx.x % C::LT) / 8;
   const int tile = blockIdx.x * C::TPC + sub;
   cpair* ex = exs + sub * N * 8 + col;
-  constexpr long RS = EPI == 1 ? (long)N * 8 : 8;  // from one element of a line to the next
-  const long base = (EPI == 1 ? ((long)(tile / N) * N * N + tile % N) * 8 : (long)tile * N * 8) + col;
+  constexpr long RS = EPI >= 1 ? (long)N * 8 : 8;  // from one element of a line to the next
+  const long base = (EPI >= 1 ? ((long)(tile / N) * N * N + tile % N) * 8 : (long)tile * N * 8) + col;
   float alpha = 0.0f;
-  if (EPI == 1) alpha = *alpha_ptr;
+  if (EPI >= 1) alpha = *alpha_ptr;
   auto sync = [] { __syncthreads(); };
   // EPI 1: bit 8 (m & 3) + k of hit[m / 4]: output m is a centre at radius k of
   // the batch (radius indices increase with k: the lowest bit is the first hit)
   constexpr int HW = (L::EL + 3) / 4;
-  uint32_t hit[EPI == 1 ? L::ITL : 1][HW];
+  uint32_t hit[EPI >= 1 ? L::ITL : 1][HW];
 #pragma unroll
-  for (int i = 0; i < (EPI == 1 ? L::ITL : 1); ++i)
+  for (int i = 0; i < (EPI >= 1 ? L::ITL : 1); ++i)
 #pragma unroll
-    for (int h = 0; h < HW; ++h) hit[i][h] = 0u;
+    for (int h = 0; h < HW; ++h) hit[i][h] = EPI == 2 ? 0xFFFFFFFFu : 0u;
+  // EPI 2: the batch's best ratio of each output; byte m & 3 of hit[m / 4] is its radius index
+  float best[EPI == 2 ? L::ITL : 1][L::EL];
+#pragma unroll
+  for (int i = 0; i < (EPI == 2 ? L::ITL : 1); ++i)
+#pragma unroll
+    for (int m = 0; m < L::EL; ++m) best[i][m] = -INFINITY;
+  // no source anywhere (alpha < 0): ion_R is exactly zero
+  const float crit_zeta = alpha > 0.0f ? bt.zmul : 0.0f, crit_alpha = fabsf(alpha);
   for (int k = 0; k < bt.K; k += 2) {
     cpair* box = reinterpret_cast<cpair*>(bt.r[k].work) + base;
     cpair v[L::IT1][L::E1];
@@ -192,7 +202,7 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, const float* __restrict__ alpha_
       const int ntile = tile + (more ? 0 : ahead * C::TPC);
       if (ntile < C::NTILES) {
         const cpair* nx = reinterpret_cast<const cpair*>(bt.r[more ? k + 2 : 0].work) +
-                          (EPI == 1 ? ((long)(ntile / N) * N * N + ntile % N) * 8 : (long)ntile * N * 8);
+                          (EPI >= 1 ? ((long)(ntile / N) * N * N + ntile % N) * 8 : (long)ntile * N * 8);
         for (int r = threadIdx.x % C::LT; r < N; r += C::LT)
           asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + r * RS));
       }
@@ -200,15 +210,49 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, const float* __restrict__ alpha_
     __syncthreads();  // the previous pair's exchange has been read (k = 0: twiddles)
     const float2 al2 = dup2(alpha), zm2 = dup2(bt.zmul);
     const uint32_t bit = 1u << k;
-    pair_line<L, true, 8>(v, ex, tw, t, sync, [&](int q, int m, int i, const cpair& u) {
+    pair_line<L, INV, 8>(v, ex, tw, t, sync, [&](int q, int m, int i, const cpair& u) {
       if constexpr (EPI == 0) {
         st_pair(box + (q + m * L::QL) * RS, u);
+      } else if constexpr (EPI == 2) {
+#pragma unroll
+        for (int lane = 0; lane < 2; ++lane) {
+          const float den = (lane ? u.re.y : u.re.x) * crit_alpha;  // alpha * rec_R
+          if (den > 0.0f) {
+            const float ratio = __fdiv_rn((lane ? u.im.y : u.im.x) * crit_zeta, den);
+            if (ratio > best[i][m]) {
+              best[i][m] = ratio;
+              hit[i][m >> 2] = __byte_perm(hit[i][m >> 2], (uint32_t)bt.r[k + lane].ridx,
+                                           (0x3210u & ~(0xFu << (4 * (m & 3)))) | (4u << (4 * (m & 3))));
+            }
+          }
+        }
       } else {
         const float2 y = mul2(u.im, zm2), x = mul2(u.re, al2);
         if (u.im.x > 0.0f && y.x >= x.x) hit[i][m >> 2] |= bit << (8 * (m & 3));
         if (u.im.y > 0.0f && y.y >= x.y) hit[i][m >> 2] |= bit << (8 * (m & 3) + 1);
       }
     });
+  }
+  if constexpr (EPI == 2) {
+    const int b = tile % N;
+    const int c = (tile / N) * 8 + col;
+#pragma unroll
+    for (int i = 0; i < L::ITL; ++i) {
+      const int q = t + i * L::T;
+      if (L::QL % L::T == 0 || q < L::QL) {
+        float old[L::EL];
+#pragma unroll
+        for (int m = 0; m < L::EL; ++m) old[m] = Cbuf[((long)(q + m * L::QL) * N + b) * N + c];
+#pragma unroll
+        for (int m = 0; m < L::EL; ++m) {
+          if (best[i][m] > old[m]) {
+            const long idx = ((long)(q + m * L::QL) * N + b) * N + c;
+            Cbuf[idx] = best[i][m];
+            rc[idx] = (uint8_t)(hit[i][m >> 2] >> (8 * (m & 3)));
+          }
+        }
+      }
+    }
   }
   if (EPI == 1 && alpha > 0.0f) {  // alpha <= 0: no source anywhere, no centre
     const int b = tile % N;
@@ -230,6 +274,204 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, const float* __restrict__ alpha_
           const uint32_t byte = (hit[i][m >> 2] >> (8 * (m & 3))) & 0xFFu;
           const uint32_t h = (uint32_t)(bt.r[0].ridx + __ffs(byte) - 1);
           if (byte && h < old[m]) rc[((long)(q + m * L::QL) * N + b) * N + c] = (uint8_t)h;
+        }
+      }
+    }
+  }
+}
+
+// ---- adjoint of the criterion -----------------------------------------------------
+// a axis: fields -> masked cotangents (the rule of k_cols_a_adj) -> forward a
+// axis, in place in the pair boxes; per-CTA partial sums of g C / zeta.  The
+// argmax bytes of the tile are read once; a slot with ridx < 0 (the one that
+// fills an odd batch) takes no voxel.
+template <class L, int REGS>
+__global__ void __launch_bounds__(PairCol<L, REGS>::THREADS, PairCol<L, REGS>::PER_SM)
+k_pair_cols_a_adj(Batch bt, const float* __restrict__ g, const uint8_t* __restrict__ Abuf,
+                  const float* __restrict__ alpha_ptr, float* __restrict__ zpart, const float2* __restrict__ plain) {
+  using C = PairCol<L, REGS>;
+  constexpr int N = L::N;
+  extern __shared__ __align__(16) unsigned char psm[];
+  cpair* exs = reinterpret_cast<cpair*>(psm);
+  float2* tw = reinterpret_cast<float2*>(exs + C::TPC * N * 8);
+  __shared__ float red[32];
+  pair_tw_load<L>(tw, plain);
+  const int sub = threadIdx.x / C::LT;
+  const int col = threadIdx.x % 8;
+  const int t = (threadIdx.x % C::LT) / 8;
+  const int tile = blockIdx.x * C::TPC + sub;
+  cpair* ex = exs + sub * N * 8 + col;
+  constexpr long RS = (long)N * 8;
+  const long base = ((long)(tile / N) * N * N + tile % N) * 8 + col;
+  const long vox = (long)(tile % N) * N + (tile / N) * 8 + col;  // natural index of (a = 0, b, c)
+  const float alpha = fabsf(*alpha_ptr);  // sign: the no-source mark
+  const float inv_alpha = 1.0f / alpha;   // exact: alpha is a power of two
+  auto sync = [] { __syncthreads(); };
+  uint32_t arg[L::ITL][(L::EL + 3) / 4];
+#pragma unroll
+  for (int i = 0; i < L::ITL; ++i) {
+    const int q = t + i * L::T;
+#pragma unroll
+    for (int m = 0; m < L::EL; ++m) {
+      uint32_t a = RC_NONE;
+      if (L::QL % L::T == 0 || q < L::QL) a = Abuf[vox + (long)(q + m * L::QL) * N * N];
+      arg[i][m >> 2] = (m & 3) ? arg[i][m >> 2] | a << (8 * (m & 3)) : a;
+    }
+  }
+  float zacc = 0.0f;
+  for (int k = 0; k < bt.K; k += 2) {
+    cpair* box = reinterpret_cast<cpair*>(bt.r[k].work) + base;
+    const int r0 = bt.r[k].ridx, r1 = bt.r[k + 1].ridx;
+    cpair v[L::IT1][L::E1], o[L::ITL][L::EL];
+#pragma unroll
+    for (int i = 0; i < L::IT1; ++i) {
+      const int q = t + i * L::T;
+      if (L::Q1 % L::T == 0 || q < L::Q1) {
+#pragma unroll
+        for (int m = 0; m < L::E1; ++m) v[i][m] = ld_pair(box + (q + m * L::Q1) * RS);
+      }
+    }
+    __syncthreads();  // the previous pair's exchange has been read (k = 0: twiddles)
+    pair_line<L, true, 8>(v, ex, tw, t, sync, [&](int q, int m, int i, const cpair& u) {
+      const int a = (arg[i][m >> 2] >> (8 * (m & 3))) & 0xFF;
+      cpair c = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+      if (a == r0 || a == r1) {
+        const float rec = a == r0 ? u.re.x : u.re.y;  // rec_R (> 0 where A = R)
+        const float h = (a == r0 ? u.im.x : u.im.y) * inv_alpha;
+        const float Cr = __fdiv_rn(bt.zmul * h, rec);
+        const float gg = g[vox + (long)(q + m * L::QL) * N * N];
+        const float ginv = __fdiv_rn(gg, rec);
+        const float2 w = make_float2(-ginv * Cr, ginv * bt.zmul * inv_alpha);
+        if (a == r0) {
+          c.re.x = w.x;
+          c.im.x = w.y;
+        } else {
+          c.re.y = w.x;
+          c.im.y = w.y;
+        }
+        zacc += gg * __fdiv_rn(Cr, bt.zmul);
+      }
+      o[i][m] = c;
+    });
+    __syncthreads();  // the inverse line's exchange has been read
+#pragma unroll
+    for (int i = 0; i < L::ITL; ++i) {
+      const int q = t + i * L::T;
+      if (L::QL % L::T == 0 || q < L::QL) {
+#pragma unroll
+        for (int m = 0; m < L::EL; ++m) st_pair(ex + (q + m * L::QL) * 8, o[i][m]);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < L::IT1; ++i) {
+      const int q = t + i * L::T;
+      if (L::Q1 % L::T == 0 || q < L::Q1) {
+#pragma unroll
+        for (int m = 0; m < L::E1; ++m) v[i][m] = ld_pair(ex + (q + m * L::Q1) * 8);
+      }
+    }
+    __syncthreads();
+    pair_line<L, false, 8>(v, ex, tw, t, sync,
+                           [&](int q, int m, int, const cpair& u) { st_pair(box + (q + m * L::QL) * RS, u); });
+  }
+  // deterministic partial of the CTA (accumulated over the batches in stream order)
+  for (int s = 16; s > 0; s >>= 1) zacc += __shfl_xor_sync(0xffffffffu, zacc, s);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = zacc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float s = 0.0f;
+    for (int w = 0; w < (C::THREADS + 31) / 32; ++w) s += red[w];
+    zpart[blockIdx.x] += s;
+  }
+}
+
+// c axis, forward, of the batch's cotangent pairs, times W_R, summed over the
+// batch in the order of its radii and added to the k-space accumulator
+// (k_rows_adj_acc).  The windows of a row lie in two buffers used in turn.
+template <class L, int RW, int REGS>
+__global__ void __launch_bounds__(PairRow<L, RW, REGS>::THREADS, PairRow<L, RW, REGS>::PER_SM)
+k_pair_rows_adj(Batch bt, float2* __restrict__ acc, const float2* __restrict__ plain) {
+  using R = PairRow<L, RW, REGS>;
+  constexpr int N = L::N;
+  extern __shared__ __align__(16) unsigned char psm[];
+  cpair* exs = reinterpret_cast<cpair*>(psm);
+  float2* ws = reinterpret_cast<float2*>(exs + RW * L::XR);
+  float2* tw = ws + 2 * RW * R::WS;
+  constexpr int NG = N * N / RW;  // row groups
+  const int row = threadIdx.x / L::T, t = threadIdx.x % L::T;
+  cpair* ex = exs + row * L::XR;
+  auto sync = [] {
+    if constexpr (R::THREADS <= 32) __syncwarp();
+    else __syncthreads();
+  };
+  pair_tw_load<L>(tw, plain);
+  __syncthreads();
+  int buf = 0;
+  for (int group = blockIdx.x; group < NG; group += gridDim.x) {
+    const int rid = group * RW + row;
+    float kmag[R::NW];
+    {
+      const int a = rid / N, b = rid % N;
+      const int ka = kfreq(a, N), kb = kfreq(b, N);
+      const int kab = ka * ka + kb * kb;
+#pragma unroll
+      for (int i = 0; i < R::NW; ++i) {
+        const int kc = t + i * L::T;
+        kmag[i] = sqrtf((float)(kab + kc * kc));
+      }
+    }
+    float2 sum[L::ITL][L::EL];
+#pragma unroll
+    for (int i = 0; i < L::ITL; ++i)
+#pragma unroll
+      for (int m = 0; m < L::EL; ++m) sum[i][m] = make_float2(0.0f, 0.0f);
+    for (int k = 0; k < bt.K; k += 2, buf ^= 1) {
+      const cpair* box = reinterpret_cast<const cpair*>(bt.r[k].work) + (long)rid * 8;
+      cpair v[L::IT1][L::E1];
+#pragma unroll
+      for (int i = 0; i < L::IT1; ++i) {
+        const int q = t + i * L::T;
+        if (L::Q1 % L::T == 0 || q < L::Q1) {
+#pragma unroll
+          for (int m = 0; m < L::E1; ++m) {
+            const int c = q + m * L::Q1;
+            v[i][m] = ld_pair(box + (long)(c / 8) * N * N * 8 + c % 8);
+          }
+        }
+      }
+      float2* wrow = ws + (buf * RW + row) * R::WS;
+      const float d0 = bt.r[k].dkR, d1 = bt.r[k + 1].dkR;
+#pragma unroll
+      for (int i = 0; i < R::NW; ++i) {
+        const int kc = t + i * L::T;
+        if (kc <= N / 2) wrow[kc] = make_float2(w_tophat(d0 * kmag[i]), w_tophat(d1 * kmag[i]));
+      }
+      sync();  // the windows are in; the previous pair's exchange has been read
+      const bool both = k + 1 < bt.K;
+      pair_line<L, false, 1>(v, ex, tw, t, sync, [&](int q, int m, int i, const cpair& u) {
+        const int c = q + m * L::QL;
+        const float2 w = wrow[c <= N / 2 ? c : N - c];
+        float2 s = sum[i][m];
+        s.x = fmaf(w.x, u.re.x, s.x);
+        s.y = fmaf(w.x, u.im.x, s.y);
+        if (both) {
+          s.x = fmaf(w.y, u.re.y, s.x);
+          s.y = fmaf(w.y, u.im.y, s.y);
+        }
+        sum[i][m] = s;
+      });
+    }
+    float2* dst = acc + (long)rid * N;
+#pragma unroll
+    for (int i = 0; i < L::ITL; ++i) {
+      const int q = t + i * L::T;
+      if (L::QL % L::T == 0 || q < L::QL) {
+#pragma unroll
+        for (int m = 0; m < L::EL; ++m) {
+          const int c = q + m * L::QL;
+          const float2 old = dst[c];
+          dst[c] = make_float2(old.x + sum[i][m].x, old.y + sum[i][m].y);
         }
       }
     }
@@ -306,17 +548,17 @@ cudaError_t pair_rows_launch(const float2* spec, const Batch& bt, const float2* 
   k_pair_rows_filter<L, RW, REGS><<<pair_min(ng, most), R::THREADS, R::SMEM, st>>>(spec, bt, tw);
   return cudaGetLastError();
 }
-template <class L, int EPI, int REGS>
+template <class L, bool INV, int EPI, int REGS>
 cudaError_t pair_cols_setup() {
-  return cudaFuncSetAttribute(k_pair_cols<L, EPI, REGS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(k_pair_cols<L, INV, EPI, REGS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)PairCol<L, REGS>::SMEM);
 }
-template <class L, int EPI, int REGS, bool AHEAD>
-cudaError_t pair_cols_launch(const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw, int nsm,
+template <class L, bool INV, int EPI, int REGS, bool AHEAD>
+cudaError_t pair_cols_launch(const Batch& bt, uint8_t* rc, float* C, const float* alpha, const float2* tw, int nsm,
                              cudaStream_t st) {
-  using C = PairCol<L, REGS>;
-  k_pair_cols<L, EPI, REGS><<<C::NTILES / C::TPC, C::THREADS, C::SMEM, st>>>(bt, rc, alpha, tw,
-                                                                             AHEAD ? nsm * C::PER_SM : 0);
+  using G = PairCol<L, REGS>;
+  k_pair_cols<L, INV, EPI, REGS><<<G::NTILES / G::TPC, G::THREADS, G::SMEM, st>>>(bt, rc, C, alpha, tw,
+                                                                                  AHEAD ? nsm * G::PER_SM : 0);
   return cudaGetLastError();
 }
 
@@ -329,17 +571,51 @@ struct PairLaunch {
   // side, in the ky pass where an SM holds two CTAs (512: 0.74 against 0.78 clk),
   // not at the small sides (240: 0.78 against 0.75)
   static constexpr bool AHEAD_B = N >= 300;
+  // the criterion and the adjoint hold more per thread than the centre test
+  static constexpr int CRA = S::CR <= 80 ? 112 : S::CR <= 112 ? 128 : 168;
+  static constexpr size_t ADJ_ROW_SMEM =
+      PairRow<Row, S::RW, S::RR>::SMEM + (size_t)S::RW * PairRow<Row, S::RW, S::RR>::WS * sizeof(float2);
   static cudaError_t setup() {
     cudaError_t e = pair_rows_setup<Row, S::RW, S::RR>();
-    if (!e) e = pair_cols_setup<Col, 0, S::CR>();
-    if (!e) e = pair_cols_setup<Col, 1, S::CR>();
+    if (!e) e = pair_cols_setup<Col, true, 0, S::CR>();
+    if (!e) e = pair_cols_setup<Col, true, 1, S::CR>();
+    if (!e) e = pair_cols_setup<Col, true, 2, CRA>();
+    if (!e) e = pair_cols_setup<Col, false, 0, S::CR>();
+    if (!e)
+      e = cudaFuncSetAttribute(k_pair_cols_a_adj<Col, CRA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)PairCol<Col, CRA>::SMEM);
+    if (!e)
+      e = cudaFuncSetAttribute(k_pair_rows_adj<Row, S::RW, S::RR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)ADJ_ROW_SMEM);
     return e;
   }
-  static cudaError_t cols_b(const Batch& bt, const float2* tw, int nsm, cudaStream_t st) {
-    return pair_cols_launch<Col, 0, S::CR, AHEAD_B>(bt, nullptr, nullptr, tw, nsm, st);
+  static cudaError_t cols_b(const Batch& bt, bool inverse, const float2* tw, int nsm, cudaStream_t st) {
+    return inverse ? pair_cols_launch<Col, true, 0, S::CR, AHEAD_B>(bt, nullptr, nullptr, nullptr, tw, nsm, st)
+                   : pair_cols_launch<Col, false, 0, S::CR, AHEAD_B>(bt, nullptr, nullptr, nullptr, tw, nsm, st);
+  }
+  static cudaError_t cols_a_test(const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw, int nsm,
+                                 cudaStream_t st) {
+    return pair_cols_launch<Col, true, 1, S::CR, true>(bt, rc, nullptr, alpha, tw, nsm, st);
+  }
+  static cudaError_t cols_a_crit(const Batch& bt, float* C, uint8_t* A, const float* alpha, const float2* tw, int nsm,
+                                 cudaStream_t st) {
+    return pair_cols_launch<Col, true, 2, CRA, true>(bt, A, C, alpha, tw, nsm, st);
+  }
+  static cudaError_t cols_a_adj(const Batch& bt, const float* g, const uint8_t* A, const float* alpha, float* zpart,
+                                const float2* tw, cudaStream_t st) {
+    using G = PairCol<Col, CRA>;
+    k_pair_cols_a_adj<Col, CRA><<<G::NTILES / G::TPC, G::THREADS, G::SMEM, st>>>(bt, g, A, alpha, zpart, tw);
+    return cudaGetLastError();
+  }
+  static cudaError_t rows_adj(const Batch& bt, float2* acc, const float2* tw, int nsm, cudaStream_t st) {
+    using R = PairRow<Row, S::RW, S::RR>;
+    const int ng = N * N / S::RW, most = nsm * R::PER_SM;
+    k_pair_rows_adj<Row, S::RW, S::RR><<<pair_min(ng, most), R::THREADS, ADJ_ROW_SMEM, st>>>(bt, acc, tw);
+    return cudaGetLastError();
   }
   static constexpr PairOps ops() {
-    return {setup, pair_rows_launch<Row, S::RW, S::RR>, cols_b, pair_cols_launch<Col, 1, S::CR, true>};
+    return {setup,       pair_rows_launch<Row, S::RW, S::RR>, cols_b,   cols_a_test,
+            cols_a_crit, cols_a_adj,                          rows_adj, PairCol<Col, CRA>::NTILES / PairCol<Col, CRA>::TPC};
   }
 };
 

@@ -107,16 +107,28 @@ cudaError_t launch_cols_b_cb(int N, const Batch& bt, const float2* tw, cudaStrea
 cudaError_t launch_cols_a_test_cb(int N, const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw, int nsm,
                                   cudaStream_t st);
 
-// Radius pipeline over pairs of radii (kernels_pair.cuh): the c-axis filter
-// pass, the in-place b-axis pass, the a-axis pass + centre test, on boxes of
-// 16-byte pair values (r[k].work and r[k + 1].work consecutive; slot K holds
-// the last radius again when K is odd).  tw: the plain table exp(-2 pi i t / N).
+// Passes over pairs of radii (kernels_pair.cuh), on boxes of 16-byte pair values
+// (r[k].work and r[k + 1].work consecutive; slot K holds the last radius again
+// when K is odd, with ridx < 0 for the adjoint).  tw: the plain table
+// exp(-2 pi i t / N).
 struct PairOps {  // the launches of one box side
   cudaError_t (*setup)();
+  // c axis with the top-hat filter: spec -> the batch's pair boxes
   cudaError_t (*rows_filter)(const float2* spec, const Batch& bt, const float2* tw, int nsm, cudaStream_t st);
-  cudaError_t (*cols_b)(const Batch& bt, const float2* tw, int nsm, cudaStream_t st);
+  // b axis, in place
+  cudaError_t (*cols_b)(const Batch& bt, bool inverse, const float2* tw, int nsm, cudaStream_t st);
+  // a axis + centre test + first-hit update
   cudaError_t (*cols_a_test)(const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw, int nsm,
                              cudaStream_t st);
+  // a axis + running maximum of the ratio
+  cudaError_t (*cols_a_crit)(const Batch& bt, float* C, uint8_t* A, const float* alpha, const float2* tw, int nsm,
+                             cudaStream_t st);
+  // a axis, cotangents, forward a axis; zpart: adj_blocks partial sums
+  cudaError_t (*cols_a_adj)(const Batch& bt, const float* g, const uint8_t* A, const float* alpha, float* zpart,
+                            const float2* tw, cudaStream_t st);
+  // forward c axis, windows, sum over the batch
+  cudaError_t (*rows_adj)(const Batch& bt, float2* acc, const float2* tw, int nsm, cudaStream_t st);
+  int adj_blocks;
 };
 const PairOps* pair_ops(int N);  // null: no pair kernels for this side
 
