@@ -126,8 +126,6 @@ struct sf21_hii_ctx {
   float* d_xhii2 = nullptr;
   cudaEvent_t ev_done[2] = {nullptr, nullptr}, ev_copied[2] = {nullptr, nullptr};
   float *d_delta = nullptr, *d_src = nullptr, *d_rec0 = nullptr, *d_fres = nullptr;
-  uint64_t* d_chain = nullptr;  // source chain before zeta (double bits), per redshift
-  float2* d_om = nullptr;       // 1 - fresid rounded down / to nearest, per redshift
   float *d_partials = nullptr, *d_alpha = nullptr, *d_xhii = nullptr;
   // criterion / adjoint buffers (allocated on first use)
   float* d_C = nullptr;
@@ -330,7 +328,7 @@ static void free_ctx(sf21_hii_ctx* c) {
   void* ptrs[] = {c->d_delta, c->d_src, c->d_rec0, c->d_fres, c->d_partials, c->d_alpha,
                   c->d_xhii, c->d_spec, c->d_tw, c->d_twp, c->d_rc, c->d_mask, c->d_flag, c->d_box2,
                   c->d_C, c->d_A, c->d_acc, c->d_zpart, c->d_g, c->d_gd, c->d_gs, c->d_halos, c->d_fine,
-                  c->d_hscratch, c->d_chain, c->d_om, c->d_xhii2, c->d_pk, c->d_pk_w, c->d_pk_part,
+                  c->d_hscratch, c->d_xhii2, c->d_pk, c->d_pk_w, c->d_pk_part,
                   c->d_pk_cnt, c->d_t21, c->d_t21_part};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -475,8 +473,6 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
   CREATE_CUDA(dev_malloc(&c->d_src, box_f));
   CREATE_CUDA(dev_malloc(&c->d_rec0, box_f));
   CREATE_CUDA(dev_malloc(&c->d_fres, box_f));
-  CREATE_CUDA(dev_malloc(&c->d_chain, sizeof(uint64_t) * c->n3));
-  CREATE_CUDA(dev_malloc(&c->d_om, sizeof(float2) * c->n3));
   CREATE_CUDA(dev_malloc(&c->d_xhii, box_f));
   CREATE_CUDA(dev_malloc(&c->d_spec, box_c));
   CREATE_CUDA(dev_malloc(&c->d_rc, c->n3));
@@ -736,9 +732,6 @@ static int enqueue_front(sf21_hii_ctx* c, double z, int kind, const float* delta
   int e4 = mark(c, st);
   CTX_CUDA(c, x_cols(c, c->d_spec, none, 1, 0, false, st));
   int e5 = mark(c, st);
-  CTX_CUDA(c, launch_finish_prep(c->n3, src, c->d_fres, c->pa, c->d_chain, c->d_om, st));
-  int e6 = mark(c, st);
-  span(c, KD_PREP, e5, e6);
   span(c, KD_PRO, e0, e1);
   span(c, KD_ALPHA, e1, e2);
   span(c, KD_FROWS, e2, e3);
@@ -860,9 +853,9 @@ static int enqueue_radii(sf21_hii_ctx* c, int set, cudaStream_t st) {
   return SF21_OK;
 }
 
-// Dilation + finish of one set; the per-voxel inputs (rec0, chain, om) are
-// those of the last enqueue_front.
-static int enqueue_finish(sf21_hii_ctx* c, int set, float* xhii, cudaStream_t st) {
+// Dilation + finish of one set; the per-voxel inputs (src, rec0, fresid) and
+// the source multipliers are those of the last enqueue_front.
+static int enqueue_finish(sf21_hii_ctx* c, int set, const float* src, float* xhii, cudaStream_t st) {
   const SetInfo& s = c->sets[set];
   const int N = (int)c->N;
   int* dt0 = reinterpret_cast<int*>(c->d_work[0]);
@@ -872,7 +865,13 @@ static int enqueue_finish(sf21_hii_ctx* c, int set, float* xhii, cudaStream_t st
   int e1 = mark(c, st);
   CTX_CUDA(c, launch_dt_pb(N, dt0, dt1, st));
   int e2 = mark(c, st);
-  CTX_CUDA(c, launch_dt_pc_finish(N, dt1, dbits(s.fesc), c->d_chain, c->d_rec0, c->d_om, xhii, st));
+  FinishArgs fin;
+  memset(&fin, 0, sizeof(fin));
+  for (int m = 0; m < c->pa.n_src_mul; ++m) fin.mul[m] = c->pa.src_mul[m];
+  fin.mul[c->pa.n_src_mul] = dbits(s.fesc);
+  fin.n = c->pa.n_src_mul + 1;
+  fin.pf = prod_fast_prepare(fin.mul, fin.n);
+  CTX_CUDA(c, launch_dt_pc_finish(N, dt1, fin, src, c->d_rec0, c->d_fres, xhii, st));
   int e3 = mark(c, st);
   span(c, KD_DTR, e0, e1);
   span(c, KD_DTB, e1, e2);
@@ -893,7 +892,7 @@ static int enqueue_run(sf21_hii_ctx* c, double z, int kind, const float* delta_d
   if ((rc = enqueue_front(c, z, kind, delta_dev, src_dev, st))) return rc;
   for (int s = 0; s < (int)c->sets.size(); ++s) {
     if ((rc = enqueue_radii(c, s, st))) return rc;
-    if ((rc = enqueue_finish(c, s, xhii_dev + (size_t)s * c->n3, st))) return rc;
+    if ((rc = enqueue_finish(c, s, src_dev, xhii_dev + (size_t)s * c->n3, st))) return rc;
   }
   return SF21_OK;
 }
@@ -982,7 +981,7 @@ static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, doubl
     cudaError_t e = cudaSuccess;
     if (s >= 2) e = cudaStreamWaitEvent(st, c->ev_copied[b], 0);  // staging box free again
     if (e == cudaSuccess && (status = enqueue_radii(c, s, st)) == SF21_OK &&
-        (status = enqueue_finish(c, s, stage[b], st)) == SF21_OK) {
+        (status = enqueue_finish(c, s, c->d_src, stage[b], st)) == SF21_OK) {
       e = cudaEventRecord(c->ev_done[b], st);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(c->copy_stream, c->ev_done[b], 0);
       if (e == cudaSuccess)

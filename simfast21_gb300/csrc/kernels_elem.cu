@@ -27,13 +27,18 @@ __global__ void __launch_bounds__(PRO_THREADS)
 k_prologue(long n3, const float* __restrict__ delta, const float* __restrict__ src,
            const PrologueArgs pa, float* __restrict__ rec0, float* __restrict__ fres,
            float2* __restrict__ packed, float* __restrict__ partials) {
+  // rrec_quick's tables: lanes index them by their own densities
+  __shared__ uint64_t tab[384];
+  for (int t = threadIdx.x; t < 384; t += blockDim.x) tab[t] = rrec_table(t);
+  __syncthreads();
   float sd2 = 0.f, sh2 = 0.f;
   int nz = 0;  // some ionisation rate is not exactly zero
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n3; i += (long)gridDim.x * blockDim.x) {
     const float d = delta[i];
     const sd_t one_d = sd_add(SD_ONE, sd_from_float(d));  // 1. + density_map[i]
     // Each quantity takes its fast path (prologue_fast.h), which returns the
-    // exact chain's float for all but about one voxel in 2^21; those voxels
+    // exact chain's float for all but about one voxel in 2^18 (Rrec: the
+    // quick path for all but one in 2^15, then the fast one); those voxels
     // evaluate the exact chain.
     // fresid = XHI((float)((1+d) * 1.881e-7 * pow(1+z,3) * G_H(z)))      (:220-221)
     float fr;
@@ -41,9 +46,9 @@ k_prologue(long n3, const float* __restrict__ delta, const float* __restrict__ s
       fr = sd_to_float(sd_mul(sd_mul(sd_mul(one_d, pa.c_resid), pa.one_plus_z_cubed), pa.g_h));
     const float fx = xhi_float(fr);
     // density_map = (float)Rrec((float)(1 + d), z)                          (:222)
-    const float od = sd_to_float(one_d);
+    const float od = 1.0f + d;  // one_d rounded to float: rounding it twice is innocuous (53 >= 2 24 + 1)
     float rr;
-    if (!rrec_fast(od, pa.rf, &rr))
+    if (!rrec_quick(od, pa.rf, tab, &rr) && !rrec_fast(od, pa.rf, &rr))
       rr = sd_to_float(rrec_exact(od, pa.r2c, pa.r3, pa.rec1, pa.dvv, pa.v_normc));
     // source before zeta                                                   (:272-274)
     const float s = src[i];

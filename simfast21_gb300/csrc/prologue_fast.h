@@ -20,12 +20,24 @@
 // Host and device compile the same code, so the CPU tests can compare every
 // fast path with its exact chain on any number of inputs.
 #pragma once
+#include <math.h>
+
 #include "softdouble.h"
 
 // ---- shared pieces ----------------------------------------------------------
 
 // floor(a b / 2^62) for signed Q.62 values whose product stays below 2^125.
 SD_HD int64_t pf_mulq62(int64_t a, int64_t b) { return (int64_t)(((sd_i128)a * b) >> 62); }
+
+// Float seeds of the Newton iterations (relative error below 2^-21; the
+// iterations and guard bands allow for it, so host and device may differ).
+SD_HD float pf_seed_recip(float x) {
+#ifdef __CUDA_ARCH__
+  return __fdividef(1.0f, x);
+#else
+  return 1.0f / x;
+#endif
+}
 
 // Product of two significands with bit 63 set, normalised so that bit 63 is
 // set again.  *e gains the product's binary exponent change.  Relative
@@ -61,13 +73,13 @@ SD_HD float pf_bits_float(uint32_t u) {
 }
 
 // Round F = Fm 2^(eF - 64) (bit 63 of Fm set) to float, with sign bit `sign`
-// (bit 31).  Returns false when F lies within 2^18 units of Fm (relative
-// 2^-46) of a float rounding midpoint, or when the float would not be normal.
-SD_HD bool pf_round_guard(uint64_t Fm, int eF, uint32_t sign, float* out) {
+// (bit 31).  Returns false when F lies within `band` units of Fm (2^18:
+// relative 2^-46) of a float rounding midpoint, or when the float would not be normal.
+SD_HD bool pf_round_guard(uint64_t Fm, int eF, uint32_t sign, float* out, uint64_t band = 1ULL << 18) {
   const uint64_t rem = Fm & ((1ULL << 40) - 1);  // the dropped bits; midpoint 2^39
   const uint64_t half = 1ULL << 39;
   const uint64_t dist = rem > half ? rem - half : half - rem;
-  if (dist <= (1ULL << 18)) return false;
+  if (dist <= band) return false;
   uint32_t sig = (uint32_t)(Fm >> 40) + (rem > half ? 1u : 0u);
   int E = eF - 1;  // F = (Fm / 2^63) 2^(eF - 1)
   if (sig >> 24) {
@@ -249,6 +261,80 @@ SD_HD bool rrec_fast(float od, const RrecFast& k, float* out) {
   return pf_round_guard(Fm, eF, 0u, out);
 }
 
+// The same value to relative 2^-41, with a guard band of 2^24 units (2^-40 or
+// more): it declines for about one input in 2^15, which then takes rrec_fast.
+// The series' terms of third and higher order (below 2^-25) are evaluated in
+// float, the squares from 31-bit factors.  tab: rrec_table's 3 x 128 words.
+SD_HD bool rrec_quick(float od, const RrecFast& k, const uint64_t* tab, float* out) {
+  union {
+    float f;
+    uint32_t u;
+  } cv;
+  cv.f = od;
+  const uint32_t fb = cv.u;
+  const int eo = (int)((fb >> 23) & 255);
+  const int e = eo - 127;
+  if (!k.ok || (fb >> 31) || e < -60 || e > 60) return false;
+  const uint64_t mo = (fb & 0x7FFFFFu) | 0x800000u;
+  const int j = (int)((mo >> 16) & 127);
+  // t = m / c_j - 1 in Q.52 (|t| <= 2^-8), ln(1 + t): error below 2^-45
+  const sd_u128 P = (sd_u128)mo * tab[j];
+  const int64_t T = (int64_t)(uint64_t)(P >> 33) - ((int64_t)1 << 52);
+  const int32_t th = (int32_t)(T >> 14);  // Q.38
+  const float tf = (float)th * 3.637978807091713e-12f;
+  const float tc = tf * tf * tf * (0.33333333f + tf * (-0.25f + tf * (0.2f - tf * 0.16666667f)));
+  const int64_t lnp = T - (((int64_t)th * th) >> 25) + (int32_t)(tc * 4503599627370496.0f);
+  // w = r3 (e + log2 parts) in Q.52
+  const int64_t inv_ln2 = (int64_t)((SD_POW_INV_LN2_HI << 2) | (SD_POW_INV_LN2_LO >> 62));
+  const int64_t L = ((int64_t)e << 52) + (int64_t)(tab[128 + j] >> 10) + pf_mulq62(lnp, inv_ln2) - (k.l2r2 >> 10);
+  const int64_t v = -(int64_t)(((sd_i128)L * (int64_t)k.r3) >> 63);
+  const int nv = (int)(v >> 52);
+  const uint64_t f = (uint64_t)v & ((1ULL << 52) - 1);
+  // 2^f = 2^(j2/128) e^x, x < 2^-7.5 in Q.52: error below 2^-44
+  const int j2 = (int)(f >> 45);
+  const uint64_t X = sd_mulhi64(f & ((1ULL << 45) - 1), SD_POW_LN2_HI << 4);
+  const uint32_t xh = (uint32_t)(X >> 14);  // Q.38
+  const float xf = (float)xh * 3.637978807091713e-12f;
+  const float xc = xf * xf * xf * (0.16666667f + xf * (0.041666667f + xf * 0.0083333333f));
+  const uint64_t ex = (1ULL << 52) + X + (((uint64_t)xh * xh) >> 25) + (uint32_t)(xc * 4503599627370496.0f);
+  const uint64_t U = sd_mulhi64(tab[256 + j2] << 1, ex << 11);  // Q.62, [1, 2)
+  uint64_t S;
+  int es;
+  if (nv >= 0) {
+    S = U + (nv < 63 ? (1ULL << 62) >> nv : 0);
+    es = nv;
+  } else {
+    S = (1ULL << 62) + (nv > -64 ? U >> (-nv) : 0);
+    es = 0;
+  }
+  if (S >> 63) {
+    S >>= 1;
+    es += 1;
+  }
+  // 1 / S by one Newton step from a float seed: error below 2^-42
+  const float yf = pf_seed_recip((float)(uint32_t)(S >> 32) * (1.0f / 1073741824.0f));
+  const uint64_t Y0 = (uint64_t)(uint32_t)(yf * 1073741824.0f) << 32;           // Q.62
+  const uint64_t t1 = (1ULL << 61) - sd_mulhi64(S, Y0);                         // 2 - S Y0, Q.60
+  const uint64_t Y = sd_mulhi64(Y0, t1) << 4;                                   // Q.62
+  if (Y == 0) return false;
+  const int lz = sd_clz64(Y);
+  const uint64_t ym = Y << lz;
+  int e2 = 2 * (2 - lz);
+  const uint64_t y2 = pf_mulnorm(ym, ym, &e2);
+  int e4 = 2 * e2;
+  const uint64_t y4 = pf_mulnorm(y2, y2, &e4);
+  int eF = e4 + k.cx - 4 * es;
+  const uint64_t Fm = pf_mulnorm(y4, k.cm, &eF);
+  return pf_round_guard(Fm, eF, 0u, out, 1ULL << 24);
+}
+// Word i of the table: 2^62 / c_j, log2 c_j (Q.62), 2^(j/128) (Q.62).
+SD_HD uint64_t rrec_table(int i) {
+  const int j = i & 127;
+  if (i < 128) return SD_POW_INV[j];
+  if (i < 256) return (SD_POW_L2C_HI[j] << 30) | (SD_POW_L2C_LO[j] >> 34);
+  return (SD_POW_EXP2T_HI[j] << 2) | (SD_POW_EXP2T_LO[j] >> 62);
+}
+
 // ---- the residual neutral fraction -----------------------------------------
 // XHI(ratio), user_functions.c:101-106, operation by operation in double.
 SD_HD sd_t xhi_exact(sd_t r) {
@@ -262,10 +348,75 @@ SD_HD sd_t xhi_exact(sd_t r) {
   return sd_div(num, two_r);                                // /(2.*ratio)
 }
 
+// (float)XHI(ratio) for 2^-30 <= ratio < 2^-4.  With b = 2 ratio there 1 + b
+// and 1 + 2 b are exact doubles, and the reference's c = (1 + b)^2 rounded,
+// minus 4 ratio^2 = b^2 (exact), rounds back to exactly 1 + 2 b: the rounding
+// error of c is at most 2^-53, 1 + 2 b is a multiple of 2^-51.  So its
+// numerator is 1 + b - g with g = sqrt(1 + 2 b) rounded to a multiple of
+// 2^-52, i.e. n 2^-52 with n the integer nearest to
+//   2^52 (1 + b - sqrt(1 + 2 b)) = 2^52 b^2 u,  u = 1 / (1 + b + sqrt(1 + 2 b)),
+// u the root of b^2 u^2 - 2 (1 + b) u + 1 = 0: two Newton steps from a float
+// seed, with the derivative -2 sqrt(1 + 2 b) in float (error of u below 2^-60).
+// Then n 2^-52 / b, whose two roundings give the float unless the quotient
+// lies near a midpoint.  False: outside the range, n undecided (its fraction
+// within 64 units of one half), or the quotient in the guard band.
+SD_HD bool xhi_fast(float ratio, float* out) {
+  union {
+    float f;
+    uint32_t u;
+  } cv;
+  cv.f = ratio;
+  const int er = (int)(cv.u >> 23) - 127;  // a sign bit makes it large
+  if (er < -30 || er > -5) return false;
+  const uint64_t M = (cv.u & 0x7FFFFFu) | 0x800000u;
+  const int k = 22 - er;  // b = M 2^-k, 27 <= k <= 52
+  const uint64_t M2 = M * M;
+  const int s2 = 64 - 2 * k;
+  const uint64_t B2 = s2 >= 0 ? M2 << s2 : M2 >> -s2;           // b^2, Q.64
+  const uint64_t A = (1ULL << 63) + (M << (63 - k));            // 2 (1 + b), Q.62
+  const float bf = 2.0f * ratio;
+  const float sf = sqrtf(1.0f + 2.0f * bf);
+  const float g2 = pf_seed_recip(sf) * 2.0f;                     // 4 / (2 sqrt(1 + 2 b))
+  uint64_t U = (uint64_t)(uint32_t)(pf_seed_recip(1.0f + bf + sf) * 4294967296.0f) << 32;  // u, Q.64
+  // residual 1 - u (2 (1 + b) - b^2 u) in Q.62; the correction in Q.64 is residual x g2
+  int64_t f = (int64_t)((1ULL << 62) - sd_mulhi64(A - (sd_mulhi64(B2, U) >> 2), U));
+  U += (uint64_t)((int64_t)(int32_t)((float)(int32_t)(f >> 14) * g2) * 16384);
+  f = (int64_t)((1ULL << 62) - sd_mulhi64(A - (sd_mulhi64(B2, U) >> 2), U));
+  U += (uint64_t)(int64_t)(int32_t)((float)(int32_t)f * g2);
+  const uint64_t V = sd_mulhi64(M2 << 16, U);                    // M^2 u 2^16; n = V 2^-(2k - 36)
+  const int sh = 2 * k - 36;
+  if (sh >= 64) {  // V < 2^63: n = 0
+    *out = 0.0f;
+    return true;
+  }
+  const uint64_t rem = V & ((1ULL << sh) - 1), half = 1ULL << (sh - 1);
+  if ((rem > half ? rem - half : half - rem) < 64) return false;
+  const uint64_t n = (V >> sh) + (rem > half ? 1 : 0);
+  if (n == 0) {
+    *out = 0.0f;
+    return true;
+  }
+  // F = n 2^(k - 52) / M, 1 / M by one Newton step from a float seed (error
+  // below 2^-42; band 2^23 units)
+  const float mf = (float)(uint32_t)M * 1.1920928955078125e-07f;  // M 2^-23, exact
+  const uint32_t y0 = (uint32_t)(pf_seed_recip(mf) * 2147483648.0f);  // Q.31
+  const uint64_t Y0 = (uint64_t)y0 << 32;                             // Q.63
+  const uint64_t t1 = (1ULL << 63) - sd_mulhi64(M << 40, Y0);         // 2 - m y0, Q.62
+  uint64_t Y = sd_mulhi64(Y0, t1);                                    // Q.61
+  const int lz2 = sd_clz64(Y);                                        // 1/m in (1/2, 1]: 2 or 3
+  Y <<= lz2;
+  const int lz = sd_clz64(n);
+  int eF = k - 10 - lz - (lz2 - 2);
+  const uint64_t Fm = pf_mulnorm(n << lz, Y, &eF);
+  return pf_round_guard(Fm, eF, 0u, out, 1ULL << 23);
+}
+
 // (float)XHI(ratio).  The subtraction 2 ratio + 1 - sqrt(..) cancels most
-// digits for small ratios, so every step before it stays exact; only the
-// last division takes the fast path (div_fast).
+// digits for small ratios, so outside xhi_fast every step before the division
+// stays exact; the division takes the fast path (div_fast).
 SD_HD float xhi_float(float ratio) {
+  float q;
+  if (xhi_fast(ratio, &q)) return q;
   const sd_t r = sd_from_float(ratio);
   if (sd_is_zero(r)) return 0.0f;
   const sd_t two_r = sd_ldexp(r, 1);
@@ -277,6 +428,24 @@ SD_HD float xhi_float(float ratio) {
   float x;
   if (!div_fast(num, two_r, &x)) x = sd_to_float(sd_div(num, two_r));
   return x;
+}
+
+// ---- the cap 1 - fresid (:469-471) -------------------------------------------
+// o = 1.0 - f in double for a float f in [0, 1]: *lo = the largest float <= o,
+// *rn = the float nearest to o.  1 - f rounded once to float equals the double
+// rounded to float (53 >= 2 24 + 1), and o < rn exactly when 1 - f lies more
+// than half a double ulp (2^-54 below 1; a tie goes to rn) under rn; for
+// f >= 1/2 the float difference is exact.
+SD_HD void one_minus(float f, float* lo, float* rn) {
+  const float r = 1.0f - f;
+  union {
+    float f;
+    uint32_t u;
+  } cv;
+  cv.f = r;
+  if (f < 0.5f && f - (1.0f - r) > 5.5511151231257827e-17f) cv.u -= 1;
+  *rn = r;
+  *lo = cv.f;
 }
 
 // ---- host preparation of the constants (host code; visible to both nvcc passes) ---------------------------------------

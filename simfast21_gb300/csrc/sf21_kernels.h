@@ -61,15 +61,16 @@ int prologue_blocks(long n3);
 // Dilation of the first-hit radius field and the final xHII box of one set
 // (kernels_dt.cu): three max-plus passes (a: rc -> i1, b: i1 -> i2,
 // c: i2 -> xhii); the last one also applies the single-cell fill and the cap.
-// finish_prep, once per redshift: source chain before zeta (double bits) and
-// 1 - fresid rounded down / to nearest per voxel.
 cudaError_t dt_setup(int N);
 cudaError_t launch_dt_pa(int N, const uint8_t* rc, const int* nmax, int* i1, cudaStream_t st);
 cudaError_t launch_dt_pb(int N, const int* i1, int* i2, cudaStream_t st);
-cudaError_t launch_dt_pc_finish(int N, const int* i2, uint64_t zeta, const uint64_t* chain, const float* rec0,
-                                const float2* om, float* xhii, cudaStream_t st);
-cudaError_t launch_finish_prep(long n3, const float* src, const float* fres, const PrologueArgs& pa, uint64_t* chain,
-                               float2* om, cudaStream_t st);
+struct FinishArgs {  // the set's source rate: src times mul[0..n-1] (the last one is zeta), as doubles
+  ProdFast pf;
+  uint64_t mul[7];
+  int n;
+};
+cudaError_t launch_dt_pc_finish(int N, const int* i2, const FinishArgs& fin, const float* src, const float* rec0,
+                                const float* fres, float* xhii, cudaStream_t st);
 cudaError_t launch_fill0(long n3, uint64_t zeta, const float* src, const float* rec0,
                          const PrologueArgs& pa, float* fill, cudaStream_t st);
 

@@ -76,3 +76,24 @@ def test_prologue_fast_paths_match_exact_chains(tmp_path):
         assert n > 0 and bad == 0, (name, stats[name], r.stdout)
         if name != "rrec_wide":  # wide exponents include results below the float range
             assert fallback <= max(8, n * 1e-5), (name, stats[name])
+
+
+def test_prologue_quick_paths_match_exact_chains(tmp_path):
+    """The shorter paths (xhi_fast, rrec_quick, one_minus) against the exact
+    soft-double chains: the same float whenever they return, over whole octaves
+    at the ends and in the middle of XHI's range, random inputs on both sides
+    of it, and floats near the points where the cap's rounding changes."""
+    cxx = shutil.which("g++")
+    if not cxx:
+        pytest.skip("g++ not available")
+    exe = str(tmp_path / "prologue_quick_check")
+    subprocess.run([cxx, "-O2", "-std=c++17", "-ffp-contract=off",
+                    "-I", os.path.join(ROOT, "simfast21_gb300", "csrc"),
+                    os.path.join(ROOT, "tests", "native", "prologue_quick_check.cpp"), "-o", exe], check=True)
+    r = subprocess.run([exe, "40000", "31"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+    stats = {l.split()[0]: list(map(int, l.split()[1:])) for l in r.stdout.strip().splitlines()
+             if not l.startswith("#")}
+    for name, (n, bad, fallback) in stats.items():
+        assert n > 0 and bad == 0, (name, stats[name], r.stdout)
+    assert stats["xhi_octaves"][2] <= 1e-3 * stats["xhi_octaves"][0]
