@@ -112,6 +112,7 @@ struct sf21_hii_ctx {
   } gkey = {0, -1, nullptr, nullptr, nullptr, nullptr};
   PipeMaps pmaps;
   const PairOps* pair = nullptr;  // passes over pairs of radii, when the context may use them
+  const PairOps* nat = nullptr;   // the same lines on one natural-layout box
   float2* d_twp = nullptr;        // plain twiddle table of the pair passes (powers of two)
   int* d_err = nullptr;
   int* d_ctl = nullptr;     // work-queue control block of pipeline 8
@@ -143,6 +144,7 @@ struct sf21_hii_ctx {
   float2* d_pk = nullptr;
   float* d_pk_w = nullptr;
   float* d_pk_part = nullptr;
+  float2* d_pk_sum = nullptr;
   unsigned long long* d_pk_cnt = nullptr;
   // 21-cm brightness-temperature buffers (allocated on first use)
   float* d_t21 = nullptr;  // xc, xalpha, TK, T_b boxes
@@ -328,7 +330,7 @@ static void free_ctx(sf21_hii_ctx* c) {
   void* ptrs[] = {c->d_delta, c->d_src, c->d_rec0, c->d_fres, c->d_partials, c->d_alpha,
                   c->d_xhii, c->d_spec, c->d_tw, c->d_twp, c->d_rc, c->d_mask, c->d_flag, c->d_box2,
                   c->d_C, c->d_A, c->d_acc, c->d_zpart, c->d_g, c->d_gd, c->d_gs, c->d_halos, c->d_fine,
-                  c->d_hscratch, c->d_xhii2, c->d_pk, c->d_pk_w, c->d_pk_part,
+                  c->d_hscratch, c->d_xhii2, c->d_pk, c->d_pk_w, c->d_pk_part, c->d_pk_sum,
                   c->d_pk_cnt, c->d_t21, c->d_t21_part};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -480,10 +482,9 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
   // not powers of two): an even number of boxes.  Sides that are not powers
   // of two take one radius at a time when only one box is asked for.
   const PairOps* po = pair_ops((int)N);
-  if (c->gen ? (po && K > 1) : (cfg->path == 0 || cfg->path == 5)) {
-    c->pair = po;
-    CREATE_CUDA(po->setup());
-  }
+  if (po) CREATE_CUDA(po->setup());
+  c->nat = po;
+  if (c->gen ? (po && K > 1) : (cfg->path == 0 || cfg->path == 5)) c->pair = po;
   const int Kw = c->pair ? K + (K & 1) : K;
   c->d_work.assign(Kw, nullptr);
   CREATE_CUDA(dev_malloc(&c->d_work_base, box_c * Kw));
@@ -509,7 +510,7 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
   }
   CREATE_CUDA(dev_malloc(&c->d_tw, sizeof(float2) * N));
   CREATE_CUDA(cudaMemcpy(c->d_tw, tw.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
-  if (c->pair && !c->gen) {  // the plain table as well
+  if (c->nat && !c->gen) {  // the plain table as well
     for (long t = 0; t < N; ++t) {
       const double ang = -2.0 * kPI * t / N;
       tw[t] = make_float2((float)cos(ang), (float)sin(ang));
@@ -680,6 +681,7 @@ const PairOps* pair_ops(int N) {
 static cudaError_t x_fwd_rows(sf21_hii_ctx* c, const float2* in, float2* out, const float* alpha, cudaStream_t st) {
   Batch none;
   memset(&none, 0, sizeof(none));
+  if (c->nat) return c->nat->nat_rows(in, nullptr, nullptr, out, (int)c->N, false, alpha, pair_tw(c), c->nsm, st);
   if (c->gen && gen600_supported((int)c->N)) return launch_gen600_rows(0, in, out, none, alpha, c->d_tw, false, st);
   return c->gen ? launch_gen_fwd_rows(c->gp, in, out, alpha, c->d_tw, st)
                 : launch_fwd_rows((int)c->N, in, out, alpha, c->d_tw, st);
@@ -687,6 +689,7 @@ static cudaError_t x_fwd_rows(sf21_hii_ctx* c, const float2* in, float2* out, co
 static cudaError_t x_inv_rows_plain(sf21_hii_ctx* c, float2* box, cudaStream_t st) {
   Batch none;
   memset(&none, 0, sizeof(none));
+  if (c->nat) return c->nat->nat_rows(box, nullptr, nullptr, box, (int)c->N, true, nullptr, pair_tw(c), c->nsm, st);
   if (c->gen && gen600_supported((int)c->N)) return launch_gen600_rows(1, box, box, none, nullptr, c->d_tw, false, st);
   return c->gen ? launch_gen_inv_rows_plain(c->gp, box, c->d_tw, st) : launch_inv_rows_plain((int)c->N, box, c->d_tw, st);
 }
@@ -700,6 +703,7 @@ static cudaError_t x_inv_rows_filter(sf21_hii_ctx* c, const float2* spec, const 
 // box, or (box null) the batch's nbox = bt.K boxes
 static cudaError_t x_cols(sf21_hii_ctx* c, float2* box, const Batch& bt, int nbox, int axis, bool inverse,
                           cudaStream_t st, bool cb = false) {
+  if (box && c->nat) return c->nat->nat_cols(box, axis, inverse, (int)c->N, pair_tw(c), st);
   if (!c->gen) return launch_cols((int)c->N, box, bt, nbox, axis, inverse, c->d_tw, st);
   if (!box && nbox != bt.K) return cudaErrorInvalidValue;
   if (gen600_supported((int)c->N)) return launch_gen600_cols(box, bt, axis, inverse, cb, c->d_tw, st);
@@ -1512,6 +1516,7 @@ static int power_spectrum_device(sf21_hii_ctx* c, const float* box_dev, int flag
   if (!c->d_pk) CTX_CUDA(c, dev_malloc(&c->d_pk, sizeof(float2) * c->n3));
   if (!c->d_pk_w) CTX_CUDA(c, dev_malloc(&c->d_pk_w, sizeof(float) * N));
   if (!c->d_pk_part) CTX_CUDA(c, dev_malloc(&c->d_pk_part, sizeof(float) * (size_t)grid * nk));
+  if (!c->d_pk_sum) CTX_CUDA(c, dev_malloc(&c->d_pk_sum, sizeof(float2) * nk));
   if (!c->d_pk_cnt) CTX_CUDA(c, dev_malloc(&c->d_pk_cnt, sizeof(unsigned long long) * nk));
   std::vector<float> wax(N);
   double s1 = 0.;
@@ -1525,22 +1530,29 @@ static int power_spectrum_device(sf21_hii_ctx* c, const float* box_dev, int flag
   Batch none;
   memset(&none, 0, sizeof(none));
   CTX_CUDA(c, cudaMemcpyAsync(c->d_pk_w, wax.data(), sizeof(float) * N, cudaMemcpyHostToDevice, st));
-  CTX_CUDA(c, launch_pk_pack(N, box_dev, c->d_pk_w, packed, st));
-  CTX_CUDA(c, x_fwd_rows(c, packed, c->d_pk, nullptr, st));
-  CTX_CUDA(c, x_cols(c, c->d_pk, none, 1, 1, false, st));
-  CTX_CUDA(c, x_cols(c, c->d_pk, none, 1, 0, false, st));
+  if (c->nat) {  // the binning reads p = 0..N/2 only: the other columns are not transformed
+    const int half = N / 2 + 1;
+    CTX_CUDA(c, c->nat->nat_rows(nullptr, box_dev, c->d_pk_w, c->d_pk, half, false, nullptr, pair_tw(c), c->nsm, st));
+    CTX_CUDA(c, c->nat->nat_cols(c->d_pk, 1, false, half, pair_tw(c), st));
+    CTX_CUDA(c, c->nat->nat_cols(c->d_pk, 0, false, half, pair_tw(c), st));
+  } else {
+    CTX_CUDA(c, launch_pk_pack(N, box_dev, c->d_pk_w, packed, st));
+    CTX_CUDA(c, x_fwd_rows(c, packed, c->d_pk, nullptr, st));
+    CTX_CUDA(c, x_cols(c, c->d_pk, none, 1, 1, false, st));
+    CTX_CUDA(c, x_cols(c, c->d_pk, none, 1, 0, false, st));
+  }
   CTX_CUDA(c, cudaMemsetAsync(c->d_pk_cnt, 0, sizeof(unsigned long long) * nk, st));
   CTX_CUDA(c, launch_pk_bin(N, c->d_pk, nk, c->d_pk_part, c->d_pk_cnt, st));
-  std::vector<float> part((size_t)grid * nk);
+  CTX_CUDA(c, launch_pk_reduce(N, nk, c->d_pk_part, c->d_pk_sum, st));
+  std::vector<float2> sums(nk);
   std::vector<unsigned long long> cnt(nk);
-  CTX_CUDA(c, cudaMemcpyAsync(part.data(), c->d_pk_part, sizeof(float) * part.size(), cudaMemcpyDeviceToHost, st));
+  CTX_CUDA(c, cudaMemcpyAsync(sums.data(), c->d_pk_sum, sizeof(float2) * nk, cudaMemcpyDeviceToHost, st));
   CTX_CUDA(c, cudaMemcpyAsync(cnt.data(), c->d_pk_cnt, sizeof(unsigned long long) * nk, cudaMemcpyDeviceToHost, st));
   CTX_CUDA(c, cudaStreamSynchronize(st));
   const double dk = 2.0 * kPI / (N * dl);
   const double dl3 = dl * dl * dl;
   for (int b = 0; b < nk && b < cap; ++b) {
-    double sum = 0.;
-    for (int g = 0; g < grid; ++g) sum += (double)part[(size_t)g * nk + b];
+    const double sum = (double)sums[b].x + (double)sums[b].y;
     const double n = cnt[b] ? (double)cnt[b] : 1.0;
     k[b] = b * dk;
     P[b] = sum / n / wsum * dl3;
@@ -1635,8 +1647,12 @@ extern "C" int sf21_t21_run_z(sf21_hii_ctx* c, const sf21_t21_cosmo* cosmo, doub
   Batch none;
   memset(&none, 0, sizeof(none));
   float2* packed = c->d_work[0];
-  CTX_CUDA(c, launch_t21_pack(n3, c->d_delta, packed, st));
-  CTX_CUDA(c, x_fwd_rows(c, packed, c->d_pk, nullptr, st));
+  if (c->nat) {
+    CTX_CUDA(c, c->nat->nat_rows(nullptr, c->d_delta, nullptr, c->d_pk, N, false, nullptr, pair_tw(c), c->nsm, st));
+  } else {
+    CTX_CUDA(c, launch_t21_pack(n3, c->d_delta, packed, st));
+    CTX_CUDA(c, x_fwd_rows(c, packed, c->d_pk, nullptr, st));
+  }
   CTX_CUDA(c, x_cols(c, c->d_pk, none, 1, 1, false, st));
   CTX_CUDA(c, x_cols(c, c->d_pk, none, 1, 0, false, st));
   CTX_CUDA(c, launch_t21_kfilter(N, cosmo->vel_comp, c->d_pk, st));

@@ -478,6 +478,108 @@ k_pair_rows_adj(Batch bt, float2* __restrict__ acc, const float2* __restrict__ p
   }
 }
 
+// ---- one natural-layout box: pairs of rows, pairs of columns ------------------------
+// The same lines on one complex box a N^2 + b N + c, the lanes being two rows
+// (2r, 2r + 1) or two adjacent columns.
+//
+// c axis, forward or inverse.  in: complex rows (the imaginary part times
+// |*alpha|), or real rows times the axis windows (real: wax of N values, or null).
+// Only the columns c < ncol of the result are stored.
+template <class L, int RW, int REGS, bool INV>
+__global__ void __launch_bounds__(PairRow<L, RW, REGS>::THREADS, PairRow<L, RW, REGS>::PER_SM)
+k_pair_nat_rows(const float2* in, const float* __restrict__ real, const float* __restrict__ wax, float2* out, int ncol,
+                const float* __restrict__ alpha_ptr, const float2* __restrict__ plain) {
+  using R = PairRow<L, RW, REGS>;
+  constexpr int N = L::N;
+  extern __shared__ __align__(16) unsigned char psm[];
+  cpair* exs = reinterpret_cast<cpair*>(psm);
+  float2* tw = reinterpret_cast<float2*>(exs + RW * L::XR);
+  constexpr int NG = N * N / 2 / RW;  // groups of row pairs
+  const int row = threadIdx.x / L::T, t = threadIdx.x % L::T;
+  cpair* ex = exs + row * L::XR;
+  auto sync = [] {
+    if constexpr (R::THREADS <= 32) __syncwarp();
+    else __syncthreads();
+  };
+  pair_tw_load<L>(tw, plain);
+  const float alpha = alpha_ptr ? fabsf(*alpha_ptr) : 1.0f;
+  for (int group = blockIdx.x; group < NG; group += gridDim.x) {
+    const long r0 = 2 * ((long)group * RW + row);
+    cpair v[L::IT1][L::E1];
+    float w0 = 1.0f, w1 = 1.0f;  // the windows of the a and b axes
+    if (real && wax) {
+      const float wa = wax[r0 / N];  // N is even: both rows have the same a
+      w0 = __fmul_rn(wa, wax[r0 % N]);
+      w1 = __fmul_rn(wa, wax[r0 % N + 1]);
+    }
+#pragma unroll
+    for (int i = 0; i < L::IT1; ++i) {
+      const int q = t + i * L::T;
+      if (L::Q1 % L::T == 0 || q < L::Q1) {
+#pragma unroll
+        for (int m = 0; m < L::E1; ++m) {
+          const int c = q + m * L::Q1;
+          if (real) {
+            float x0 = real[r0 * N + c], x1 = real[(r0 + 1) * N + c];
+            if (wax) {
+              x0 = __fmul_rn(x0, __fmul_rn(w0, wax[c]));
+              x1 = __fmul_rn(x1, __fmul_rn(w1, wax[c]));
+            }
+            v[i][m] = {make_float2(x0, x1), make_float2(0.0f, 0.0f)};
+          } else {
+            const float2 x0 = in[r0 * N + c], x1 = in[(r0 + 1) * N + c];
+            v[i][m] = {make_float2(x0.x, x1.x), make_float2(x0.y * alpha, x1.y * alpha)};
+          }
+        }
+      }
+    }
+    sync();  // twiddles; the previous group's exchange has been read
+    pair_line<L, INV, 1>(v, ex, tw, t, sync, [&](int q, int m, int, const cpair& u) {
+      const int c = q + m * L::QL;
+      if (c < ncol) {
+        out[r0 * N + c] = make_float2(u.re.x, u.im.x);
+        out[(r0 + 1) * N + c] = make_float2(u.re.y, u.im.y);
+      }
+    });
+  }
+}
+
+// b (AXIS 1) or a (AXIS 0) axis in place: tiles of 16 columns, as 8 pairs.
+// blockIdx.x = column block + nblk outer index (nblk blocks cover the columns
+// that are wanted; a block past the side is cut).
+template <class L, bool INV, int AXIS, int REGS>
+__global__ void __launch_bounds__(PairCol<L, REGS>::LT, PairCol<L, REGS>::PER_SM)
+k_pair_nat_cols(float2* box, int nblk, const float2* __restrict__ plain) {
+  constexpr int N = L::N;
+  extern __shared__ __align__(16) unsigned char psm[];
+  cpair* exs = reinterpret_cast<cpair*>(psm);
+  float2* tw = reinterpret_cast<float2*>(exs + N * 8);
+  pair_tw_load<L>(tw, plain);
+  const int col = threadIdx.x % 8, t = threadIdx.x / 8;
+  const int outer = blockIdx.x / nblk, c = (blockIdx.x % nblk) * 16 + 2 * col;
+  constexpr long RS = AXIS == 1 ? N : (long)N * N;
+  const bool on = N % 16 == 0 || c < N;
+  float4* line = reinterpret_cast<float4*>(box + (AXIS == 1 ? (long)outer * N * N : (long)outer * N) + (on ? c : 0));
+  constexpr long RS2 = RS / 2;  // float4 from one element of a line to the next
+  cpair v[L::IT1][L::E1];
+#pragma unroll
+  for (int i = 0; i < L::IT1; ++i) {
+    const int q = t + i * L::T;
+    if (L::Q1 % L::T == 0 || q < L::Q1) {
+#pragma unroll
+      for (int m = 0; m < L::E1; ++m) {
+        const float4 x = line[(q + m * L::Q1) * RS2];
+        v[i][m] = {make_float2(x.x, x.z), make_float2(x.y, x.w)};
+      }
+    }
+  }
+  __syncthreads();
+  auto sync = [] { __syncthreads(); };
+  pair_line<L, INV, 8>(v, exs + col, tw, t, sync, [&](int q, int m, int, const cpair& u) {
+    if (on) line[(q + m * L::QL) * RS2] = make_float4(u.re.x, u.im.x, u.re.y, u.im.y);
+  });
+}
+
 // ---- the lines of each side ----------------------------------------------------------
 // Column tiles: threads per line, codes, planned registers.  Rows: threads per
 // line, rows per CTA, planned registers, codes.  Chosen by timing candidates
@@ -587,7 +689,35 @@ struct PairLaunch {
     if (!e)
       e = cudaFuncSetAttribute(k_pair_rows_adj<Row, S::RW, S::RR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)ADJ_ROW_SMEM);
+    if (!e) e = nat_setup();
     return e;
+  }
+  // one natural-layout box
+  static constexpr size_t NAT_COL_SMEM = (size_t)N * 8 * sizeof(cpair) + Col::TW * sizeof(float2);
+  static cudaError_t nat_setup() {
+    cudaError_t e = cudaSuccess;
+    for (auto f : {k_pair_nat_rows<Row, S::RW, S::RR, false>, k_pair_nat_rows<Row, S::RW, S::RR, true>})
+      if (!e)
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairRow<Row, S::RW, S::RR>::SMEM);
+    for (auto f : {k_pair_nat_cols<Col, false, 0, S::CR>, k_pair_nat_cols<Col, false, 1, S::CR>,
+                   k_pair_nat_cols<Col, true, 0, S::CR>, k_pair_nat_cols<Col, true, 1, S::CR>})
+      if (!e) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NAT_COL_SMEM);
+    return e;
+  }
+  static cudaError_t nat_rows(const float2* in, const float* real, const float* wax, float2* out, int ncol, bool inverse,
+                              const float* alpha, const float2* tw, int nsm, cudaStream_t st) {
+    using R = PairRow<Row, S::RW, S::RR>;
+    const int ng = N * N / 2 / S::RW, most = nsm * R::PER_SM;
+    auto f = inverse ? k_pair_nat_rows<Row, S::RW, S::RR, true> : k_pair_nat_rows<Row, S::RW, S::RR, false>;
+    f<<<pair_min(ng, most), R::THREADS, R::SMEM, st>>>(in, real, wax, out, ncol, alpha, tw);
+    return cudaGetLastError();
+  }
+  static cudaError_t nat_cols(float2* box, int axis, bool inverse, int ncol, const float2* tw, cudaStream_t st) {
+    auto f = inverse ? (axis ? k_pair_nat_cols<Col, true, 1, S::CR> : k_pair_nat_cols<Col, true, 0, S::CR>)
+                     : (axis ? k_pair_nat_cols<Col, false, 1, S::CR> : k_pair_nat_cols<Col, false, 0, S::CR>);
+    const int nblk = (ncol + 15) / 16;
+    f<<<N * nblk, PairCol<Col, S::CR>::LT, NAT_COL_SMEM, st>>>(box, nblk, tw);
+    return cudaGetLastError();
   }
   static cudaError_t cols_b(const Batch& bt, bool inverse, const float2* tw, int nsm, cudaStream_t st) {
     return inverse ? pair_cols_launch<Col, true, 0, S::CR, AHEAD_B>(bt, nullptr, nullptr, nullptr, tw, nsm, st)
@@ -615,7 +745,8 @@ struct PairLaunch {
   }
   static constexpr PairOps ops() {
     return {setup,       pair_rows_launch<Row, S::RW, S::RR>, cols_b,   cols_a_test,
-            cols_a_crit, cols_a_adj,                          rows_adj, PairCol<Col, CRA>::NTILES / PairCol<Col, CRA>::TPC};
+            cols_a_crit, cols_a_adj,                          rows_adj, PairCol<Col, CRA>::NTILES / PairCol<Col, CRA>::TPC,
+            nat_rows,    nat_cols};
   }
 };
 

@@ -130,6 +130,12 @@ struct PairOps {  // the launches of one box side
   // forward c axis, windows, sum over the batch
   cudaError_t (*rows_adj)(const Batch& bt, float2* acc, const float2* tw, int nsm, cudaStream_t st);
   int adj_blocks;
+  // one natural-layout complex box.  c axis: from complex rows (imaginary part
+  // times |*alpha|) or real rows (times the axis windows wax, if given) to the
+  // columns c < ncol; b (1) or a (0) axis: in place, the columns c < ncol.
+  cudaError_t (*nat_rows)(const float2* in, const float* real, const float* wax, float2* out, int ncol, bool inverse,
+                          const float* alpha, const float2* tw, int nsm, cudaStream_t st);
+  cudaError_t (*nat_cols)(float2* box, int axis, bool inverse, int ncol, const float2* tw, cudaStream_t st);
 };
 const PairOps* pair_ops(int N);  // null: no pair kernels for this side
 
@@ -189,6 +195,8 @@ int pk_bin_grid(int N);
 cudaError_t launch_pk_pack(int N, const float* box, const float* wax, float2* out, cudaStream_t st);
 cudaError_t launch_pk_bin(int N, const float2* spec, int nk, float* partials, unsigned long long* counts,
                           cudaStream_t st);
+// sums[b] = the CTAs' sums of bin b as a pair of floats (hi + lo)
+cudaError_t launch_pk_reduce(int N, int nk, const float* partials, float2* sums, cudaStream_t st);
 
 // 21-cm brightness temperature (kernels_t21.cu).
 struct T21Args {
