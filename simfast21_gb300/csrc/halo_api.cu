@@ -433,6 +433,9 @@ struct sf21_halo_ctx {
   double dx = 0, dk = 0;
   cudaStream_t stream = nullptr;
   float2 *d_tw = nullptr, *d_spec = nullptr, *d_work = nullptr;
+  const PairOps* pair = nullptr;  // pair lines of the side, if it has them
+  float2* d_twp = nullptr;        // their plain twiddle table
+  int nsm = 0;
   int KP = 2;  // mass pairs per filter-bank pass
   bool gen = false;  // side not a power of two: the shared-memory transforms (kernels_gen.cu)
   GenPlan gp = {};
@@ -564,7 +567,7 @@ static void taus_jump(uint32_t s[3], uint64_t q) {
 static void free_hctx(sf21_halo_ctx* c) {
   if (!c) return;
   if (c->device >= 0) cudaSetDevice(c->device);
-  void* ptrs[] = {c->d_tw,        c->d_spec,      c->d_work,      c->d_delta,     c->d_FL,        c->d_UND,
+  void* ptrs[] = {c->d_twp,       c->d_tw,        c->d_spec,      c->d_work,      c->d_delta,     c->d_FL,        c->d_UND,
                   c->d_ACC,       c->d_bits,      c->d_list,      c->d_list2,     c->d_status,    c->d_chunk,
                   c->d_cnt,       c->d_cat,       c->d_runs,      c->d_sg_pow2,   c->d_sg_local,  c->d_sgL,
                   c->d_sgX,       c->d_sgD,       c->d_sg_cnt,    c->d_sg_start,  c->d_sgLB,      c->sg_eb.gx,    c->sg_eb.sx,    c->sg_eb.gentry,
@@ -660,6 +663,18 @@ extern "C" int sf21_halo_create(const sf21_halo_config* cfg, sf21_halo_ctx** out
   }
   HCREATE(dev_malloc(&c->d_tw, sizeof(float2) * N));
   HCREATE(cudaMemcpy(c->d_tw, tw.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
+  // sides with pair lines: the filter bank takes two transforms at a time
+  c->pair = N == 600 ? nullptr : pair_ops(N);
+  if (c->pair) {
+    HCREATE(c->pair->setup());
+    HCREATE(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device));
+    for (int t = 0; t < N; ++t) {
+      const double ang = -2.0 * kPI * t / N;
+      tw[t] = make_float2((float)cos(ang), (float)sin(ang));
+    }
+    HCREATE(dev_malloc(&c->d_twp, sizeof(float2) * N));
+    HCREATE(cudaMemcpy(c->d_twp, tw.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
+  }
 #undef HCREATE
   *out = c;
   return SF21_OK;
@@ -677,8 +692,12 @@ static int set_density_dev(sf21_halo_ctx* c, const float* d, cudaStream_t st) {
   memset(&none, 0, sizeof(none));
   if (d != c->d_delta) HCTX_CUDA(c, cudaMemcpyAsync(c->d_delta, d, sizeof(float) * c->n3, cudaMemcpyDeviceToDevice, st));
   float2* packed = c->d_work;
-  HCTX_CUDA(c, launch_t21_pack(c->n3, c->d_delta, packed, st));
-  if (c->gen) {
+  if (!c->pair) HCTX_CUDA(c, launch_t21_pack(c->n3, c->d_delta, packed, st));
+  if (c->pair) {
+    HCTX_CUDA(c, c->pair->nat_rows(nullptr, c->d_delta, nullptr, c->d_spec, N, false, nullptr, c->d_twp, c->nsm, st));
+    HCTX_CUDA(c, c->pair->nat_cols(c->d_spec, 1, false, N, c->d_twp, st));
+    HCTX_CUDA(c, c->pair->nat_cols(c->d_spec, 0, false, N, c->d_twp, st));
+  } else if (c->gen) {
     HCTX_CUDA(c, launch_gen_fwd_rows(c->gp, packed, c->d_spec, nullptr, c->d_tw, st));
     HCTX_CUDA(c, launch_gen_cols(c->gp, c->d_spec, none, 1, false, c->d_tw, st));
     HCTX_CUDA(c, launch_gen_cols(c->gp, c->d_spec, none, 0, false, c->d_tw, st));
@@ -1047,7 +1066,12 @@ static int run_filter_bank(sf21_halo_ctx* c, const std::vector<MassPlan>& plan, 
       ++hb.K;
     }
     bt.K = hb.K;
-    if (c->gen) {
+    if (c->pair) {
+      if (hb.K & 1) hb.p[hb.K] = hb.p[hb.K - 1];
+      HCTX_CUDA(c, c->pair->hf_rows(c->d_spec, hb, c->d_twp, c->nsm, st));
+      HCTX_CUDA(c, c->pair->cols_b(bt, true, c->d_twp, c->nsm, st));
+      HCTX_CUDA(c, c->pair->hf_cols_a(hb, c->d_twp, c->nsm, st));
+    } else if (c->gen) {
       HCTX_CUDA(c, launch_gen_hf_rows_filter(c->gp, c->d_spec, hb, c->d_tw, st));
       HCTX_CUDA(c, launch_gen_hf_cols(c->gp, hb, 1, false, c->d_tw, st));
       HCTX_CUDA(c, launch_gen_hf_cols(c->gp, hb, 0, true, c->d_tw, st));

@@ -478,6 +478,171 @@ k_pair_rows_adj(Batch bt, float2* __restrict__ acc, const float2* __restrict__ p
   }
 }
 
+// ---- the halo finder's filter bank ---------------------------------------------------
+// Two complex transforms (of two masses each: F (s W_a + i s W_b), kernels_hf.cu)
+// as the lanes of a pair.  Slot K of a batch with an odd number of transforms
+// repeats the last one.
+// The product is written with the fused multiply-adds that the compiler forms
+// for z.x wa - z.y wb and z.x wb + z.y wa in the one-transform kernels
+// (kernels_hf.cu at the powers of two, kernels_gen.cu at the other sides; the
+// other three forms differ from them in more than half of the values).
+template <bool POW2>
+__device__ __forceinline__ float2 hf_mul(float2 z, float wa, float wb) {
+  return make_float2(fmaf(z.x, wa, -__fmul_rn(z.y, wb)),
+                     POW2 ? fmaf(z.x, wb, __fmul_rn(z.y, wa)) : fmaf(z.y, wa, __fmul_rn(z.x, wb)));
+}
+
+template <class L, int RW, int REGS>
+__global__ void __launch_bounds__(PairRow<L, RW, REGS>::THREADS, PairRow<L, RW, REGS>::PER_SM)
+k_pair_hf_rows(const float2* __restrict__ spec, HfBatch hb, const float2* __restrict__ plain) {
+  using R = PairRow<L, RW, REGS>;
+  constexpr int N = L::N;
+  extern __shared__ __align__(16) unsigned char psm[];
+  cpair* exs = reinterpret_cast<cpair*>(psm);
+  float4* ws = reinterpret_cast<float4*>(exs + RW * L::XR);  // the four masses' windows of a row
+  float2* tw = reinterpret_cast<float2*>(ws + RW * R::WS);
+  constexpr int NG = N * N / RW;  // row groups
+  const int row = threadIdx.x / L::T, t = threadIdx.x % L::T;
+  cpair* ex = exs + row * L::XR;
+  float4* wrow = ws + row * R::WS;
+  auto sync = [] {
+    if constexpr (R::THREADS <= 32) __syncwarp();
+    else __syncthreads();
+  };
+  pair_tw_load<L>(tw, plain);
+  __syncthreads();
+  for (int group = blockIdx.x; group < NG; group += gridDim.x) {
+    const int rid = group * RW + row;
+    const int a = rid / N, b = rid % N;
+    const int ka = kfreq(a, N), kb = kfreq(b, N);
+    const int kab = ka * ka + kb * kb;
+    float2 z[L::IT1][L::E1];
+    const float2* src = spec + (long)rid * N;
+#pragma unroll
+    for (int i = 0; i < L::IT1; ++i) {
+      const int q = t + i * L::T;
+      if (L::Q1 % L::T == 0 || q < L::Q1) {
+#pragma unroll
+        for (int m = 0; m < L::E1; ++m) z[i][m] = __ldg(src + q + m * L::Q1);
+      }
+    }
+    if (group + gridDim.x < NG)  // the next group's rows on their way into L2
+      for (int i = threadIdx.x; i < RW * N / 16; i += R::THREADS)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(spec + (long)(group + gridDim.x) * RW * N + 16 * i));
+    for (int k = 0; k < hb.K; k += 2) {
+      const HfPair &p0 = hb.p[k], &p1 = hb.p[k + 1];
+      sync();  // the previous windows and exchange have been read
+      for (int kc = t; kc <= N / 2; kc += L::T) {
+        const float kmag = sqrtf((float)(kab + kc * kc));
+        float4 w;
+        w.x = __fmul_rn(hb.scale, w_tophat(p0.dkRa * kmag));
+        w.y = p0.bits_b ? __fmul_rn(hb.scale, w_tophat(p0.dkRb * kmag)) : 0.0f;
+        w.z = __fmul_rn(hb.scale, w_tophat(p1.dkRa * kmag));
+        w.w = p1.bits_b ? __fmul_rn(hb.scale, w_tophat(p1.dkRb * kmag)) : 0.0f;
+        wrow[kc] = w;
+      }
+      sync();
+      cpair v[L::IT1][L::E1];
+#pragma unroll
+      for (int i = 0; i < L::IT1; ++i) {
+        const int q = t + i * L::T;
+        if (L::Q1 % L::T == 0 || q < L::Q1) {
+#pragma unroll
+          for (int m = 0; m < L::E1; ++m) {
+            const int c = q + m * L::Q1;
+            const float4 w = wrow[c <= N / 2 ? c : N - c];
+            constexpr bool POW2 = (N & (N - 1)) == 0;
+            const float2 x = hf_mul<POW2>(z[i][m], w.x, w.y), y = hf_mul<POW2>(z[i][m], w.z, w.w);
+            v[i][m].re = make_float2(x.x, y.x);
+            v[i][m].im = make_float2(x.y, y.y);
+          }
+        }
+      }
+      cpair* box = reinterpret_cast<cpair*>(p0.work) + (long)rid * 8;
+      pair_line<L, true, 1>(v, ex, tw, t, sync, [&](int q, int m, int, const cpair& u) {
+        const int c = q + m * L::QL;
+        st_pair(box + (long)(c / 8) * N * N * 8 + c % 8, u);
+      });
+    }
+  }
+}
+
+// a axis + the four thresholds: one bit per cell and mass, a byte of the bit
+// sets per row of a tile.  The column blocks run fastest, so that the bytes of
+// a sector are written close together.
+template <class L, int REGS>
+__global__ void __launch_bounds__(PairCol<L, REGS>::THREADS, PairCol<L, REGS>::PER_SM)
+k_pair_hf_cols_a(HfBatch hb, const float2* __restrict__ plain, int ahead) {
+  using C = PairCol<L, REGS>;
+  constexpr int N = L::N;
+  extern __shared__ __align__(16) unsigned char psm[];
+  cpair* exs = reinterpret_cast<cpair*>(psm);
+  float2* tw = reinterpret_cast<float2*>(exs + C::TPC * N * 8);
+  pair_tw_load<L>(tw, plain);
+  const int sub = threadIdx.x / C::LT;
+  const int col = threadIdx.x % 8;
+  const int t = (threadIdx.x % C::LT) / 8;
+  const int tile = blockIdx.x * C::TPC + sub;
+  const int cb = tile % (N / 8), b = tile / (N / 8);
+  cpair* ex = exs + sub * N * 8 + col;
+  constexpr long RS = (long)N * 8;
+  const long base = ((long)cb * N * N + b) * 8;
+  const int lane = threadIdx.x & 31;
+  const unsigned wmask =
+      C::THREADS % 32 && threadIdx.x / 32 == C::THREADS / 32 ? (1u << (C::THREADS % 32)) - 1u : 0xffffffffu;
+  auto sync = [] { __syncthreads(); };
+  for (int k = 0; k < hb.K; k += 2) {
+    const HfPair &p0 = hb.p[k], &p1 = hb.p[k + 1];
+    const bool both = k + 1 < hb.K;
+    const cpair* box = reinterpret_cast<const cpair*>(p0.work) + base + col;
+    cpair v[L::IT1][L::E1];
+#pragma unroll
+    for (int i = 0; i < L::IT1; ++i) {
+      const int q = t + i * L::T;
+      if (L::Q1 % L::T == 0 || q < L::Q1) {
+#pragma unroll
+        for (int m = 0; m < L::E1; ++m) v[i][m] = ld_pair(box + (q + m * L::Q1) * RS);
+      }
+    }
+    const int ntile = tile + ahead * C::TPC;
+    if (ntile < C::NTILES) {  // a later tile's lines on their way into L2
+      const cpair* nx = reinterpret_cast<const cpair*>(p0.work) + ((long)(ntile % (N / 8)) * N * N + ntile / (N / 8)) * 8;
+      for (int r = threadIdx.x % C::LT; r < N; r += C::LT) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + r * RS));
+    }
+    __syncthreads();  // the previous pair's exchange has been read (k = 0: twiddles)
+    uint32_t over[L::ITL][(L::EL + 7) / 8];  // four bits per output: field of mass i above its threshold
+#pragma unroll
+    for (int i = 0; i < L::ITL; ++i)
+#pragma unroll
+      for (int h = 0; h < (L::EL + 7) / 8; ++h) over[i][h] = 0u;
+    pair_line<L, true, 8>(v, ex, tw, t, sync, [&](int q, int m, int i, const cpair& u) {
+      const uint32_t o = (u.re.x > p0.thr_a ? 1u : 0u) | (u.im.x > p0.thr_b ? 2u : 0u) | (u.re.y > p1.thr_a ? 4u : 0u) |
+                         (u.im.y > p1.thr_b ? 8u : 0u);
+      over[i][m >> 3] |= o << (4 * (m & 7));
+    });
+#pragma unroll
+    for (int i = 0; i < L::ITL; ++i) {
+      const int q = t + i * L::T;
+      const bool mine = col == 0 && (L::QL % L::T == 0 || q < L::QL);
+#pragma unroll
+      for (int m = 0; m < L::EL; ++m) {
+        const uint32_t o = over[i][m >> 3] >> (4 * (m & 7));
+        const unsigned b0 = __ballot_sync(wmask, o & 1u), b1 = __ballot_sync(wmask, o & 2u);
+        const unsigned b2 = __ballot_sync(wmask, o & 4u), b3 = __ballot_sync(wmask, o & 8u);
+        if (mine) {
+          const long byte = (((long)(q + m * L::QL) * N + b) * N >> 3) + cb;  // 8 cells per byte
+          reinterpret_cast<uint8_t*>(p0.bits_a)[byte] = (uint8_t)(b0 >> lane);
+          if (p0.bits_b) reinterpret_cast<uint8_t*>(p0.bits_b)[byte] = (uint8_t)(b1 >> lane);
+          if (both) {
+            reinterpret_cast<uint8_t*>(p1.bits_a)[byte] = (uint8_t)(b2 >> lane);
+            if (p1.bits_b) reinterpret_cast<uint8_t*>(p1.bits_b)[byte] = (uint8_t)(b3 >> lane);
+          }
+        }
+      }
+    }
+  }
+}
+
 // ---- one natural-layout box: pairs of rows, pairs of columns ------------------------
 // The same lines on one complex box a N^2 + b N + c, the lanes being two rows
 // (2r, 2r + 1) or two adjacent columns.
@@ -690,7 +855,27 @@ struct PairLaunch {
       e = cudaFuncSetAttribute(k_pair_rows_adj<Row, S::RW, S::RR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)ADJ_ROW_SMEM);
     if (!e) e = nat_setup();
+    if (!e)
+      e = cudaFuncSetAttribute(k_pair_hf_rows<Row, S::RW, S::RR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)HF_ROW_SMEM);
+    if (!e)
+      e = cudaFuncSetAttribute(k_pair_hf_cols_a<Col, S::CR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)PairCol<Col, S::CR>::SMEM);
     return e;
+  }
+  // the halo finder's filter bank
+  static constexpr size_t HF_ROW_SMEM =
+      PairRow<Row, S::RW, S::RR>::SMEM + (size_t)S::RW * PairRow<Row, S::RW, S::RR>::WS * sizeof(float2);
+  static cudaError_t hf_rows(const float2* spec, const HfBatch& hb, const float2* tw, int nsm, cudaStream_t st) {
+    using R = PairRow<Row, S::RW, S::RR>;
+    const int ng = N * N / S::RW, most = nsm * R::PER_SM;
+    k_pair_hf_rows<Row, S::RW, S::RR><<<pair_min(ng, most), R::THREADS, HF_ROW_SMEM, st>>>(spec, hb, tw);
+    return cudaGetLastError();
+  }
+  static cudaError_t hf_cols_a(const HfBatch& hb, const float2* tw, int nsm, cudaStream_t st) {
+    using G = PairCol<Col, S::CR>;
+    k_pair_hf_cols_a<Col, S::CR><<<G::NTILES / G::TPC, G::THREADS, G::SMEM, st>>>(hb, tw, nsm * G::PER_SM);
+    return cudaGetLastError();
   }
   // one natural-layout box
   static constexpr size_t NAT_COL_SMEM = (size_t)N * 8 * sizeof(cpair) + Col::TW * sizeof(float2);
@@ -746,7 +931,7 @@ struct PairLaunch {
   static constexpr PairOps ops() {
     return {setup,       pair_rows_launch<Row, S::RW, S::RR>, cols_b,   cols_a_test,
             cols_a_crit, cols_a_adj,                          rows_adj, PairCol<Col, CRA>::NTILES / PairCol<Col, CRA>::TPC,
-            nat_rows,    nat_cols};
+            nat_rows,    nat_cols,                            hf_rows,  hf_cols_a};
   }
 };
 

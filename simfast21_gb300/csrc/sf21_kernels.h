@@ -112,6 +112,7 @@ cudaError_t launch_cols_a_test_cb(int N, const Batch& bt, uint8_t* rc, const flo
 // (r[k].work and r[k + 1].work consecutive; slot K holds the last radius again
 // when K is odd, with ridx < 0 for the adjoint).  tw: the plain table
 // exp(-2 pi i t / N).
+struct HfBatch;
 struct PairOps {  // the launches of one box side
   cudaError_t (*setup)();
   // c axis with the top-hat filter: spec -> the batch's pair boxes
@@ -136,6 +137,10 @@ struct PairOps {  // the launches of one box side
   cudaError_t (*nat_rows)(const float2* in, const float* real, const float* wax, float2* out, int ncol, bool inverse,
                           const float* alpha, const float2* tw, int nsm, cudaStream_t st);
   cudaError_t (*nat_cols)(float2* box, int axis, bool inverse, int ncol, const float2* tw, cudaStream_t st);
+  // the halo finder's filter bank, two transforms (p[k], p[k + 1]) per pair box
+  // at p[k].work; its b axis is cols_b of the same boxes
+  cudaError_t (*hf_rows)(const float2* spec, const HfBatch& hb, const float2* tw, int nsm, cudaStream_t st);
+  cudaError_t (*hf_cols_a)(const HfBatch& hb, const float2* tw, int nsm, cudaStream_t st);
 };
 const PairOps* pair_ops(int N);  // null: no pair kernels for this side
 
