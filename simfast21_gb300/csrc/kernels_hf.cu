@@ -463,37 +463,47 @@ __global__ void __launch_bounds__(1024) k_scan_counts(uint32_t* __restrict__ cnt
   if (threadIdx.x == 0) *tot = carry;
 }
 
+// A warp owns CMP_CHUNK / 8 words, 128 at a time, four per lane: whole lines,
+// all asked for before the first is used.  (Each thread reading 32 words of
+// its own: 36 us for the bits of 512^3 cells, bound by the lines' latency.)
 __global__ void __launch_bounds__(CMP_THREADS) k_bits_emit(const uint32_t* __restrict__ W, long nwords,
                                                            const uint32_t* __restrict__ off,
                                                            uint32_t* __restrict__ out) {
-  // thread t owns words w0 + t*CMP_WPT .. +CMP_WPT-1 (contiguous, keeps order)
-  const long w0 = blockIdx.x * CMP_CHUNK + (long)threadIdx.x * CMP_WPT;
-  uint32_t s = 0;
-  for (int k = 0; k < CMP_WPT; ++k)
-    if (w0 + k < nwords) s += __popc(__ldg(W + w0 + k));
-  // block exclusive scan of s
-  __shared__ uint32_t wsum[CMP_THREADS / 32];
+  constexpr int WARPS = CMP_THREADS / 32, IT = CMP_WPT / 4;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t x = s;
+  const long w0 = blockIdx.x * CMP_CHUNK + (long)w * (CMP_CHUNK / WARPS) + 4 * lane;
+  uint4 v[IT];  // nwords is a multiple of 16 (the side is one of 8)
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
+  for (int i = 0; i < IT; ++i)
+    v[i] = w0 + 128 * i < nwords ? __ldg(reinterpret_cast<const uint4*>(W + w0 + 128 * i)) : make_uint4(0, 0, 0, 0);
+  uint32_t n[IT], s = 0;
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    n[i] = __popc(v[i].x) + __popc(v[i].y) + __popc(v[i].z) + __popc(v[i].w);
+    s += n[i];
   }
-  if (lane == 31) wsum[w] = x;
+  __shared__ uint32_t wsum[WARPS];
+  s = __reduce_add_sync(0xffffffffu, s);
+  if (lane == 0) wsum[w] = s;
   __syncthreads();
-  uint32_t before = 0;
-  for (int k = 0; k < w; ++k) before += wsum[k];
-  uint32_t pos = off[blockIdx.x] + before + x - s;
-  for (int k = 0; k < CMP_WPT; ++k) {
-    const long wi = w0 + k;
-    if (wi >= nwords) break;
-    uint32_t m = __ldg(W + wi);
-    while (m) {
-      const int bit = __ffs(m) - 1;
-      out[pos++] = (uint32_t)(wi * 32 + bit);
-      m &= m - 1;
+  if (s == 0) return;
+  uint32_t pos = off[blockIdx.x];
+  for (int k = 0; k < w; ++k) pos += wsum[k];
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    if (!__any_sync(0xffffffffu, n[i])) continue;
+    uint32_t x = n[i];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
     }
+    uint32_t p = pos + x - n[i];
+    const uint32_t m4[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      for (uint32_t m = m4[k]; m; m &= m - 1) out[p++] = (uint32_t)((w0 + 128 * i + k) * 32 + __ffs(m) - 1);
+    pos += __shfl_sync(0xffffffffu, x, 31);
   }
 }
 
@@ -688,12 +698,23 @@ __global__ void k_hf_cell(long nwords, const float* __restrict__ delta, float tc
                           uint32_t* __restrict__ bits) {
   const int lane = threadIdx.x & 31;
   for (long w0 = warp_id_global() * 32; w0 < nwords; w0 += warps_total() * 32) {
+    // lane l's four cells of every group of 128: bits 4 (l & 7) .. of word l / 8
+    // of the group (nwords is a multiple of 16)
+    float4 d[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      d[i] = w0 + 4 * i < nwords ? __ldg(reinterpret_cast<const float4*>(delta + (w0 + 4 * i) * 32) + lane)
+                                 : make_float4(0.f, 0.f, 0.f, 0.f);
     uint32_t mine = 0;
-    for (int k = 0; k < 32; ++k) {
-      const long w = w0 + k;
-      if (w >= nwords) break;
-      const uint32_t m = __ballot_sync(0xffffffffu, delta[w * 32 + lane] >= tcell);
-      if (lane == k) mine = m;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      uint32_t m = (d[i].x >= tcell ? 1u : 0u) | (d[i].y >= tcell ? 2u : 0u) | (d[i].z >= tcell ? 4u : 0u) |
+                   (d[i].w >= tcell ? 8u : 0u);
+      m <<= 4 * (lane & 7);
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
+      m = __shfl_sync(0xffffffffu, m, 8 * (lane & 3));
+      if (lane / 4 == i) mine = m;
     }
     const long w = w0 + lane;
     if (w < nwords) {

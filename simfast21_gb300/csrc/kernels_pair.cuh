@@ -567,14 +567,29 @@ k_pair_hf_rows(const float2* __restrict__ spec, HfBatch hb, const float2* __rest
   }
 }
 
-// a axis + the four thresholds: one bit per cell and mass, a byte of the bit
-// sets per row of a tile.  The column blocks run fastest, so that the bytes of
-// a sector are written close together.
+// a axis + the four thresholds: one bit per cell and mass.  A CTA takes up to
+// four tiles in a row of cells, one after the other, and stores their bytes as
+// one word: with a byte per tile row the stores' sectors took as long as the
+// transform's exchanges (512^3, two transforms: 880 us; 550 us with words, the
+// radius passes' a axis with its test 520 us).  The bits of eight outputs and
+// four masses are gathered by one 8 x 8 transposition among the columns' lanes.
+
+// Tiles of eight columns that a CTA takes one after the other along a row of
+// the bit sets, to store their bytes as one word (whole words in every row)
+template <class C>
+__host__ __device__ constexpr int pair_hf_run() {
+  for (int j = 4; j > 1; j /= 2)
+    if (C::N / 8 % j == 0 && C::NTILES / j % C::TPC == 0) return j;
+  return 1;
+}
 template <class L, int REGS>
 __global__ void __launch_bounds__(PairCol<L, REGS>::THREADS, PairCol<L, REGS>::PER_SM)
 k_pair_hf_cols_a(HfBatch hb, const float2* __restrict__ plain, int ahead) {
   using C = PairCol<L, REGS>;
   constexpr int N = L::N;
+  constexpr int J = pair_hf_run<C>();
+  constexpr int NB = N / 8 / J;  // runs per row of the bit sets
+  constexpr int H = (L::EL + 7) / 8;
   extern __shared__ __align__(16) unsigned char psm[];
   cpair* exs = reinterpret_cast<cpair*>(psm);
   float2* tw = reinterpret_cast<float2*>(exs + C::TPC * N * 8);
@@ -582,60 +597,88 @@ k_pair_hf_cols_a(HfBatch hb, const float2* __restrict__ plain, int ahead) {
   const int sub = threadIdx.x / C::LT;
   const int col = threadIdx.x % 8;
   const int t = (threadIdx.x % C::LT) / 8;
-  const int tile = blockIdx.x * C::TPC + sub;
-  const int cb = tile % (N / 8), b = tile / (N / 8);
+  const int run = blockIdx.x * C::TPC + sub;
+  const int cb0 = run % NB * J, b = run / NB;
   cpair* ex = exs + sub * N * 8 + col;
-  constexpr long RS = (long)N * 8;
-  const long base = ((long)cb * N * N + b) * 8;
-  const int lane = threadIdx.x & 31;
+  constexpr long RS = (long)N * 8, CBS = (long)N * N * 8;
+  const long base = (long)cb0 * CBS + (long)b * 8;
   const unsigned wmask =
       C::THREADS % 32 && threadIdx.x / 32 == C::THREADS / 32 ? (1u << (C::THREADS % 32)) - 1u : 0xffffffffu;
   auto sync = [] { __syncthreads(); };
   for (int k = 0; k < hb.K; k += 2) {
     const HfPair &p0 = hb.p[k], &p1 = hb.p[k + 1];
-    const bool both = k + 1 < hb.K;
-    const cpair* box = reinterpret_cast<const cpair*>(p0.work) + base + col;
-    cpair v[L::IT1][L::E1];
+    uint32_t run_bits[4][L::ITL][H];  // mass, then the lane's output: its run's bytes, tile j in byte j
 #pragma unroll
-    for (int i = 0; i < L::IT1; ++i) {
-      const int q = t + i * L::T;
-      if (L::Q1 % L::T == 0 || q < L::Q1) {
+    for (int s = 0; s < 4; ++s)
 #pragma unroll
-        for (int m = 0; m < L::E1; ++m) v[i][m] = ld_pair(box + (q + m * L::Q1) * RS);
+      for (int i = 0; i < L::ITL; ++i)
+#pragma unroll
+        for (int h = 0; h < H; ++h) run_bits[s][i][h] = 0u;
+    for (int j = 0; j < J; ++j) {
+      const cpair* box = reinterpret_cast<const cpair*>(p0.work) + base + j * CBS + col;
+      cpair v[L::IT1][L::E1];
+#pragma unroll
+      for (int i = 0; i < L::IT1; ++i) {
+        const int q = t + i * L::T;
+        if (L::Q1 % L::T == 0 || q < L::Q1) {
+#pragma unroll
+          for (int m = 0; m < L::E1; ++m) v[i][m] = ld_pair(box + (q + m * L::Q1) * RS);
+        }
       }
-    }
-    const int ntile = tile + ahead * C::TPC;
-    if (ntile < C::NTILES) {  // a later tile's lines on their way into L2
-      const cpair* nx = reinterpret_cast<const cpair*>(p0.work) + ((long)(ntile % (N / 8)) * N * N + ntile / (N / 8)) * 8;
-      for (int r = threadIdx.x % C::LT; r < N; r += C::LT) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + r * RS));
-    }
-    __syncthreads();  // the previous pair's exchange has been read (k = 0: twiddles)
-    uint32_t over[L::ITL][(L::EL + 7) / 8];  // four bits per output: field of mass i above its threshold
+      const int nrun = run + ahead * C::TPC;
+      if (j + 1 < J || nrun < N * NB) {  // a later tile's lines on their way into L2
+        const cpair* nx = reinterpret_cast<const cpair*>(p0.work) +
+                          (j + 1 < J ? base + (j + 1) * CBS : (long)(nrun % NB * J) * CBS + (long)(nrun / NB) * 8);
+        for (int r = threadIdx.x % C::LT; r < N; r += C::LT)
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + r * RS));
+      }
+      __syncthreads();  // the previous tile's exchange has been read (the first: twiddles)
+      uint32_t over[L::ITL][H];  // bit 8 s + (m & 7) of word m / 8: output m of mass s above its threshold
 #pragma unroll
-    for (int i = 0; i < L::ITL; ++i)
+      for (int i = 0; i < L::ITL; ++i)
 #pragma unroll
-      for (int h = 0; h < (L::EL + 7) / 8; ++h) over[i][h] = 0u;
-    pair_line<L, true, 8>(v, ex, tw, t, sync, [&](int q, int m, int i, const cpair& u) {
-      const uint32_t o = (u.re.x > p0.thr_a ? 1u : 0u) | (u.im.x > p0.thr_b ? 2u : 0u) | (u.re.y > p1.thr_a ? 4u : 0u) |
-                         (u.im.y > p1.thr_b ? 8u : 0u);
-      over[i][m >> 3] |= o << (4 * (m & 7));
-    });
+        for (int h = 0; h < H; ++h) over[i][h] = 0u;
+      pair_line<L, true, 8>(v, ex, tw, t, sync, [&](int q, int m, int i, const cpair& u) {
+        const uint32_t o = (u.re.x > p0.thr_a ? 1u : 0u) | (u.im.x > p0.thr_b ? 1u << 8 : 0u) |
+                           (u.re.y > p1.thr_a ? 1u << 16 : 0u) | (u.im.y > p1.thr_b ? 1u << 24 : 0u);
+        over[i][m >> 3] |= o << (m & 7);
+      });
+#pragma unroll
+      for (int i = 0; i < L::ITL; ++i)
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          // the eight columns' lanes transpose the bits of eight outputs, all
+          // masses at once: then lane m has output 8 h + m, bit c is column c
+          uint32_t w = over[i][h];
+#pragma unroll
+          for (int s = 4; s > 0; s >>= 1) {
+            const uint32_t keep = s == 4 ? 0x0f0f0f0fu : s == 2 ? 0x33333333u : 0x55555555u;
+            const uint32_t x = __shfl_xor_sync(wmask, w, s);
+            w = col & s ? (w & ~keep) | ((x & ~keep) >> s) : (w & keep) | ((x & keep) << s);
+          }
+#pragma unroll
+          for (int s = 0; s < 4; ++s) run_bits[s][i][h] |= (w >> (8 * s) & 0xffu) << (8 * j);
+        }
+    }
 #pragma unroll
     for (int i = 0; i < L::ITL; ++i) {
       const int q = t + i * L::T;
-      const bool mine = col == 0 && (L::QL % L::T == 0 || q < L::QL);
 #pragma unroll
-      for (int m = 0; m < L::EL; ++m) {
-        const uint32_t o = over[i][m >> 3] >> (4 * (m & 7));
-        const unsigned b0 = __ballot_sync(wmask, o & 1u), b1 = __ballot_sync(wmask, o & 2u);
-        const unsigned b2 = __ballot_sync(wmask, o & 4u), b3 = __ballot_sync(wmask, o & 8u);
-        if (mine) {
-          const long byte = (((long)(q + m * L::QL) * N + b) * N >> 3) + cb;  // 8 cells per byte
-          reinterpret_cast<uint8_t*>(p0.bits_a)[byte] = (uint8_t)(b0 >> lane);
-          if (p0.bits_b) reinterpret_cast<uint8_t*>(p0.bits_b)[byte] = (uint8_t)(b1 >> lane);
-          if (both) {
-            reinterpret_cast<uint8_t*>(p1.bits_a)[byte] = (uint8_t)(b2 >> lane);
-            if (p1.bits_b) reinterpret_cast<uint8_t*>(p1.bits_b)[byte] = (uint8_t)(b3 >> lane);
+      for (int h = 0; h < H; ++h) {
+        const int m = 8 * h + col;
+        if ((L::QL % L::T == 0 || q < L::QL) && (L::EL % 8 == 0 || m < L::EL)) {
+          const long byte = (((long)(q + m * L::QL) * N + b) * N >> 3) + cb0;  // 8 cells per byte
+          auto put = [&](uint32_t* bits, uint32_t w) {
+            unsigned char* dst = reinterpret_cast<unsigned char*>(bits) + byte;
+            if constexpr (J == 4) *reinterpret_cast<uint32_t*>(dst) = w;
+            else if constexpr (J == 2) *reinterpret_cast<uint16_t*>(dst) = (uint16_t)w;
+            else *dst = (unsigned char)w;
+          };
+          put(p0.bits_a, run_bits[0][i][h]);
+          if (p0.bits_b) put(p0.bits_b, run_bits[1][i][h]);
+          if (k + 1 < hb.K) {
+            put(p1.bits_a, run_bits[2][i][h]);
+            if (p1.bits_b) put(p1.bits_b, run_bits[3][i][h]);
           }
         }
       }
@@ -874,7 +917,7 @@ struct PairLaunch {
   }
   static cudaError_t hf_cols_a(const HfBatch& hb, const float2* tw, int nsm, cudaStream_t st) {
     using G = PairCol<Col, S::CR>;
-    k_pair_hf_cols_a<Col, S::CR><<<G::NTILES / G::TPC, G::THREADS, G::SMEM, st>>>(hb, tw, nsm * G::PER_SM);
+    k_pair_hf_cols_a<Col, S::CR><<<G::NTILES / pair_hf_run<G>() / G::TPC, G::THREADS, G::SMEM, st>>>(hb, tw, nsm * G::PER_SM);
     return cudaGetLastError();
   }
   // one natural-layout box
