@@ -861,13 +861,13 @@ static int sg_tables(sf21_halo_ctx* c) {
     for (int cc = 0; cc < 3; ++cc) memcpy(&p2[((size_t)k * 3 + cc) * 32], m.col[cc], 128);
     m = taus_mul(m, m);
   }
-  const TausMat t1 = taus_one_step();
-  const TausMat t4 = taus_mul(taus_mul(t1, t1), taus_mul(t1, t1));
+  TausMat seg = taus_one_step();
+  for (int k = 1; k < SG_SEG; k *= 2) seg = taus_mul(seg, seg);
   TausMat acc = taus_identity();
   for (int i = 0; i < SG_LOCAL; ++i) {  // column-major over i (see kernels_sg.cu)
     for (int cc = 0; cc < 3; ++cc)
       for (int k = 0; k < 32; ++k) loc[((size_t)cc * 32 + k) * SG_LOCAL + i] = acc.col[cc][k];
-    acc = taus_mul(t4, acc);
+    acc = taus_mul(seg, acc);
   }
   HCTX_CUDA(c, dev_malloc(&c->d_sg_pow2, sizeof(uint32_t) * p2.size()));
   HCTX_CUDA(c, dev_malloc(&c->d_sg_local, sizeof(uint32_t) * loc.size()));
@@ -930,6 +930,8 @@ static int subgrid_cycle(sf21_halo_ctx* c, const Cosmo& cs, double z, double gro
       const double xt = floor(ldexp(emu, 32));
       a.x1 = xt >= 4294967295.0 ? 0xffffffffu : (uint32_t)xt;
       memcpy(&a.emu, &emu, 8);
+      a.lo = (float)(emu * (1.0 - 0x1p-15));
+      a.hi = (float)(emu * (1.0 + 0x1p-15));
       // positions to generate: the mean consumption (1 + mu) per draw plus a margin
       const double need = (double)U * (1.0 + dndm) + 12.0 * sqrt((double)U * (1.0 + dndm) * (1.0 + dndm)) + 8 * SG_B;
       long nblocks = (long)ceil(need / SG_B);
@@ -953,7 +955,7 @@ static int subgrid_cycle(sf21_halo_ctx* c, const Cosmo& cs, double z, double gro
           HCTX_CUDA(c, dev_malloc(&c->d_sgX, (size_t)nb * SG_LMAX));
           HCTX_CUDA(c, dev_malloc(&c->d_sgD, sizeof(uint16_t) * (size_t)nb * SG_LMAX));
           HCTX_CUDA(c, dev_malloc(&c->d_sg_cnt, sizeof(uint32_t) * (size_t)nb));
-          HCTX_CUDA(c, dev_malloc(&c->d_sg_start, sizeof(uint32_t) * 3 * (size_t)nb));
+          HCTX_CUDA(c, dev_malloc(&c->d_sg_start, sizeof(uint32_t) * 3 * (size_t)sg_padded(nb)));
           HCTX_CUDA(c, dev_malloc(&c->d_sgLB, sizeof(uint32_t) * (SG_B / 32) * (size_t)nb));
           HCTX_CUDA(c, dev_malloc(&c->sg_eb.gx, (size_t)ng * SG_LMAX));
           HCTX_CUDA(c, dev_malloc(&c->sg_eb.gd, sizeof(uint32_t) * (size_t)ng * SG_LMAX));

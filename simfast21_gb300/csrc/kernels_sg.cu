@@ -9,11 +9,12 @@
 // reproduces that stream exactly:
 //   A  per block of SG_B positions: the generator's state is jumped to the
 //      block (the generator is linear over GF(2): 32x32 bit matrices of its
-//      powers), each thread steps 4 consecutive positions, L(s) is computed
-//      for every position (one integer compare decides L = 1; longer chains
-//      multiply with the IEEE double rounding done in integers), and pointer
-//      jumping gives, for every entry
-//      offset e < SG_LMAX, the block's exit offset and draw count;
+//      powers), a warp's lanes step 32 consecutive positions each, L(s) is
+//      computed for every position (one integer compare decides L = 1; longer
+//      chains multiply in float, and with the IEEE double rounding done in
+//      integers where the float product is too close to exp(-mu)), and the
+//      segments' tables compose to, for every entry offset e < SG_LMAX, the
+//      block's exit offset and draw count;
 //   B  the entries of all blocks follow by composing those tables (groups of
 //      SG_G blocks, supergroups of SG_G groups, in parallel; the supergroups
 //      in order; then down to the groups and the blocks);
@@ -64,110 +65,194 @@ __device__ __forceinline__ void sg_bad(int* err, int site, uint64_t idx) {
 
 // A ------------------------------------------------------------------------
 // jumps: pow2[(k 3 + c) 32 + col] = column col of component c of T^(2^k)
-// (k < SG_POW2); local[(c 32 + col) SG_LOCAL + i] = the same of T^(4 i)
-// (i < SG_LOCAL), stored so that the threads of a warp, each applying its own
+// (k < SG_POW2); local[(c 32 + col) SG_LOCAL + i] = the same of T^(SG_SEG i)
+// (i < SG_LOCAL), stored so that the lanes of a warp, each applying its own
 // power, read consecutive words.  S0: the state whose next step gives
 // position 0.
 // The state at the start of every block, T^(b SG_B) S0: one thread per
-// (block, component), so the jumps of all blocks run in parallel instead of
-// keeping a block's other threads waiting.
+// component and run of SG_RUN blocks, the first by its bits, the others by
+// one T^SG_B each.
+constexpr int SG_RUN = 4;
+static_assert(SG_WARPS % SG_RUN == 0, "runs of blocks");
 __global__ void k_sg_start(SgArgs a, const uint32_t* __restrict__ pow2, long nblocks, uint32_t* __restrict__ start) {
   const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nblocks * 3) return;
-  const long b = t / 3;
+  if (t >= nblocks / SG_RUN * 3) return;
+  const long b = t / 3 * SG_RUN;
   const int c = (int)(t % 3);
   const uint64_t base = (uint64_t)b * SG_B;
   uint32_t v = a.s0[c];
   for (int k = 0; k < SG_POW2; ++k)
     if ((base >> k) & 1u) v = gf2_apply(pow2 + ((size_t)k * 3 + c) * 32, v);
-  start[t] = v;
+  for (int r = 0;; ++r) {
+    start[(b + r) * 3 + c] = v;
+    if (r + 1 == SG_RUN) break;
+    v = gf2_apply(pow2 + ((size_t)SG_LOG2B * 3 + c) * 32, v);
+  }
 }
 
+// Where word j of a segment's row lies: rows of 33 words, so that the lanes'
+// rows start on different banks; j may run on into the rows that follow.
+__device__ __forceinline__ int sg_at(int row, int j) { return row * 33 + j + (j >> 5); }
+
+// Draw length at a position whose first uniform exceeds exp(-mu), in the
+// reference's arithmetic (products in double).
+__device__ __noinline__ int sg_draw_exact(const uint32_t* sx, int row, int p, uint64_t emu_bits) {
+  const DMant emu = dm_from_bits(emu_bits);
+  DMant prod = dm_from_u32(sx[sg_at(row, p)]);
+  int L = 2;
+  for (; L <= SG_LMAX; ++L) {
+    const uint32_t xn = sx[sg_at(row, p + L - 1)];
+    if (xn == 0) break;  // a zero factor ends the draw
+    prod = dm_mul_u32(prod, xn);
+    if (dm_le(prod, emu)) break;
+  }
+  return L;
+}
+
+// One warp per block of SG_B positions, one lane per segment of SG_SEG = 32.
+//   1  each lane jumps to its segment and steps through it, the outputs into
+//      shared memory and the positions with L >= 2 into a mask;
+//   2  L at the positions of the mask, by products in float: their error is
+//      under 2 SG_LMAX 2^-24 = 2^-17 of the value, so a product outside
+//      (lo, hi) = exp(-mu) (1 -+ 2^-15) is on its side of exp(-mu) in double
+//      too, and only the others (one in 2^14) take sg_draw_exact;
+//   3  for every position of the mask, from the last back to the first: where
+//      the chain from it leaves the segment and after how many draws (between
+//      the positions of the mask every draw takes one uniform);
+//   4  the block's table: the chains of all SG_LMAX entries, two per lane, go
+//      through the segments until they have met (two or three segments, as a
+//      rule); for the rest every lane walks its own segment, from entry 0
+//      first and then from its neighbour's exit until nothing changes (the
+//      exits settle from the left, mostly after two or three rounds).
+// What bounds it: the integer pipe, about 17 operations per position for the
+// generator itself and 10 for the jump.  512^3 cells, mean 0.03 per cell (138 M
+// positions): 0.225 ms, 2.32 ms when every position took part in ten rounds of
+// pointer jumping in shared memory and four positions shared a jump.
 __global__ void __launch_bounds__(SG_THREADS)
-k_sg_len(SgArgs a, const uint32_t* __restrict__ start, const uint32_t* __restrict__ local, uint8_t* __restrict__ Lout,
-         uint32_t* __restrict__ LB, uint8_t* __restrict__ X, uint16_t* __restrict__ D, int* __restrict__ err) {
-  __shared__ uint32_t sx[SG_B + SG_LMAX];
-  __shared__ uint16_t nxt[SG_B], cnt[SG_B];
-  const long b = blockIdx.x;
-  const uint64_t base = (uint64_t)b * SG_B;
-  const uint32_t sS[3] = {__ldg(start + 3 * b), __ldg(start + 3 * b + 1), __ldg(start + 3 * b + 2)};
-  for (int pass = 0; pass < 2; ++pass) {
-    const int i0 = pass ? SG_B + 4 * threadIdx.x : 4 * threadIdx.x;
-    if (pass && 4 * (int)threadIdx.x >= SG_LMAX) break;
-    const uint32_t* J = local + i0 / 4;
-    uint32_t x = gf2_apply_strided(J, sS[0]), y = gf2_apply_strided(J + 32 * SG_LOCAL, sS[1]),
-             z = gf2_apply_strided(J + 64 * SG_LOCAL, sS[2]);
+k_sg_len(SgArgs a, long nblocks, const uint32_t* __restrict__ start, const uint32_t* __restrict__ local,
+         uint8_t* __restrict__ Lout, uint32_t* __restrict__ LB, uint8_t* __restrict__ X, uint16_t* __restrict__ D,
+         int* __restrict__ err) {
+  __shared__ uint32_t sx[(SG_WARPS * 32 + SG_LMAX / 32) * 33];
+  __shared__ uint32_t sl[SG_WARPS * 32 * 9];  // draw lengths, rows of 32 bytes and a word between
+  const int w = threadIdx.x / 32, lane = threadIdx.x % 32, row = threadIdx.x;
+  const long b = (long)blockIdx.x * SG_WARPS + w;
+  uint32_t mask = 0;
+  // the segments of the CTA's blocks, and (warp 0) those that its last draws run into
+  for (int pass = 0; pass < (w ? 1 : 2); ++pass) {
+    if (pass && lane >= SG_LMAX / 32) break;
+    const uint32_t* s = start + 3 * (pass ? b + SG_WARPS - 1 : b);
+    const uint32_t* J = local + (pass ? 32 + lane : lane);
+    const int r0 = pass ? SG_WARPS * 32 + lane : row;
+    uint32_t x = gf2_apply_strided(J, __ldg(s)), y = gf2_apply_strided(J + 32 * SG_LOCAL, __ldg(s + 1)),
+             z = gf2_apply_strided(J + 64 * SG_LOCAL, __ldg(s + 2));
+    uint32_t mk = 0;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
+    for (int r = 0; r < SG_SEG; ++r) {
       taus_step(x, y, z);
-      sx[i0 + r] = x ^ y ^ z;
+      const uint32_t u = x ^ y ^ z;
+      sx[r0 * 33 + r] = u;
+      // x <= X1 <=> u = x 2^-32 <= exp(-mu) <=> one uniform
+      if (u > a.x1) mk |= 1u << r;
     }
+    if (!pass) mask = mk;
   }
-  __syncthreads();
-  // L(s): x <= X1 <=> u = x 2^-32 <= exp(-mu) <=> one uniform
-  const DMant emu = dm_from_bits(a.emu);
-  uint32_t packed = 0;
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    const int i = 4 * threadIdx.x + r;
-    int L = 1;
-    const uint32_t xv = sx[i];
-    if (xv > a.x1) {  // u_0 > exp(-mu) > 0, so xv > 0
-      DMant prod = dm_from_u32(xv);
-      for (L = 2; L <= SG_LMAX; ++L) {
-        const uint32_t xn = sx[i + L - 1];
-        if (xn == 0) break;  // a zero factor ends the draw
-        prod = dm_mul_u32(prod, xn);
-        if (dm_le(prod, emu)) break;
-      }
-      if (L > SG_LMAX) {
-        atomicOr(err, 1);
-        L = SG_LMAX;
-      }
+  for (int k = 0; k < 8; ++k) sl[row * 9 + k] = 0x01010101u;
+  __syncthreads();
+  uint8_t* lrow = reinterpret_cast<uint8_t*>(sl + row * 9);
+  for (uint32_t m = mask; m; m &= m - 1) {
+    const int p = __ffs(m) - 1;
+    float prod = __uint2float_rn(sx[row * 33 + p]) * 0x1p-32f;
+    int L = 2;
+    for (; L <= SG_LMAX; ++L) {
+      prod *= __uint2float_rn(sx[sg_at(row, p + L - 1)]) * 0x1p-32f;
+      if (prod <= a.hi) break;
     }
-    packed |= (uint32_t)L << (8 * r);
-    nxt[i] = (uint16_t)(i + L);
-    cnt[i] = 1;
+    if (L > SG_LMAX || prod > a.lo) L = sg_draw_exact(sx, row, p, a.emu);
+    if (L > SG_LMAX) {
+      atomicOr(err, 1);
+      L = SG_LMAX;
+    }
+    lrow[p] = (uint8_t)L;
   }
-  reinterpret_cast<uint32_t*>(Lout + base)[threadIdx.x] = packed;
-  // bit set of the positions whose draw takes two uniforms or more (k >= 1):
-  // 4 bits per thread, 8 threads per word
-  uint32_t nib = 0;
-#pragma unroll
-  for (int r = 0; r < 4; ++r) nib |= (((packed >> (8 * r)) & 0xFFu) >= 2u ? 1u : 0u) << r;
-  uint32_t word = nib << (4 * (threadIdx.x & 7));
-  word |= __shfl_xor_sync(0xffffffffu, word, 1);
-  word |= __shfl_xor_sync(0xffffffffu, word, 2);
-  word |= __shfl_xor_sync(0xffffffffu, word, 4);
-  if ((threadIdx.x & 7) == 0) LB[(size_t)b * (SG_B / 32) + (threadIdx.x >> 3)] = word;
-  __syncthreads();
-  // pointer jumping: after log2(SG_B) rounds every chain has left the block
-  for (int round = 0; (1 << round) < SG_B; ++round) {
-    uint16_t nn[4], cc[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int i = 4 * threadIdx.x + r;
-      const int n = nxt[i];
-      if (n < SG_B) {
-        nn[r] = nxt[n];
-        cc[r] = (uint16_t)(cnt[i] + cnt[n]);
+  __syncthreads();  // the outputs have been read: the rows take the chains, exit | draws << 8
+  for (uint32_t m = mask; m;) {
+    const int p = 31 - __clz(m);
+    m ^= 1u << p;
+    const int n = p + lrow[p];
+    uint32_t v;
+    if (n >= SG_SEG) {
+      v = (uint32_t)(n - SG_SEG) | 1u << 8;
+    } else {
+      const uint32_t mm = mask & (0xffffffffu << n);
+      if (!mm) {
+        v = (uint32_t)(1 + SG_SEG - n) << 8;
       } else {
-        nn[r] = (uint16_t)n;
-        cc[r] = cnt[i];
+        const int q = __ffs(mm) - 1;
+        v = sx[row * 33 + q] + ((uint32_t)(1 + q - n) << 8);
       }
     }
-    __syncthreads();
+    sx[row * 33 + p] = v;
+  }
+  __syncwarp();
+  if (b >= nblocks) return;
+  uint32_t* Lw = reinterpret_cast<uint32_t*>(Lout + (uint64_t)b * SG_B);
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      nxt[4 * threadIdx.x + r] = nn[r];
-      cnt[4 * threadIdx.x + r] = cc[r];
+  for (int k = 0; k < 8; ++k) {
+    const int i = k * 32 + lane;
+    Lw[i] = sl[(w * 32 + i / 8) * 9 + i % 8];
+  }
+  LB[(size_t)b * (SG_B / 32) + lane] = mask;
+  // entry e of the segment in row r with mask mk: its exit in place of e, its draws added to c
+  auto walk = [&](int& e, uint32_t& c, uint32_t mk, int r) {
+    if (e >= SG_SEG) {
+      e -= SG_SEG;
+      return;
     }
-    __syncthreads();
+    const uint32_t mm = mk & (0xffffffffu << e);
+    if (!mm) {
+      c += (uint32_t)(SG_SEG - e);
+      e = 0;
+    } else {
+      const int p = __ffs(mm) - 1;
+      const uint32_t v = sx[r * 33 + p];
+      c += (uint32_t)(p - e) + (v >> 8);
+      e = (int)(v & 0xffu);
+    }
+  };
+  int e0 = lane, e1 = lane + 32, j = 0;
+  uint32_t c0 = 0, c1 = 0;
+  bool met = false;
+  while (j < 32 && !met) {
+    const uint32_t mk = __shfl_sync(0xffffffffu, mask, j);
+    walk(e0, c0, mk, w * 32 + j);
+    walk(e1, c1, mk, w * 32 + j);
+    ++j;
+    const int f = __shfl_sync(0xffffffffu, e0, 0);
+    met = __all_sync(0xffffffffu, e0 == f && e1 == f);
   }
-  if (threadIdx.x < SG_LMAX) {
-    X[(size_t)b * SG_LMAX + threadIdx.x] = (uint8_t)(nxt[threadIdx.x] - SG_B);
-    D[(size_t)b * SG_LMAX + threadIdx.x] = cnt[threadIdx.x];
+  if (j < 32) {  // all at entry e0 of segment j
+    int entry = lane == j ? e0 : 0, x;
+    uint32_t c;
+    for (int round = 0; round < 32; ++round) {
+      x = entry;
+      c = 0;
+      walk(x, c, mask, row);
+      int next = __shfl_up_sync(0xffffffffu, x, 1);
+      if (lane <= j) next = entry;
+      const bool same = __all_sync(0xffffffffu, next == entry);
+      entry = next;
+      if (same) break;
+    }
+    const uint32_t rest = __reduce_add_sync(0xffffffffu, lane >= j ? c : 0u);
+    c0 += rest;
+    c1 += rest;
+    e0 = e1 = __shfl_sync(0xffffffffu, x, 31);
   }
+  X[(size_t)b * SG_LMAX + lane] = (uint8_t)e0;
+  X[(size_t)b * SG_LMAX + 32 + lane] = (uint8_t)e1;
+  D[(size_t)b * SG_LMAX + lane] = (uint16_t)c0;
+  D[(size_t)b * SG_LMAX + 32 + lane] = (uint16_t)c1;
 }
 
 // B ------------------------------------------------------------------------
@@ -383,34 +468,60 @@ __global__ void __launch_bounds__(SC_THREADS) k_chunk_sum(const uint32_t* __rest
   }
 }
 
-// a and out may be the same array (in-place scans): no __restrict__ on
-// them, so every element is loaded before its slot is overwritten.
+// a and out may be the same array (in-place scans): no __restrict__ on them,
+// and a CTA's elements are all loaded before the first slot is overwritten.
+// A warp owns SC_CHUNK / 8 consecutive elements, 128 at a time, four per lane
+// (32 consecutive ones per thread: 46 us for the words of 512^3 cells, 8 us so).
 __global__ void __launch_bounds__(SC_THREADS) k_chunk_scan(const uint32_t* a, long n,
                                                            const uint32_t* __restrict__ off, uint32_t* out) {
-  // each thread scans SC_CHUNK / SC_THREADS consecutive elements
-  constexpr int PER = (int)(SC_CHUNK / SC_THREADS);
-  const long i0 = blockIdx.x * SC_CHUNK + (long)threadIdx.x * PER;
-  uint32_t s = 0;
-  for (int k = 0; k < PER; ++k)
-    if (i0 + k < n) s += a[i0 + k];
-  __shared__ uint32_t wsum[SC_THREADS / 32];
+  constexpr int WARPS = SC_THREADS / 32, IT = (int)(SC_CHUNK / SC_THREADS / 4);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t x = s;
+  const long i0 = blockIdx.x * SC_CHUNK + (long)w * (SC_CHUNK / WARPS) + 4 * lane;
+  uint4 v[IT];
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
+  for (int i = 0; i < IT; ++i) {
+    const long p = i0 + 128 * i;
+    if (p + 3 < n) {
+      v[i] = *reinterpret_cast<const uint4*>(a + p);
+    } else {
+      v[i].x = p < n ? a[p] : 0u;
+      v[i].y = p + 1 < n ? a[p + 1] : 0u;
+      v[i].z = p + 2 < n ? a[p + 2] : 0u;
+      v[i].w = 0u;
+    }
   }
-  if (lane == 31) wsum[w] = x;
+  uint32_t s = 0;
+#pragma unroll
+  for (int i = 0; i < IT; ++i) s += v[i].x + v[i].y + v[i].z + v[i].w;
+  __shared__ uint32_t wsum[WARPS];
+  s = __reduce_add_sync(0xffffffffu, s);
+  if (lane == 0) wsum[w] = s;
   __syncthreads();
-  uint32_t before = 0;
-  for (int k = 0; k < w; ++k) before += wsum[k];
-  uint32_t run = off[blockIdx.x] + before + x - s;
-  for (int k = 0; k < PER; ++k) {
-    if (i0 + k >= n) break;
-    const uint32_t v = a[i0 + k];
-    out[i0 + k] = run;
-    run += v;
+  uint32_t pos = off[blockIdx.x];
+  for (int k = 0; k < w; ++k) pos += wsum[k];
+#pragma unroll
+  for (int i = 0; i < IT; ++i) {
+    const uint32_t t = v[i].x + v[i].y + v[i].z + v[i].w;
+    uint32_t x = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    const long p = i0 + 128 * i;
+    uint4 r;
+    r.x = pos + x - t;
+    r.y = r.x + v[i].x;
+    r.z = r.y + v[i].y;
+    r.w = r.z + v[i].z;
+    if (p + 3 < n) {
+      *reinterpret_cast<uint4*>(out + p) = r;
+    } else {
+      if (p < n) out[p] = r.x;
+      if (p + 1 < n) out[p + 1] = r.y;
+      if (p + 2 < n) out[p + 2] = r.z;
+    }
+    pos += __shfl_sync(0xffffffffu, x, 31);
   }
 }
 
@@ -437,13 +548,15 @@ static unsigned grid_for(long n, int threads) {
 
 cudaError_t launch_sg_len(long nblocks, const SgArgs& a, const uint32_t* pow2, const uint32_t* local, uint32_t* start,
                           uint8_t* L, uint32_t* LB, uint8_t* X, uint16_t* D, int* err, cudaStream_t st) {
-  k_sg_start<<<(unsigned)((nblocks * 3 + 255) / 256), 256, 0, st>>>(a, pow2, nblocks, start);
+  const long padded = sg_padded(nblocks);
+  k_sg_start<<<(unsigned)((padded / SG_RUN * 3 + 255) / 256), 256, 0, st>>>(a, pow2, padded, start);
   cudaError_t e = cudaGetLastError();
   if (e) return e;
-  k_sg_len<<<(unsigned)nblocks, SG_THREADS, 0, st>>>(a, start, local, L, LB, X, D, err);
+  k_sg_len<<<(unsigned)(padded / SG_WARPS), SG_THREADS, 0, st>>>(a, nblocks, start, local, L, LB, X, D, err);
   return cudaGetLastError();
 }
 
+long sg_padded(long nblocks) { return (nblocks + SG_WARPS - 1) / SG_WARPS * SG_WARPS; }
 long sg_groups(long n) { return (n + SG_G - 1) / SG_G; }
 
 cudaError_t launch_sg_entries(const uint8_t* X, const uint16_t* D, long nblocks, const SgEntryBufs& eb,

@@ -264,17 +264,23 @@ cudaError_t launch_hf_records(const uint32_t* idx, long n, int N, float mass, fl
 
 // Subgrid Poisson cycle of the halo finder (kernels_sg.cu).
 constexpr int SG_B = 1024;               // stream positions per block
-constexpr int SG_THREADS = SG_B / 4;     // 4 consecutive positions per thread
+constexpr int SG_LOG2B = 10;
+constexpr int SG_SEG = SG_B / 32;        // consecutive positions per lane, a warp per block
+constexpr int SG_WARPS = 8;              // blocks per CTA
+constexpr int SG_THREADS = 32 * SG_WARPS;
 constexpr int SG_LMAX = 64;              // uniforms one draw may consume at most
 constexpr int SG_G = 64;                 // children per parent in the entry composition
 constexpr int SG_POW2 = 40;              // jump matrices T^(2^k), k < SG_POW2
-constexpr int SG_LOCAL = (SG_B + SG_LMAX) / 4;  // jump matrices T^(4 i), i < SG_LOCAL
+constexpr int SG_LOCAL = 32 + SG_LMAX / SG_SEG;  // jump matrices T^(SG_SEG i), i < SG_LOCAL
+static_assert(SG_B == 1 << SG_LOG2B && SG_SEG == 32 && SG_LMAX == 64, "k_sg_len's masks and entries");
 struct SgArgs {
   uint32_t s0[3];  // taus state before position 0
   uint32_t x1;     // one uniform suffices <=> its 32-bit draw <= x1 (= floor(exp(-mu) 2^32))
   uint64_t emu;    // exp(-mu), double bits
+  float lo, hi;    // exp(-mu) (1 -+ 2^-15)
 };
-// start: 3 words per block (the state at its first position); L: draw length
+long sg_padded(long nblocks);  // whole CTAs of blocks
+// start: 3 words per block of sg_padded(nblocks) (the state at its first position); L: draw length
 // per position; LB: SG_B/32 words per block, bit = draw length >= 2
 cudaError_t launch_sg_len(long nblocks, const SgArgs& a, const uint32_t* pow2, const uint32_t* local, uint32_t* start,
                           uint8_t* L, uint32_t* LB, uint8_t* X, uint16_t* D, int* err, cudaStream_t st);
