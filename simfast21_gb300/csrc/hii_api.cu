@@ -1458,7 +1458,7 @@ static int enqueue_halo_source(sf21_hii_ctx* c, double z, long nhalos, const voi
   if (c->N_halo < c->N) CTX_FAIL(c, SF21_E_ARG, "N_halo < N_smoothed (smooth_box, auxiliary.c:651-654)");
   if (nhalos >= (1L << 28)) CTX_FAIL(c, SF21_E_UNSUPPORTED, "2^28 halos or more (8 CIC entries each, int count)");
   const long nh3 = c->N_halo * c->N_halo * c->N_halo;
-  if (!c->d_fine) CTX_CUDA(c, dev_malloc(&c->d_fine, sizeof(float) * nh3));
+  if (!c->d_fine && !halo_by_tiles(c->N_halo, c->N)) CTX_CUDA(c, dev_malloc(&c->d_fine, sizeof(float) * nh3));
   if (nhalos > c->halo_cap) {
     if (c->d_halos) cudaFree(c->d_halos);
     if (c->d_hscratch) cudaFree(c->d_hscratch);
@@ -1467,7 +1467,7 @@ static int enqueue_halo_source(sf21_hii_ctx* c, double z, long nhalos, const voi
     c->halo_cap = 0;
     const long cap = nhalos + nhalos / 4 + 1024;
     CTX_CUDA(c, dev_malloc(&c->d_halos, (size_t)cap * 16));
-    c->hscratch_bytes = halo_scratch_bytes(cap);
+    c->hscratch_bytes = halo_scratch_bytes(cap, c->N_halo, c->N);
     CTX_CUDA(c, dev_malloc(&c->d_hscratch, c->hscratch_bytes));
     c->halo_cap = cap;
   }

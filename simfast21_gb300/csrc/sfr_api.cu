@@ -90,7 +90,7 @@ extern "C" int sf21_sfr_create(const sf21_sfr_config* cfg, sf21_sfr_ctx** out) {
   } while (0)
   SCREATE(cudaSetDevice(cfg->device));
   SCREATE(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-  SCREATE(dev_malloc(&c->d_fine, sizeof(float) * c->n3_halo));
+  if (!halo_by_tiles(cfg->N_halo, cfg->N_smoothed)) SCREATE(dev_malloc(&c->d_fine, sizeof(float) * c->n3_halo));
   SCREATE(dev_malloc(&c->d_out, sizeof(float) * c->n3));
 #undef SCREATE
   *out = c;
@@ -112,7 +112,7 @@ static int ensure_halo_cap(sf21_sfr_ctx* c, long nhalos) {
   long cap = nhalos + nhalos / 4 + 1024;
   if (cap >= (1L << 28)) cap = (1L << 28) - 1;
   SCTX_CUDA(c, dev_malloc(&c->d_halos, (size_t)cap * 16));
-  c->scratch_bytes = halo_scratch_bytes(cap);
+  c->scratch_bytes = halo_scratch_bytes(cap, c->cfg.N_halo, c->cfg.N_smoothed);
   SCTX_CUDA(c, dev_malloc(&c->d_scratch, c->scratch_bytes));
   c->halo_cap = cap;
   return SF21_OK;
