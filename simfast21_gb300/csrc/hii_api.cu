@@ -26,7 +26,6 @@
 #include <future>
 #include <string>
 #include <system_error>
-#include <thread>
 #include <vector>
 
 #include "../../include/sf21_hii.h"
@@ -144,6 +143,7 @@ struct sf21_hii_ctx {
   void* d_halos = nullptr;
   long halo_cap = 0;
   float* d_fine = nullptr;
+  double* d_neutral = nullptr;  // block sums of the sets' neutral fractions
   // power-spectrum buffers (allocated on first use)
   float2* d_pk = nullptr;
   float* d_pk_w = nullptr;
@@ -333,7 +333,7 @@ static void free_ctx(sf21_hii_ctx* c) {
   cudaSetDevice(c->device);
   void* ptrs[] = {c->d_delta, c->d_src, c->d_rec0, c->d_fres, c->d_partials, c->d_alpha,
                   c->d_xhii, c->d_spec, c->d_tw, c->d_twp, c->d_rc, c->d_mask, c->d_flag, c->d_box2,
-                  c->d_C, c->d_A, c->d_acc, c->d_zpart, c->d_g, c->d_gd, c->d_gs, c->d_halos, c->d_fine,
+                  c->d_C, c->d_A, c->d_acc, c->d_zpart, c->d_g, c->d_gd, c->d_gs, c->d_halos, c->d_fine, c->d_neutral,
                   c->d_hscratch, c->d_xhii2, c->d_pk, c->d_pk_w, c->d_pk_part, c->d_pk_sum,
                   c->d_pk_cnt, c->d_t21, c->d_t21_part};
   for (void* p : ptrs)
@@ -956,8 +956,8 @@ extern "C" int sf21_hii_run_z_device(sf21_hii_ctx* c, double z, int kind, const 
 // the host while the GPU works on the next set: set s is written into
 // staging box s mod 2 on the compute stream, copied out on the copy stream,
 // and the staging box is reused only after its copy has completed.  Each
-// set's neutral fraction is the serial double sum of the reference
-// (:473-477), on a host thread once the box has arrived.
+// set's neutral fraction (:473-477) is summed in double on the GPU before its
+// box leaves; the host adds the blocks' sums.
 static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, double* neutral) {
   const size_t bf = sizeof(float) * c->n3;
   if (!c->copy_stream) {
@@ -968,22 +968,21 @@ static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, doubl
     }
   }
   if (!c->d_xhii2) CTX_CUDA(c, dev_malloc(&c->d_xhii2, bf));
+  const int ns = (int)c->sets.size(), nb = neutral_blocks();
+  if (neutral && !c->d_neutral) CTX_CUDA(c, dev_malloc(&c->d_neutral, sizeof(double) * nb * ns));
+  std::vector<double> part(neutral ? (size_t)nb * ns : 0);
   float* stage[2] = {c->d_xhii, c->d_xhii2};
-  std::vector<std::thread> sums;
   int status = SF21_OK;
-  const int ns = (int)c->sets.size();
-  auto start_sum = [&](int s) {
-    if (!neutral) return;
-    const float* dst = xhii + (size_t)s * c->n3;
-    const long n3 = c->n3;
-    double* out = neutral + s;
-    sums.emplace_back([dst, n3, out]() {
-      double acc = 0.;
-      for (long i = 0; i < n3; ++i) acc += 1.0 - dst[i];
-      *out = acc / n3;
-    });
+  // a copy to pageable memory may keep this thread: it is issued when the next
+  // set's work is in the queue
+  auto copy_out = [&](int s) {
+    const int b = s & 1;
+    cudaError_t e = cudaStreamWaitEvent(c->copy_stream, c->ev_done[b], 0);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(xhii + (size_t)s * c->n3, stage[b], bf, cudaMemcpyDeviceToHost, c->copy_stream);
+    if (e == cudaSuccess) e = cudaEventRecord(c->ev_copied[b], c->copy_stream);
+    return e;
   };
-  int copied = 0;  // sets whose download has been waited for
   for (int s = 0; s < ns && status == SF21_OK; ++s) {
     const int b = s & 1;
     cudaError_t e = cudaSuccess;
@@ -991,40 +990,32 @@ static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, doubl
     if (e == cudaSuccess && (status = enqueue_radii(c, s, st)) == SF21_OK &&
         (status = enqueue_finish(c, s, c->d_src, stage[b], st)) == SF21_OK) {
       e = cudaEventRecord(c->ev_done[b], st);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(c->copy_stream, c->ev_done[b], 0);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(xhii + (size_t)s * c->n3, stage[b], bf, cudaMemcpyDeviceToHost, c->copy_stream);
-      if (e == cudaSuccess) e = cudaEventRecord(c->ev_copied[b], c->copy_stream);
-      // the previous set's box has been on its way while this set was enqueued
-      if (e == cudaSuccess && s >= 1) {
-        e = cudaEventSynchronize(c->ev_copied[(s - 1) & 1]);
-        if (e == cudaSuccess) start_sum(copied++);
-      }
+      if (e == cudaSuccess && neutral) e = launch_neutral(c->n3, stage[b], c->d_neutral + (size_t)s * nb, st);
+      if (e == cudaSuccess && s >= 1) e = copy_out(s - 1);
+      if (e == cudaSuccess && s + 1 == ns) e = copy_out(s);
     }
     if (e != cudaSuccess) {
       c->err = std::string("xHII download failed: ") + cudaGetErrorString(e);
       status = SF21_E_CUDA;
     }
   }
-  if (status == SF21_OK && copied < ns) {
-    cudaError_t e = cudaEventSynchronize(c->ev_copied[(ns - 1) & 1]);
-    if (e == cudaSuccess) {
-      start_sum(copied++);
-    } else {
-      c->err = std::string("xHII download failed: ") + cudaGetErrorString(e);
-      status = SF21_E_CUDA;
-    }
-  }
-  cudaStreamSynchronize(c->copy_stream);
-  for (std::thread& t : sums) t.join();
-  if (status == SF21_OK) {
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-      c->err = std::string("stream failed: ") + cudaGetErrorString(e);
-      status = SF21_E_CUDA;
-    }
+  cudaError_t e = cudaSuccess;
+  if (status == SF21_OK && neutral)
+    e = cudaMemcpyAsync(part.data(), c->d_neutral, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, st);
+  const cudaError_t ec = cudaStreamSynchronize(c->copy_stream), es = cudaStreamSynchronize(st);
+  for (cudaError_t x : {ec, es})
+    if (e == cudaSuccess) e = x;
+  if (status == SF21_OK && e != cudaSuccess) {
+    c->err = std::string("stream failed: ") + cudaGetErrorString(e);
+    status = SF21_E_CUDA;
   }
   if (status == SF21_OK) status = check_device_flag(c);
+  if (status == SF21_OK && neutral)
+    for (int s = 0; s < ns; ++s) {
+      double acc = 0.;
+      for (int k = 0; k < nb; ++k) acc += part[(size_t)s * nb + k];
+      neutral[s] = acc / c->n3;
+    }
   return status;
 }
 

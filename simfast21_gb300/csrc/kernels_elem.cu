@@ -162,4 +162,34 @@ cudaError_t launch_fill0(long n3, uint64_t zeta, const float* src, const float* 
   return cudaGetLastError();
 }
 
+// Neutral fraction: the sum of 1 - x.  Every thread adds the terms of its own
+// four columns in double, then the threads of a block as a tree, and the host
+// adds the 608 blocks: within (n3 / 600 000 + 620) 2^-53 of the sum, where a
+// serial sum is within n3 2^-53.  The serial sum on the host took 10 ms at
+// 256^3, one addition after the other; 12 us here, bound by the read.
+constexpr int NEU_THREADS = 256, NEU_BLOCKS = 608;
+__global__ void __launch_bounds__(NEU_THREADS) k_neutral(long n4, const float4* __restrict__ x, double* __restrict__ part) {
+  double s[4] = {0., 0., 0., 0.};
+  for (long i = (long)blockIdx.x * NEU_THREADS + threadIdx.x; i < n4; i += (long)NEU_BLOCKS * NEU_THREADS) {
+    const float4 v = __ldg(x + i);
+    s[0] += 1.0 - v.x;
+    s[1] += 1.0 - v.y;
+    s[2] += 1.0 - v.z;
+    s[3] += 1.0 - v.w;
+  }
+  __shared__ double sh[NEU_THREADS];
+  sh[threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
+  for (int o = NEU_THREADS / 2; o > 0; o >>= 1) {
+    __syncthreads();
+    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+  }
+  if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+}
+
+int neutral_blocks() { return NEU_BLOCKS; }
+cudaError_t launch_neutral(long n3, const float* x, double* part, cudaStream_t st) {
+  k_neutral<<<NEU_BLOCKS, NEU_THREADS, 0, st>>>(n3 / 4, reinterpret_cast<const float4*>(x), part);
+  return cudaGetLastError();
+}
+
 }  // namespace sf21

@@ -175,6 +175,10 @@ cudaError_t launch_grad_finish(long n3, const float2* G, const float* alpha, con
 cudaError_t launch_crit_init(long n3, float* C, uint8_t* A, cudaStream_t st);
 cudaError_t launch_crit_finalize(long n3, float* C, const uint8_t* A, cudaStream_t st);
 
+// Block sums of 1 - x in double (neutral_blocks() of them); n3 a multiple of 4
+int neutral_blocks();
+cudaError_t launch_neutral(long n3, const float* x, double* part, cudaStream_t st);
+
 // Halo-catalogue source box (kernels_halo.cu): CIC of Rion + block average,
 // bit-identical with the reference's serial loop.  halos_dev: nh records
 // {float Mass, x, y, z}; fine: N_halo^3 floats; out: N_smooth^3 floats.
