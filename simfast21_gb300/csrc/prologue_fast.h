@@ -348,7 +348,7 @@ SD_HD sd_t xhi_exact(sd_t r) {
   return sd_div(num, two_r);                                // /(2.*ratio)
 }
 
-// (float)XHI(ratio) for 2^-30 <= ratio < 2^-4.  With b = 2 ratio there 1 + b
+// (float)XHI(ratio) for 2^-30 <= ratio < 1/2.  Below 2^-4, with b = 2 ratio, 1 + b
 // and 1 + 2 b are exact doubles, and the reference's c = (1 + b)^2 rounded,
 // minus 4 ratio^2 = b^2 (exact), rounds back to exactly 1 + 2 b: the rounding
 // error of c is at most 2^-53, 1 + 2 b is a multiple of 2^-51.  So its
@@ -360,6 +360,11 @@ SD_HD sd_t xhi_exact(sd_t r) {
 // Then n 2^-52 / b, whose two roundings give the float unless the quotient
 // lies near a midpoint.  False: outside the range, n undecided (its fraction
 // within 64 units of one half), or the quotient in the guard band.
+// For 2^-4 <= ratio < 1/2 (b < 1), the bulk of a box from redshift 11 up, c
+// and c - 4 ratio^2 (< 4) are rounded by 2^-52 at most each and g by 2^-53, so
+// the numerator (exact, 2^-7.2 at least) is within 1.4 2^-52 of 1 + b - g, a
+// relative 2^-44.3, and the quotient is b u to that: the same u, and a guard
+// band of 2^-42 at least (256^3 at redshift 12, 60 % of the cells there: 1.9 -> 0.5 ms).
 SD_HD bool xhi_fast(float ratio, float* out) {
   union {
     float f;
@@ -367,9 +372,9 @@ SD_HD bool xhi_fast(float ratio, float* out) {
   } cv;
   cv.f = ratio;
   const int er = (int)(cv.u >> 23) - 127;  // a sign bit makes it large
-  if (er < -30 || er > -5) return false;
+  if (er < -30 || er > -2) return false;
   const uint64_t M = (cv.u & 0x7FFFFFu) | 0x800000u;
-  const int k = 22 - er;  // b = M 2^-k, 27 <= k <= 52
+  const int k = 22 - er;  // b = M 2^-k, 24 <= k <= 52
   const uint64_t M2 = M * M;
   const int s2 = 64 - 2 * k;
   const uint64_t B2 = s2 >= 0 ? M2 << s2 : M2 >> -s2;           // b^2, Q.64
@@ -383,6 +388,12 @@ SD_HD bool xhi_fast(float ratio, float* out) {
   U += (uint64_t)((int64_t)(int32_t)((float)(int32_t)(f >> 14) * g2) * 16384);
   f = (int64_t)((1ULL << 62) - sd_mulhi64(A - (sd_mulhi64(B2, U) >> 2), U));
   U += (uint64_t)(int64_t)(int32_t)((float)(int32_t)f * g2);
+  if (er > -5) {
+    const int lu = sd_clz64(U);
+    int eF = 24 - k - lu;
+    const uint64_t Fm = pf_mulnorm(M << 40, U << lu, &eF);
+    return pf_round_guard(Fm, eF, 0u, out, 1ULL << 22);
+  }
   const uint64_t V = sd_mulhi64(M2 << 16, U);                    // M^2 u 2^16; n = V 2^-(2k - 36)
   const int sh = 2 * k - 36;
   if (sh >= 64) {  // V < 2^63: n = 0
