@@ -23,6 +23,7 @@
 #include <stdlib.h>
 
 #include <atomic>
+#include <algorithm>
 #include <future>
 #include <string>
 #include <system_error>
@@ -143,6 +144,9 @@ struct sf21_hii_ctx {
   void* d_halos = nullptr;
   long halo_cap = 0;
   float* d_fine = nullptr;
+  unsigned int* d_done = nullptr;  // the prologue's finished blocks (zero between launches)
+  bool rc_clear = false;           // d_rc as the prologue left it
+  int K_launch = 0;                // radii per launch of the pair passes
   double* d_neutral = nullptr;  // block sums of the sets' neutral fractions
   // power-spectrum buffers (allocated on first use)
   float2* d_pk = nullptr;
@@ -333,7 +337,7 @@ static void free_ctx(sf21_hii_ctx* c) {
   cudaSetDevice(c->device);
   void* ptrs[] = {c->d_delta, c->d_src, c->d_rec0, c->d_fres, c->d_partials, c->d_alpha,
                   c->d_xhii, c->d_spec, c->d_tw, c->d_twp, c->d_rc, c->d_mask, c->d_flag, c->d_box2,
-                  c->d_C, c->d_A, c->d_acc, c->d_zpart, c->d_g, c->d_gd, c->d_gs, c->d_halos, c->d_fine, c->d_neutral,
+                  c->d_C, c->d_A, c->d_acc, c->d_zpart, c->d_g, c->d_gd, c->d_gs, c->d_halos, c->d_fine, c->d_neutral, c->d_done,
                   c->d_hscratch, c->d_xhii2, c->d_pk, c->d_pk_w, c->d_pk_part, c->d_pk_sum,
                   c->d_pk_cnt, c->d_t21, c->d_t21_part};
   for (void* p : ptrs)
@@ -395,6 +399,8 @@ static void pad_pair(const sf21_hii_ctx* c, Batch& bt) {
     bt.r[bt.K].work = c->d_work[bt.K];
   }
 }
+
+static bool use_pairs(const sf21_hii_ctx* c) { return c->pair && (c->gen || c->path == 5); }
 
 // The plain twiddle table of the pair passes.
 static const float2* pair_tw(const sf21_hii_ctx* c) { return c->gen ? c->d_tw : c->d_twp; }
@@ -489,12 +495,21 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
   if (po) CREATE_CUDA(po->setup());
   c->nat = po;
   if (c->gen ? (po && K > 1) : (cfg->path == 0 || cfg->path == 5)) c->pair = po;
-  const int Kw = c->pair ? K + (K & 1) : K;
+  // Small boxes take more radii to a launch, several to a grid row, while the
+  // boxes of all of them are well inside the L2: a launch takes 1.5 us and
+  // fills a part of the device.  64^3, 43 radii: 111 us with 8 to a launch,
+  // 101 with 24, 92 with 43; 96^3: 390 with 8 (57 MB), 393 with 16 (113 MB).
+  c->K_launch = K;
+  if (c->pair && cfg->kmax <= 0)
+    c->K_launch = (int)std::max<long>(K, std::min<long>(po->launch_radii, (104L << 20) / (long)box_c / KMAX * KMAX));
+  const int Kw = c->pair ? c->K_launch + (c->K_launch & 1) : K;
   c->d_work.assign(Kw, nullptr);
   CREATE_CUDA(dev_malloc(&c->d_work_base, box_c * Kw));
   for (int k = 0; k < Kw; ++k) c->d_work[k] = c->d_work_base + (size_t)k * c->n3;
   CREATE_CUDA(dev_malloc(&c->d_err, sizeof(int)));
   CREATE_CUDA(cudaMemset(c->d_err, 0, sizeof(int)));
+  CREATE_CUDA(dev_malloc(&c->d_done, sizeof(unsigned int)));
+  CREATE_CUDA(cudaMemset(c->d_done, 0, sizeof(unsigned int)));
   CREATE_CUDA(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device));
   c->pro_blocks = prologue_blocks(c->n3);
   CREATE_CUDA(dev_malloc(&c->d_partials, sizeof(float) * 2 * c->pro_blocks));
@@ -547,7 +562,7 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
     free_ctx(c);
     return SF21_E_UNSUPPORTED;
   }
-  c->path = want ? want : 1;
+  c->path = want ? want : c->pair && !c->gen ? 5 : 1;
   // a tuning result cached for this device, box size and batch size skips the timing
   // Autotuner: the radius pipeline and the radii per spectrum read K.  For
   // each candidate K (the cap, and 6 and 4 below it unless the caller fixed
@@ -632,8 +647,12 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
     }
     if (t0) cudaEventDestroy(t0);
     if (t1) cudaEventDestroy(t1);
-    c->path = best_path;
-    c->K = best_K;
+    if (c->K_launch <= K) {
+      c->path = best_path;
+      c->K = best_K;
+    } else {
+      c->path = 5;  // the timings are of one batch to a launch
+    }
     if (best_per_radius < 1e29)
       for (int p = 0; p <= NPATH; ++p) c->tune_ms[p] = best_ms[p];
   }
@@ -730,9 +749,8 @@ static int enqueue_front(sf21_hii_ctx* c, double z, int kind, const float* delta
   memset(&none, 0, sizeof(none));
   int e0 = mark(c, st);
   CTX_CUDA(c, launch_prologue(c->n3, delta, src, c->pa, c->d_rec0, c->d_fres, packed, c->d_partials,
-                              c->pro_blocks, st));
-  int e1 = mark(c, st);
-  CTX_CUDA(c, launch_alpha(c->d_partials, c->pro_blocks, c->d_alpha, st));
+                              c->pro_blocks, c->d_rc, c->d_done, c->d_alpha, st));
+  c->rc_clear = true;
   int e2 = mark(c, st);
   CTX_CUDA(c, x_fwd_rows(c, packed, c->d_spec, c->d_alpha, st));
   int e3 = mark(c, st);
@@ -740,8 +758,7 @@ static int enqueue_front(sf21_hii_ctx* c, double z, int kind, const float* delta
   int e4 = mark(c, st);
   CTX_CUDA(c, x_cols(c, c->d_spec, none, 1, 0, false, st));
   int e5 = mark(c, st);
-  span(c, KD_PRO, e0, e1);
-  span(c, KD_ALPHA, e1, e2);
+  span(c, KD_PRO, e0, e2);
   span(c, KD_FROWS, e2, e3);
   span(c, KD_FCB, e3, e4);
   span(c, KD_FCA, e4, e5);
@@ -772,7 +789,7 @@ static int enqueue_batch(sf21_hii_ctx* c, const Batch& bt, cudaStream_t st) {
     span(c, KD_FUSED, e1, e2);
     return SF21_OK;
   }
-  if (c->pair && (c->gen || c->path == 5)) {  // three axis passes over pairs of radii
+  if (use_pairs(c)) {  // three axis passes over pairs of radii
     const float2* tw = pair_tw(c);
     int e0 = mark(c, st);
     CTX_CUDA(c, c->pair->rows_filter(c->d_spec, bt, tw, c->nsm, st));
@@ -840,13 +857,15 @@ static int enqueue_batch(sf21_hii_ctx* c, const Batch& bt, cudaStream_t st) {
 static int enqueue_radii(sf21_hii_ctx* c, int set, cudaStream_t st) {
   const SetInfo& s = c->sets[set];
   int rc;
-  CTX_CUDA(c, cudaMemsetAsync(c->d_rc, RC_NONE, c->n3, st));
+  if (!c->rc_clear) CTX_CUDA(c, cudaMemsetAsync(c->d_rc, RC_NONE, c->n3, st));
+  c->rc_clear = false;
   if (c->path == 8) CTX_CUDA(c, cudaMemsetAsync(c->d_rc32, 0xFF, sizeof(unsigned int) * c->n3, st));
   const int nr = (int)s.R.size();
-  for (int k0 = 0; k0 < nr; k0 += c->K) {
+  const int per = use_pairs(c) && c->K_launch > c->K ? c->K_launch : c->K;
+  for (int k0 = 0; k0 < nr; k0 += per) {
     Batch bt;
     memset(&bt, 0, sizeof(bt));
-    bt.K = nr - k0 < c->K ? nr - k0 : c->K;
+    bt.K = nr - k0 < per ? nr - k0 : per;
     bt.set = set;
     bt.zmul = (float)s.fesc;
     for (int k = 0; k < bt.K; ++k) {

@@ -355,9 +355,11 @@ cudaError_t dt_setup(int N) {
 }
 
 // whole warps (the block reduction shuffles over all 32 lanes of every warp;
-// threads past the last strip only load and reduce)
+// threads past the last strip only load and reduce: two for every strip's one,
+// up to 256, since the small tiles wait for their loads)
 static int dt_threads(int N) {
   int t = N * dt_cols(N) / 8;
+  if (t < 256) t = 2 * t < 256 ? 2 * t : 256;
   t = (t + 31) / 32 * 32;
   return t < DT_THREADS ? t : DT_THREADS;
 }

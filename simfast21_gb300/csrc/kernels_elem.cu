@@ -23,10 +23,50 @@ __device__ __forceinline__ sd_t src_chain(float s, const PrologueArgs& pa) {
 
 constexpr int PRO_THREADS = 256;
 
+// alpha = 2^round(log2(|rec| / |ion|)), so that the two halves of the packed
+// transform have comparable norms.  An ionisation box that is zero in every
+// cell gets alpha = -1: the reference's filtered ionisation field is then
+// exactly zero and no cell is a centre (its test wants ion_R > 0,
+// get_HIIbubbles.c:339-348), while the packed transform's imaginary half
+// holds rounding cross-talk from the recombination half; is_centre reads
+// alpha <= 0 as "no centre", and the other users take |alpha|.
+// By the prologue's last block to finish (a launch of its own took as long as
+// a small box's whole pass), over all blocks' partial sums in their order.
+__device__ __forceinline__ void alpha_of(const float* partials, int nblocks, float* __restrict__ alpha) {
+  __shared__ float sa[PRO_THREADS], sb[PRO_THREADS];
+  float a = 0.f, b = 0.f;
+  for (int i = threadIdx.x; i < nblocks; i += PRO_THREADS) {
+    a += __ldcg(partials + 2 * i);
+    b += __ldcg(partials + 2 * i + 1);
+  }
+  sa[threadIdx.x] = a;
+  sb[threadIdx.x] = b;
+  __syncthreads();
+  for (int s = PRO_THREADS / 2; s > 0; s >>= 1) {
+    if (threadIdx.x < s) {
+      sa[threadIdx.x] += sa[threadIdx.x + s];
+      sb[threadIdx.x] += sb[threadIdx.x + s];
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    float r = 1.0f;
+    if (sb[0] == 0.f) {
+      r = -1.0f;
+    } else if (sa[0] > 0.f && sb[0] > 0.f && isfinite(sa[0]) && isfinite(sb[0])) {
+      float e = rintf(0.5f * log2f(sa[0] / sb[0]));
+      e = fminf(fmaxf(e, -60.f), 60.f);
+      r = exp2f(e);
+    }
+    *alpha = r;
+  }
+}
+
 __global__ void __launch_bounds__(PRO_THREADS)
 k_prologue(long n3, const float* __restrict__ delta, const float* __restrict__ src,
            const PrologueArgs pa, float* __restrict__ rec0, float* __restrict__ fres,
-           float2* __restrict__ packed, float* __restrict__ partials) {
+           float2* __restrict__ packed, float* partials, uint8_t* __restrict__ rc, unsigned int* __restrict__ done,
+           float* __restrict__ alpha) {
   // rrec_quick's tables: lanes index them by their own densities
   __shared__ uint64_t tab[384];
   for (int t = threadIdx.x; t < 384; t += blockDim.x) tab[t] = rrec_table(t);
@@ -57,6 +97,7 @@ k_prologue(long n3, const float* __restrict__ delta, const float* __restrict__ s
     rec0[i] = rr;
     fres[i] = fx;
     packed[i] = make_float2(rr, h1);
+    rc[i] = RC_NONE;
     sd2 += rr * rr;
     sh2 += h1 * h1;
     nz |= (h1 != 0.0f);
@@ -85,6 +126,15 @@ k_prologue(long n3, const float* __restrict__ delta, const float* __restrict__ s
     partials[2 * blockIdx.x] = a;
     partials[2 * blockIdx.x + 1] = b;
   }
+  __shared__ bool last;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(done, 1u) + 1 == gridDim.x;
+    if (last) *done = 0;  // for the next launch on the stream
+    __threadfence();
+  }
+  __syncthreads();
+  if (last) alpha_of(partials, gridDim.x, alpha);
 }
 
 int prologue_blocks(long n3) {
@@ -93,51 +143,9 @@ int prologue_blocks(long n3) {
 }
 
 cudaError_t launch_prologue(long n3, const float* delta, const float* src, const PrologueArgs& pa,
-                            float* rec0, float* fres, float2* packed, float* partials, int nblocks,
-                            cudaStream_t st) {
-  k_prologue<<<nblocks, PRO_THREADS, 0, st>>>(n3, delta, src, pa, rec0, fres, packed, partials);
-  return cudaGetLastError();
-}
-
-// alpha = 2^round(log2(|rec| / |ion|)), so that the two halves of the packed
-// transform have comparable norms.  An ionisation box that is zero in every
-// cell gets alpha = -1: the reference's filtered ionisation field is then
-// exactly zero and no cell is a centre (its test wants ion_R > 0,
-// get_HIIbubbles.c:339-348), while the packed transform's imaginary half
-// holds rounding cross-talk from the recombination half; is_centre reads
-// alpha <= 0 as "no centre", and the other users take |alpha|.
-__global__ void k_alpha(const float* __restrict__ partials, int nblocks, float* __restrict__ alpha) {
-  __shared__ float sa[256], sb[256];
-  float a = 0.f, b = 0.f;
-  for (int i = threadIdx.x; i < nblocks; i += blockDim.x) {
-    a += partials[2 * i];
-    b += partials[2 * i + 1];
-  }
-  sa[threadIdx.x] = a;
-  sb[threadIdx.x] = b;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      sa[threadIdx.x] += sa[threadIdx.x + s];
-      sb[threadIdx.x] += sb[threadIdx.x + s];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    float r = 1.0f;
-    if (sb[0] == 0.f) {
-      r = -1.0f;
-    } else if (sa[0] > 0.f && sb[0] > 0.f && isfinite(sa[0]) && isfinite(sb[0])) {
-      float e = rintf(0.5f * log2f(sa[0] / sb[0]));
-      e = fminf(fmaxf(e, -60.f), 60.f);
-      r = exp2f(e);
-    }
-    *alpha = r;
-  }
-}
-
-cudaError_t launch_alpha(const float* partials, int nblocks, float* alpha, cudaStream_t st) {
-  k_alpha<<<1, 256, 0, st>>>(partials, nblocks, alpha);
+                            float* rec0, float* fres, float2* packed, float* partials, int nblocks, uint8_t* rc,
+                            unsigned int* done, float* alpha, cudaStream_t st) {
+  k_prologue<<<nblocks, PRO_THREADS, 0, st>>>(n3, delta, src, pa, rec0, fres, packed, partials, rc, done, alpha);
   return cudaGetLastError();
 }
 

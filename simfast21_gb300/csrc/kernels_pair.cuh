@@ -35,6 +35,24 @@ struct PairCol {
                                                      (int)(230000 / (SMEM + 1024))));
 };
 
+// Largest side whose radii may go to several grid rows.  Larger boxes fill the
+// device with one row, and the code that lets rows meet costs them registers
+// (96^3: 390 -> 411 us with it in the kernels).
+constexpr int PAIR_MULTI_N = 80;
+// The kernels' argument: the 1 KB of RADII_MAX entries only where they are used
+// (it costs a launch 2 us)
+template <int N>
+using PairBatch = BatchOf<N <= PAIR_MULTI_N ? RADII_MAX : KMAX>;
+template <int N>
+PairBatch<N> pair_batch(const Batch& bt) {
+  PairBatch<N> b;
+  b.K = bt.K;
+  b.set = bt.set;
+  b.zmul = bt.zmul;
+  for (int k = 0; k < (int)(sizeof(b.r) / sizeof(b.r[0])); ++k) b.r[k] = bt.r[k];
+  return b;
+}
+
 // Rows: RW rows per CTA.
 template <class L, int RW_, int REGS>
 struct PairRow {
@@ -58,7 +76,8 @@ struct PairRow {
 // memory.
 template <class L, int RW, int REGS>
 __global__ void __launch_bounds__(PairRow<L, RW, REGS>::THREADS, PairRow<L, RW, REGS>::PER_SM)
-k_pair_rows_filter(const float2* __restrict__ spec, Batch bt, const float2* __restrict__ plain) {
+k_pair_rows_filter(const float2* __restrict__ spec, const __grid_constant__ PairBatch<L::N> bt, int per,
+                   const float2* __restrict__ plain) {
   using R = PairRow<L, RW, REGS>;
   constexpr int N = L::N;
   extern __shared__ __align__(16) unsigned char psm[];
@@ -84,6 +103,8 @@ k_pair_rows_filter(const float2* __restrict__ spec, Batch bt, const float2* __re
       }
     }
   };
+  constexpr bool MULTI = N <= PAIR_MULTI_N;  // this grid row's radii
+  const int k0 = MULTI ? blockIdx.y * per : 0, k1 = MULTI ? min(bt.K, k0 + per) : bt.K;
   pair_tw_load<L>(tw, plain);
   __syncthreads();
   for (int group = blockIdx.x; group < NG; group += gridDim.x) {
@@ -104,7 +125,7 @@ k_pair_rows_filter(const float2* __restrict__ spec, Batch bt, const float2* __re
     if (group + gridDim.x < NG)  // the next group's rows on their way into L2
       for (int i = threadIdx.x; i < RW * N / 16; i += R::THREADS)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(spec + (long)(group + gridDim.x) * RW * N + 16 * i));
-    for (int k = 0; k < bt.K; k += 2) {
+    for (int k = k0; k < k1; k += 2) {
       const float d0 = bt.r[k].dkR, d1 = bt.r[k + 1].dkR;
 #pragma unroll
       for (int i = 0; i < R::NW; ++i) {
@@ -151,7 +172,7 @@ k_pair_rows_filter(const float2* __restrict__ spec, Batch bt, const float2* __re
 // lines are asked into L2 a pair ahead.
 template <class L, bool INV, int EPI, int REGS>
 __global__ void __launch_bounds__(PairCol<L, REGS>::THREADS, PairCol<L, REGS>::PER_SM)
-k_pair_cols(Batch bt, uint8_t* __restrict__ rc, float* __restrict__ Cbuf, const float* __restrict__ alpha_ptr,
+k_pair_cols(const __grid_constant__ PairBatch<L::N> bt, int per, uint8_t* __restrict__ rc, float* __restrict__ Cbuf, const float* __restrict__ alpha_ptr,
             const float2* __restrict__ plain, int ahead) {
   using C = PairCol<L, REGS>;
   constexpr int N = L::N;
@@ -169,7 +190,7 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, float* __restrict__ Cbuf, const 
   float alpha = 0.0f;
   if (EPI >= 1) alpha = *alpha_ptr;
   auto sync = [] { __syncthreads(); };
-  // EPI 1: bit 8 (m & 3) + k of hit[m / 4]: output m is a centre at radius k of
+  // EPI 1: bit 8 (m & 3) + k - k0 of hit[m / 4]: output m is a centre at radius k of
   // the batch (radius indices increase with k: the lowest bit is the first hit)
   constexpr int HW = (L::EL + 3) / 4;
   uint32_t hit[EPI >= 1 ? L::ITL : 1][HW];
@@ -185,7 +206,9 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, float* __restrict__ Cbuf, const 
     for (int m = 0; m < L::EL; ++m) best[i][m] = -INFINITY;
   // no source anywhere (alpha < 0): ion_R is exactly zero
   const float crit_zeta = alpha > 0.0f ? bt.zmul : 0.0f, crit_alpha = fabsf(alpha);
-  for (int k = 0; k < bt.K; k += 2) {
+  constexpr bool MULTI = N <= PAIR_MULTI_N;  // this grid row's radii
+  const int k0 = MULTI ? blockIdx.y * per : 0, k1 = MULTI ? min(bt.K, k0 + per) : bt.K;
+  for (int k = k0; k < k1; k += 2) {
     cpair* box = reinterpret_cast<cpair*>(bt.r[k].work) + base;
     cpair v[L::IT1][L::E1];
 #pragma unroll
@@ -198,10 +221,10 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, float* __restrict__ Cbuf, const 
       }
     }
     if (ahead > 0) {  // the next pair's lines on their way into L2 (the last pair: those of a tile that comes later)
-      const bool more = k + 2 < bt.K;
+      const bool more = k + 2 < k1;
       const int ntile = tile + (more ? 0 : ahead * C::TPC);
       if (ntile < C::NTILES) {
-        const cpair* nx = reinterpret_cast<const cpair*>(bt.r[more ? k + 2 : 0].work) +
+        const cpair* nx = reinterpret_cast<const cpair*>(bt.r[more ? k + 2 : k0].work) +
                           (EPI >= 1 ? ((long)(ntile / N) * N * N + ntile % N) * 8 : (long)ntile * N * 8);
         for (int r = threadIdx.x % C::LT; r < N; r += C::LT)
           asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + r * RS));
@@ -209,7 +232,7 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, float* __restrict__ Cbuf, const 
     }
     __syncthreads();  // the previous pair's exchange has been read (k = 0: twiddles)
     const float2 al2 = dup2(alpha), zm2 = dup2(bt.zmul);
-    const uint32_t bit = 1u << k;
+    const uint32_t bit = 1u << (k - k0);
     pair_line<L, INV, 8>(v, ex, tw, t, sync, [&](int q, int m, int i, const cpair& u) {
       if constexpr (EPI == 0) {
         st_pair(box + (q + m * L::QL) * RS, u);
@@ -261,6 +284,40 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, float* __restrict__ Cbuf, const 
     for (int i = 0; i < L::ITL; ++i) {
       const int q = t + i * L::T;
       if (L::QL % L::T == 0 || q < L::QL) {
+        if constexpr (N <= PAIR_MULTI_N) {
+          if (gridDim.y > 1) {
+            // several grid rows meet in a cell: four lanes' bytes to a word, the
+            // smaller of each by compare-and-swap, all words' first tries (no
+            // hit yet) in flight together
+            const unsigned lanes = 0xFFu << (threadIdx.x & 24);
+            uint32_t w[L::EL], seen[L::EL];
+            uint32_t* dst = reinterpret_cast<uint32_t*>(rc + ((long)q * N + b) * N + (c & ~3));
+            constexpr long MS = (long)L::QL * N * N / 4;
+#pragma unroll
+            for (int m = 0; m < L::EL; ++m) {
+              const uint32_t byte = (hit[i][m >> 2] >> (8 * (m & 3))) & 0xFFu;
+              const uint32_t none = ~(0xFFu << (8 * (col & 3)));
+              w[m] = byte ? none | (uint32_t)(bt.r[k0].ridx + __ffs(byte) - 1) << (8 * (col & 3)) : 0xFFFFFFFFu;
+              w[m] &= __shfl_xor_sync(lanes, w[m], 1);
+              w[m] &= __shfl_xor_sync(lanes, w[m], 2);
+              if (col & 3) w[m] = 0xFFFFFFFFu;
+            }
+#pragma unroll
+            for (int m = 0; m < L::EL; ++m)
+              seen[m] = w[m] != 0xFFFFFFFFu ? atomicCAS(dst + m * MS, 0xFFFFFFFFu, w[m]) : 0xFFFFFFFFu;
+#pragma unroll
+            for (int m = 0; m < L::EL; ++m) {
+              uint32_t old = seen[m];
+              if (old == 0xFFFFFFFFu) continue;  // nothing to write, or written
+              for (uint32_t now = __vminu4(old, w[m]); now != old; now = __vminu4(old, w[m])) {
+                const uint32_t s = atomicCAS(dst + m * MS, old, now);
+                if (s == old) break;
+                old = s;
+              }
+            }
+            continue;
+          }
+        }
         // all the reads first (independent), then the updates; the radius
         // indices of a batch are consecutive
         uint32_t old[L::EL];
@@ -272,7 +329,7 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, float* __restrict__ Cbuf, const 
 #pragma unroll
         for (int m = 0; m < L::EL; ++m) {
           const uint32_t byte = (hit[i][m >> 2] >> (8 * (m & 3))) & 0xFFu;
-          const uint32_t h = (uint32_t)(bt.r[0].ridx + __ffs(byte) - 1);
+          const uint32_t h = (uint32_t)(bt.r[k0].ridx + __ffs(byte) - 1);
           if (byte && h < old[m]) rc[((long)(q + m * L::QL) * N + b) * N + c] = (uint8_t)h;
         }
       }
@@ -287,7 +344,7 @@ k_pair_cols(Batch bt, uint8_t* __restrict__ rc, float* __restrict__ Cbuf, const 
 // fills an odd batch) takes no voxel.
 template <class L, int REGS>
 __global__ void __launch_bounds__(PairCol<L, REGS>::THREADS, PairCol<L, REGS>::PER_SM)
-k_pair_cols_a_adj(Batch bt, const float* __restrict__ g, const uint8_t* __restrict__ Abuf,
+k_pair_cols_a_adj(const __grid_constant__ PairBatch<L::N> bt, const float* __restrict__ g, const uint8_t* __restrict__ Abuf,
                   const float* __restrict__ alpha_ptr, float* __restrict__ zpart, const float2* __restrict__ plain) {
   using C = PairCol<L, REGS>;
   constexpr int N = L::N;
@@ -391,7 +448,7 @@ k_pair_cols_a_adj(Batch bt, const float* __restrict__ g, const uint8_t* __restri
 // (k_rows_adj_acc).  The windows of a row lie in two buffers used in turn.
 template <class L, int RW, int REGS>
 __global__ void __launch_bounds__(PairRow<L, RW, REGS>::THREADS, PairRow<L, RW, REGS>::PER_SM)
-k_pair_rows_adj(Batch bt, float2* __restrict__ acc, const float2* __restrict__ plain) {
+k_pair_rows_adj(const __grid_constant__ PairBatch<L::N> bt, float2* __restrict__ acc, const float2* __restrict__ plain) {
   using R = PairRow<L, RW, REGS>;
   constexpr int N = L::N;
   extern __shared__ __align__(16) unsigned char psm[];
@@ -851,11 +908,20 @@ cudaError_t pair_rows_setup() {
   return cudaFuncSetAttribute(k_pair_rows_filter<L, RW, REGS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)PairRow<L, RW, REGS>::SMEM);
 }
+// Radii to a grid row: as few as fit the device at once (x CTAs per grid row),
+// since a CTA takes its pairs one after the other; KMAX where the tiles fill it.
+inline int pair_per(int K, int x, int most) {
+  int per = 2;
+  while (per < KMAX && (long)x * ((K + per - 1) / per) > most) per *= 2;
+  return per;
+}
 template <class L, int RW, int REGS>
 cudaError_t pair_rows_launch(const float2* spec, const Batch& bt, const float2* tw, int nsm, cudaStream_t st) {
   using R = PairRow<L, RW, REGS>;
   const int ng = L::N * L::N / RW, most = nsm * R::PER_SM;
-  k_pair_rows_filter<L, RW, REGS><<<pair_min(ng, most), R::THREADS, R::SMEM, st>>>(spec, bt, tw);
+  const int x = pair_min(ng, most), per = L::N > PAIR_MULTI_N ? KMAX : pair_per(bt.K, x, most);
+  k_pair_rows_filter<L, RW, REGS><<<dim3(x, (bt.K + per - 1) / per), R::THREADS, R::SMEM, st>>>(
+      spec, pair_batch<L::N>(bt), per, tw);
   return cudaGetLastError();
 }
 template <class L, bool INV, int EPI, int REGS>
@@ -867,8 +933,9 @@ template <class L, bool INV, int EPI, int REGS, bool AHEAD>
 cudaError_t pair_cols_launch(const Batch& bt, uint8_t* rc, float* C, const float* alpha, const float2* tw, int nsm,
                              cudaStream_t st) {
   using G = PairCol<L, REGS>;
-  k_pair_cols<L, INV, EPI, REGS><<<G::NTILES / G::TPC, G::THREADS, G::SMEM, st>>>(bt, rc, C, alpha, tw,
-                                                                                  AHEAD ? nsm * G::PER_SM : 0);
+  const int x = G::NTILES / G::TPC, per = EPI == 2 || L::N > PAIR_MULTI_N ? KMAX : pair_per(bt.K, x, nsm * G::PER_SM);
+  k_pair_cols<L, INV, EPI, REGS><<<dim3(x, (bt.K + per - 1) / per), G::THREADS, G::SMEM, st>>>(
+      pair_batch<L::N>(bt), per, rc, C, alpha, tw, AHEAD ? nsm * G::PER_SM : 0);
   return cudaGetLastError();
 }
 
@@ -962,17 +1029,18 @@ struct PairLaunch {
   static cudaError_t cols_a_adj(const Batch& bt, const float* g, const uint8_t* A, const float* alpha, float* zpart,
                                 const float2* tw, cudaStream_t st) {
     using G = PairCol<Col, CRA>;
-    k_pair_cols_a_adj<Col, CRA><<<G::NTILES / G::TPC, G::THREADS, G::SMEM, st>>>(bt, g, A, alpha, zpart, tw);
+    k_pair_cols_a_adj<Col, CRA><<<G::NTILES / G::TPC, G::THREADS, G::SMEM, st>>>(pair_batch<N>(bt), g, A, alpha, zpart, tw);
     return cudaGetLastError();
   }
   static cudaError_t rows_adj(const Batch& bt, float2* acc, const float2* tw, int nsm, cudaStream_t st) {
     using R = PairRow<Row, S::RW, S::RR>;
     const int ng = N * N / S::RW, most = nsm * R::PER_SM;
-    k_pair_rows_adj<Row, S::RW, S::RR><<<pair_min(ng, most), R::THREADS, ADJ_ROW_SMEM, st>>>(bt, acc, tw);
+    k_pair_rows_adj<Row, S::RW, S::RR><<<pair_min(ng, most), R::THREADS, ADJ_ROW_SMEM, st>>>(pair_batch<N>(bt), acc, tw);
     return cudaGetLastError();
   }
   static constexpr PairOps ops() {
-    return {setup,       pair_rows_launch<Row, S::RW, S::RR>, cols_b,   cols_a_test,
+    return {N <= PAIR_MULTI_N ? RADII_MAX : KMAX,
+            setup,       pair_rows_launch<Row, S::RW, S::RR>, cols_b,   cols_a_test,
             cols_a_crit, cols_a_adj,                          rows_adj, PairCol<Col, CRA>::NTILES / PairCol<Col, CRA>::TPC,
             nat_rows,    nat_cols,                            hf_rows,  hf_cols_a};
   }

@@ -9,6 +9,8 @@ namespace sf21 {
 
 // Max radii fused into one k-space pass (one spectrum read, K outputs).
 constexpr int KMAX = 8;
+// Max radii in one launch of the pair passes, KMAX to a grid row (small boxes).
+constexpr int RADII_MAX = 64;
 // First-hit radius index sentinel: voxel was never a bubble centre.
 constexpr uint8_t RC_NONE = 0xFF;
 
@@ -19,12 +21,14 @@ struct RadiusArg {
   float2* work;   // N^3 complex work buffer for this radius
 };
 
-struct Batch {    // radius indices r[k].ridx increase with k
-  int K;          // radii in this batch (<= KMAX)
+template <int M>
+struct BatchOf {  // radius indices r[k].ridx increase with k
+  int K;          // radii in this batch (<= KMAX; pair passes <= RADII_MAX)
   int set;        // parameter set
   float zmul;     // ionisation-rate multiplier of the set (zeta)
-  RadiusArg r[KMAX];
+  RadiusArg r[M];
 };
+using Batch = BatchOf<RADII_MAX>;
 
 // Real-space top-hat window in k-space, W(x) = 3 (sin x - x cos x) / x^3
 // (auxiliary.c:350-359).  Below x = 2 the Taylor series in x^2 (to x^14,

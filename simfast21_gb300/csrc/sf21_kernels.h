@@ -52,10 +52,11 @@ cudaError_t launch_cols(int N, float2* box, const Batch& bt, int nbox, int axis,
 cudaError_t launch_cols_a_test(int N, const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw,
                                cudaStream_t st);
 
+// Also clears the first-hit box rc and, in its last block (done: a counter that
+// is zero between launches), sets alpha.
 cudaError_t launch_prologue(long n3, const float* delta, const float* src, const PrologueArgs& pa,
-                            float* rec0, float* fres, float2* packed, float* partials, int nblocks,
-                            cudaStream_t st);
-cudaError_t launch_alpha(const float* partials, int nblocks, float* alpha, cudaStream_t st);
+                            float* rec0, float* fres, float2* packed, float* partials, int nblocks, uint8_t* rc,
+                            unsigned int* done, float* alpha, cudaStream_t st);
 int prologue_blocks(long n3);
 
 // Dilation of the first-hit radius field and the final xHII box of one set
@@ -114,6 +115,7 @@ cudaError_t launch_cols_a_test_cb(int N, const Batch& bt, uint8_t* rc, const flo
 // exp(-2 pi i t / N).
 struct HfBatch;
 struct PairOps {  // the launches of one box side
+  int launch_radii;  // radii that one launch takes at most
   cudaError_t (*setup)();
   // c axis with the top-hat filter: spec -> the batch's pair boxes
   cudaError_t (*rows_filter)(const float2* spec, const Batch& bt, const float2* tw, int nsm, cudaStream_t st);
