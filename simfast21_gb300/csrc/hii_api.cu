@@ -147,7 +147,7 @@ struct sf21_hii_ctx {
   unsigned int* d_done = nullptr;  // the prologue's finished blocks (zero between launches)
   bool rc_clear = false;           // d_rc as the prologue left it
   int K_launch = 0;                // radii per launch of the pair passes
-  double* d_neutral = nullptr;  // block sums of the sets' neutral fractions
+  unsigned char* d_neutral = nullptr;  // the sets' neutral sums, in chunks
   // power-spectrum buffers (allocated on first use)
   float2* d_pk = nullptr;
   float* d_pk_w = nullptr;
@@ -975,8 +975,8 @@ extern "C" int sf21_hii_run_z_device(sf21_hii_ctx* c, double z, int kind, const 
 // the host while the GPU works on the next set: set s is written into
 // staging box s mod 2 on the compute stream, copied out on the copy stream,
 // and the staging box is reused only after its copy has completed.  Each
-// set's neutral fraction (:473-477) is summed in double on the GPU before its
-// box leaves; the host adds the blocks' sums.
+// set's neutral fraction is the serial double sum of the reference (:473-477),
+// prepared on the GPU before its box leaves.
 static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, double* neutral) {
   const size_t bf = sizeof(float) * c->n3;
   if (!c->copy_stream) {
@@ -987,9 +987,10 @@ static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, doubl
     }
   }
   if (!c->d_xhii2) CTX_CUDA(c, dev_malloc(&c->d_xhii2, bf));
-  const int ns = (int)c->sets.size(), nb = neutral_blocks();
-  if (neutral && !c->d_neutral) CTX_CUDA(c, dev_malloc(&c->d_neutral, sizeof(double) * nb * ns));
-  std::vector<double> part(neutral ? (size_t)nb * ns : 0);
+  const int ns = (int)c->sets.size();
+  const size_t nb = neutral_bytes(c->n3);
+  if (neutral && !c->d_neutral) CTX_CUDA(c, dev_malloc(&c->d_neutral, nb * ns));
+  std::vector<unsigned char> part(neutral ? nb * ns : 0);
   float* stage[2] = {c->d_xhii, c->d_xhii2};
   int status = SF21_OK;
   // a copy to pageable memory may keep this thread: it is issued when the next
@@ -1009,7 +1010,7 @@ static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, doubl
     if (e == cudaSuccess && (status = enqueue_radii(c, s, st)) == SF21_OK &&
         (status = enqueue_finish(c, s, c->d_src, stage[b], st)) == SF21_OK) {
       e = cudaEventRecord(c->ev_done[b], st);
-      if (e == cudaSuccess && neutral) e = launch_neutral(c->n3, stage[b], c->d_neutral + (size_t)s * nb, st);
+      if (e == cudaSuccess && neutral) e = launch_neutral(c->n3, stage[b], c->d_neutral + s * nb, st);
       if (e == cudaSuccess && s >= 1) e = copy_out(s - 1);
       if (e == cudaSuccess && s + 1 == ns) e = copy_out(s);
     }
@@ -1020,7 +1021,7 @@ static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, doubl
   }
   cudaError_t e = cudaSuccess;
   if (status == SF21_OK && neutral)
-    e = cudaMemcpyAsync(part.data(), c->d_neutral, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, st);
+    e = cudaMemcpyAsync(part.data(), c->d_neutral, part.size(), cudaMemcpyDeviceToHost, st);
   const cudaError_t ec = cudaStreamSynchronize(c->copy_stream), es = cudaStreamSynchronize(st);
   for (cudaError_t x : {ec, es})
     if (e == cudaSuccess) e = x;
@@ -1030,11 +1031,8 @@ static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, doubl
   }
   if (status == SF21_OK) status = check_device_flag(c);
   if (status == SF21_OK && neutral)
-    for (int s = 0; s < ns; ++s) {
-      double acc = 0.;
-      for (int k = 0; k < nb; ++k) acc += part[(size_t)s * nb + k];
-      neutral[s] = acc / c->n3;
-    }
+    for (int s = 0; s < ns; ++s)
+      neutral[s] = neutral_sum(c->n3, part.data() + s * nb, xhii + (size_t)s * c->n3) / c->n3;
   return status;
 }
 

@@ -5,7 +5,12 @@
 // integer soft-double routines.  The dilation and the per-set finish are in
 // kernels_dt.cu.
 #include <cuda_runtime.h>
+#include <math.h>
+#include <math_constants.h>
 #include <stdint.h>
+#include <string.h>
+
+#include <algorithm>
 
 #include "sf21_kernels.h"
 #include "softdouble.h"
@@ -170,34 +175,132 @@ cudaError_t launch_fill0(long n3, uint64_t zeta, const float* src, const float* 
   return cudaGetLastError();
 }
 
-// Neutral fraction: the sum of 1 - x.  Every thread adds the terms of its own
-// four columns in double, then the threads of a block as a tree, and the host
-// adds the 608 blocks: within (n3 / 600 000 + 620) 2^-53 of the sum, where a
-// serial sum is within n3 2^-53.  The serial sum on the host took 10 ms at
-// 256^3, one addition after the other; 12 us here, bound by the read.
-constexpr int NEU_THREADS = 256, NEU_BLOCKS = 608;
-__global__ void __launch_bounds__(NEU_THREADS) k_neutral(long n4, const float4* __restrict__ x, double* __restrict__ part) {
-  double s[4] = {0., 0., 0., 0.};
-  for (long i = (long)blockIdx.x * NEU_THREADS + threadIdx.x; i < n4; i += (long)NEU_BLOCKS * NEU_THREADS) {
-    const float4 v = __ldg(x + i);
-    s[0] += 1.0 - v.x;
-    s[1] += 1.0 - v.y;
-    s[2] += 1.0 - v.z;
-    s[3] += 1.0 - v.w;
+// Neutral fraction (:473-477): the serial double sum S of 1 - x, bit for bit,
+// from chunks that are summed in parallel.  While S stays in [2^E, 2^(E+1)) an
+// addition rounds its term t to a multiple of u = 2^(E-52), whatever S is,
+// except for ties (t an odd multiple of u / 2), which go to the even multiple
+// and so depend on the parity of S / u alone.  A run of terms is therefore a
+// pair: the multiples of u that it adds to an even and to an odd S / u; such
+// pairs compose.  E of a chunk follows from approximate sums; a chunk in which
+// S may leave its binade (about one per binade), starts below 1 or has a term
+// outside [0, 1] is left to the host's serial loop (E = -1).
+// 256^3: 10 ms as a loop on the host, 40 us here.
+constexpr int NEU_THREADS = 256, NEU_PER = NEUTRAL_CHUNK / NEU_THREADS;  // consecutive terms per thread
+static_assert(NEU_PER == 16, "four float4 per thread");
+
+__device__ __forceinline__ void neutral_terms(const float* __restrict__ x, long n3, double (&t)[NEU_PER]) {
+  const long i0 = (long)blockIdx.x * NEUTRAL_CHUNK + (long)threadIdx.x * NEU_PER;
+#pragma unroll
+  for (int k = 0; k < NEU_PER; k += 4) {
+    const float4 v = i0 + k < n3 ? __ldg(reinterpret_cast<const float4*>(x + i0 + k)) : make_float4(1.f, 1.f, 1.f, 1.f);
+    t[k] = 1.0 - v.x;
+    t[k + 1] = 1.0 - v.y;
+    t[k + 2] = 1.0 - v.z;
+    t[k + 3] = 1.0 - v.w;
   }
-  __shared__ double sh[NEU_THREADS];
-  sh[threadIdx.x] = (s[0] + s[1]) + (s[2] + s[3]);
-  for (int o = NEU_THREADS / 2; o > 0; o >>= 1) {
-    __syncthreads();
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-int neutral_blocks() { return NEU_BLOCKS; }
-cudaError_t launch_neutral(long n3, const float* x, double* part, cudaStream_t st) {
-  k_neutral<<<NEU_BLOCKS, NEU_THREADS, 0, st>>>(n3 / 4, reinterpret_cast<const float4*>(x), part);
+__global__ void __launch_bounds__(NEU_THREADS) k_neutral_sums(const float* __restrict__ x, long n3, double* __restrict__ sum) {
+  double t[NEU_PER], s = 0.;
+  neutral_terms(x, n3, t);
+  bool bad = false;
+#pragma unroll
+  for (int k = 0; k < NEU_PER; ++k) {
+    bad = bad || !(t[k] >= 0.0 && t[k] <= 1.0);
+    s += t[k];
+  }
+  __shared__ double sh[NEU_THREADS];
+  sh[threadIdx.x] = s;
+  bad = __syncthreads_or(bad);
+  for (int o = NEU_THREADS / 2; o > 0; o >>= 1) {
+    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) sum[blockIdx.x] = bad ? -1.0 : sh[0];
+}
+
+// E of every chunk; a chunk with a term outside [0, 1] leaves all that follow to the host
+__global__ void __launch_bounds__(1024) k_neutral_binades(int nchunk, const double* __restrict__ sum, int* __restrict__ E) {
+  __shared__ double sh[1024];
+  const int per = (nchunk + 1023) / 1024, c0 = threadIdx.x * per, c1 = min(nchunk, c0 + per);
+  double s = 0.;
+  for (int c = c0; c < c1; ++c) s += sum[c] < 0.0 ? CUDART_NAN : sum[c];
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  double before = 0.;
+  for (int k = 0; k < (int)threadIdx.x; ++k) before += sh[k];
+  for (int c = c0; c < c1; ++c) {
+    const double v = sum[c] < 0.0 ? CUDART_NAN : sum[c];
+    const double lo = before * (1.0 - 1e-9), hi = (before + v) * (1.0 + 1e-9);
+    const int el = (int)(__double_as_longlong(lo) >> 52) - 1023, eh = (int)(__double_as_longlong(hi) >> 52) - 1023;
+    E[c] = lo >= 1.0 && el == eh ? el : -1;  // NaN: the first test fails
+    before += v;
+  }
+}
+
+__global__ void __launch_bounds__(NEU_THREADS)
+k_neutral_steps(const float* __restrict__ x, long n3, const int* __restrict__ binade, longlong2* __restrict__ step) {
+  const int E = binade[blockIdx.x];
+  if (E < 0) return;
+  double t[NEU_PER];
+  neutral_terms(x, n3, t);
+  long long d0 = 0, d1 = 0;  // added to an even and an odd S / u
+#pragma unroll
+  for (int k = 0; k < NEU_PER; ++k) {
+    const long long b = __double_as_longlong(t[k]);  // 0 or a normal number <= 1
+    const int sh = E - ((int)(b >> 52) - 1023);
+    const long long m = b ? (b & 0xFFFFFFFFFFFFFLL) | (1LL << 52) : 0;
+    if (sh > 53) continue;  // below u / 2
+    const long long q = m >> sh, rem = m & ((1LL << sh) - 1), half = sh ? 1LL << (sh - 1) : 1;
+    const long long up = rem > half;
+    const bool tie = rem == half;
+    d0 += q + (tie ? (d0 + q) & 1 : up);
+    d1 += q + (tie ? (1 + d1 + q) & 1 : up);
+  }
+  __shared__ longlong2 sh2[NEU_THREADS];
+  sh2[threadIdx.x] = make_longlong2(d0, d1);
+  for (int o = 1; o < NEU_THREADS; o <<= 1) {  // neighbours in order
+    __syncthreads();
+    if (threadIdx.x % (2 * o) == 0) {
+      const longlong2 f = sh2[threadIdx.x], g = sh2[threadIdx.x + o];
+      sh2[threadIdx.x] = make_longlong2(f.x + (f.x & 1 ? g.y : g.x), f.y + ((1 + f.y) & 1 ? g.y : g.x));
+    }
+  }
+  if (threadIdx.x == 0) step[blockIdx.x] = sh2[0];
+}
+
+int neutral_chunks(long n3) { return (int)((n3 + NEUTRAL_CHUNK - 1) / NEUTRAL_CHUNK); }
+size_t neutral_bytes(long n3) {  // whole longlong2, so that the sets' buffers can follow one another
+  return ((size_t)neutral_chunks(n3) * (sizeof(longlong2) + sizeof(double) + sizeof(int)) + 15) / 16 * 16;
+}
+cudaError_t launch_neutral(long n3, const float* x, void* buf, cudaStream_t st) {
+  const int n = neutral_chunks(n3);
+  longlong2* step = static_cast<longlong2*>(buf);
+  double* sum = reinterpret_cast<double*>(step + n);
+  int* E = reinterpret_cast<int*>(sum + n);
+  k_neutral_sums<<<n, NEU_THREADS, 0, st>>>(x, n3, sum);
+  k_neutral_binades<<<1, 1024, 0, st>>>(n, sum, E);
+  k_neutral_steps<<<n, NEU_THREADS, 0, st>>>(x, n3, E, step);
   return cudaGetLastError();
+}
+
+// The serial sum from the chunks' pairs (buf: launch_neutral's, on the host) and the box x
+double neutral_sum(long n3, const void* buf, const float* x) {
+  const int n = neutral_chunks(n3);
+  const longlong2* step = static_cast<const longlong2*>(buf);
+  const int* E = reinterpret_cast<const int*>(reinterpret_cast<const double*>(step + n) + n);
+  double S = 0.;
+  for (int c = 0; c < n; ++c) {
+    uint64_t b;
+    memcpy(&b, &S, 8);
+    if (E[c] >= 0 && (int)(b >> 52) - 1023 == E[c]) {
+      S += ldexp((double)(b & 1 ? step[c].y : step[c].x), E[c] - 52);  // exact: S stays in its binade
+    } else {
+      const long end = std::min(n3, (long)(c + 1) * NEUTRAL_CHUNK);
+      for (long i = (long)c * NEUTRAL_CHUNK; i < end; ++i) S += 1.0 - x[i];
+    }
+  }
+  return S;
 }
 
 }  // namespace sf21

@@ -177,9 +177,13 @@ cudaError_t launch_grad_finish(long n3, const float2* G, const float* alpha, con
 cudaError_t launch_crit_init(long n3, float* C, uint8_t* A, cudaStream_t st);
 cudaError_t launch_crit_finalize(long n3, float* C, const uint8_t* A, cudaStream_t st);
 
-// Block sums of 1 - x in double (neutral_blocks() of them); n3 a multiple of 4
-int neutral_blocks();
-cudaError_t launch_neutral(long n3, const float* x, double* part, cudaStream_t st);
+// The serial double sum of 1 - x (the neutral fraction's): chunks on the GPU
+// into buf (neutral_bytes; n3 a multiple of 16), then, with buf and x on the
+// host, the sum.
+constexpr int NEUTRAL_CHUNK = 4096;
+size_t neutral_bytes(long n3);
+cudaError_t launch_neutral(long n3, const float* x, void* buf, cudaStream_t st);
+double neutral_sum(long n3, const void* buf, const float* x);
 
 // Halo-catalogue source box (kernels_halo.cu): CIC of Rion + block average,
 // bit-identical with the reference's serial loop.  halos_dev: nh records
