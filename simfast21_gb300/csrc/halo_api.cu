@@ -634,8 +634,6 @@ extern "C" int sf21_halo_create(const sf21_halo_config* cfg, sf21_halo_ctx** out
     HCREATE(gen_setup(N));
   } else {
     HCREATE(fft_setup(N));
-    HCREATE(cb_setup(N));
-    HCREATE(hf_setup(N));
   }
   const size_t box_c = sizeof(float2) * c->n3, bits = sizeof(uint32_t) * c->nwords;
   HCREATE(dev_malloc(&c->d_spec, box_c));
@@ -697,14 +695,10 @@ static int set_density_dev(sf21_halo_ctx* c, const float* d, cudaStream_t st) {
     HCTX_CUDA(c, c->pair->nat_rows(nullptr, c->d_delta, nullptr, c->d_spec, N, false, nullptr, c->d_twp, c->nsm, st));
     HCTX_CUDA(c, c->pair->nat_cols(c->d_spec, 1, false, N, c->d_twp, st));
     HCTX_CUDA(c, c->pair->nat_cols(c->d_spec, 0, false, N, c->d_twp, st));
-  } else if (c->gen) {
+  } else {
     HCTX_CUDA(c, launch_gen_fwd_rows(c->gp, packed, c->d_spec, nullptr, c->d_tw, st));
     HCTX_CUDA(c, launch_gen_cols(c->gp, c->d_spec, none, 1, false, c->d_tw, st));
     HCTX_CUDA(c, launch_gen_cols(c->gp, c->d_spec, none, 0, false, c->d_tw, st));
-  } else {
-    HCTX_CUDA(c, launch_fwd_rows(N, packed, c->d_spec, nullptr, c->d_tw, st));
-    HCTX_CUDA(c, launch_cols(N, c->d_spec, none, 1, 1, false, c->d_tw, st));
-    HCTX_CUDA(c, launch_cols(N, c->d_spec, none, 1, 0, false, c->d_tw, st));
   }
   c->have_density = true;
   return SF21_OK;
@@ -1073,14 +1067,10 @@ static int run_filter_bank(sf21_halo_ctx* c, const std::vector<MassPlan>& plan, 
       HCTX_CUDA(c, c->pair->hf_rows(c->d_spec, hb, c->d_twp, c->nsm, st));
       HCTX_CUDA(c, c->pair->cols_b(bt, true, c->d_twp, c->nsm, st));
       HCTX_CUDA(c, c->pair->hf_cols_a(hb, c->d_twp, c->nsm, st));
-    } else if (c->gen) {
+    } else {  // a 2-3-5 side without pair lines (every power of two has them)
       HCTX_CUDA(c, launch_gen_hf_rows_filter(c->gp, c->d_spec, hb, c->d_tw, st));
       HCTX_CUDA(c, launch_gen_hf_cols(c->gp, hb, 1, false, c->d_tw, st));
       HCTX_CUDA(c, launch_gen_hf_cols(c->gp, hb, 0, true, c->d_tw, st));
-    } else {
-      HCTX_CUDA(c, launch_hf_rows_filter_cb(N, c->d_spec, hb, c->d_tw, st));
-      HCTX_CUDA(c, launch_cols_b_cb(N, bt, c->d_tw, st));
-      HCTX_CUDA(c, launch_hf_cols_a_thresh_cb(N, hb, c->d_tw, st));
     }
   }
   return SF21_OK;

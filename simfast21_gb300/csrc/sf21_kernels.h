@@ -102,10 +102,9 @@ cudaError_t launch_pipe(int N, int mode, int layout, const PipeMaps& pm, const B
                         uint32_t spin_limit = 0);
 
 // Radius pipeline over column-block-major work boxes (kernels_cb.cu):
-// c-axis filter pass, in-place b-axis pass, a-axis pass + centre test.
+// c-axis filter pass, a-axis pass + centre test (the b axis is launch_pipe's).
 cudaError_t cb_setup(int N);
 cudaError_t launch_rows_filter_cb(int N, const float2* spec, const Batch& bt, const float2* tw, cudaStream_t st);
-cudaError_t launch_cols_b_cb(int N, const Batch& bt, const float2* tw, cudaStream_t st);
 cudaError_t launch_cols_a_test_cb(int N, const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw, int nsm,
                                   cudaStream_t st);
 
@@ -246,14 +245,7 @@ struct HfBatch {
 };
 // candidate states of the overlap test
 constexpr uint8_t HF_UND = 0, HF_PEND_ACC = 1, HF_PEND_REJ = 2, HF_ACC = 3, HF_ACC_FLAGGED = 4, HF_REJ = 5;
-cudaError_t hf_setup(int N);
 cudaError_t launch_hf_rows_filter(int N, const float2* spec, const HfBatch& hb, const float2* tw, cudaStream_t st);
-cudaError_t launch_hf_cols_a_thresh(int N, const HfBatch& hb, const float2* tw, cudaStream_t st);
-// column-block-major form: rows_cb -> launch_cols_b_cb (a Batch over the same
-// work boxes) -> cols_a_thresh_cb
-cudaError_t launch_hf_rows_filter_cb(int N, const float2* spec, const HfBatch& hb, const float2* tw,
-                                     cudaStream_t st);
-cudaError_t launch_hf_cols_a_thresh_cb(int N, const HfBatch& hb, const float2* tw, cudaStream_t st);
 long hf_compact_chunks(long nwords);
 cudaError_t launch_bits_count(const uint32_t* W, long nwords, uint32_t* cnt, cudaStream_t st);
 cudaError_t launch_scan_counts(uint32_t* cnt, long n, uint32_t* tot, cudaStream_t st);
