@@ -13,8 +13,8 @@ value : device-resident inputs, CUDA events on the launch stream; the timed
         per-kernel split comes from a separate event-instrumented step.
 e2e   : the same through the host-buffer C-ABI call sf21_hii_run_z (pinned
         host inputs copied in, 64 xHII boxes copied out into pinned host
-        memory while the next set computes, neutral fractions summed on the
-        host) -- the reference-facing path.
+        memory while the next set computes, neutral fractions with the bits
+        of the serial sum) -- the reference-facing path.
 --impl reference: the CPU restatement of get_HIIbubbles.c (oracle/, FFTW-API
         shim, OpenMP on all host cores) timed on bounded samples of the
         workload (the front of a redshift and a spread of radii of the median

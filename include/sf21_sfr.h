@@ -10,7 +10,7 @@
  * and the division by dx_halo^3 that turns the average into an SFR density in
  * Msun/(Mpc/h)^3/yr (:129-131).  The box is bit-identical with the
  * reference's serial loop: the CIC contributions are computed in parallel and
- * replayed per cell in the catalogue's order.  The per-redshift files
+ * added per cell in the catalogue's order.  The per-redshift files
  * (SFR/sfrd_z*.dat and the Output_text_files/sfrd_av_* line) are written by
  * the drop-in driver sf21_get_SFR.
  *
