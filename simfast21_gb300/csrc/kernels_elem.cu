@@ -8,10 +8,8 @@
 #include <math.h>
 #include <math_constants.h>
 #include <stdint.h>
-#include <string.h>
 
-#include <algorithm>
-
+#include "neutral_sum.h"
 #include "sf21_kernels.h"
 #include "softdouble.h"
 
@@ -175,15 +173,11 @@ cudaError_t launch_fill0(long n3, uint64_t zeta, const float* src, const float* 
   return cudaGetLastError();
 }
 
-// Neutral fraction (:473-477): the serial double sum S of 1 - x, bit for bit,
-// from chunks that are summed in parallel.  While S stays in [2^E, 2^(E+1)) an
-// addition rounds its term t to a multiple of u = 2^(E-52), whatever S is,
-// except for ties (t an odd multiple of u / 2), which go to the even multiple
-// and so depend on the parity of S / u alone.  A run of terms is therefore a
-// pair: the multiples of u that it adds to an even and to an odd S / u; such
-// pairs compose.  E of a chunk follows from approximate sums; a chunk in which
-// S may leave its binade (about one per binade), starts below 1 or has a term
-// outside [0, 1] is left to the host's serial loop (E = -1).
+// Neutral fraction (:473-477): the serial double sum of 1 - x from chunks, each
+// a pair of multiples of u (neutral_sum.h).  Pairs compose.  E of a chunk
+// follows from approximate sums; a chunk in which S may leave its binade (about
+// one per binade), starts below 1 or has a term outside [0, 1] is left to the
+// host's serial loop (E = -1).
 // 256^3: 10 ms as a loop on the host, 40 us here.
 constexpr int NEU_THREADS = 256, NEU_PER = NEUTRAL_CHUNK / NEU_THREADS;  // consecutive terms per thread
 static_assert(NEU_PER == 16, "four float4 per thread");
@@ -289,18 +283,7 @@ double neutral_sum(long n3, const void* buf, const float* x) {
   const int n = neutral_chunks(n3);
   const longlong2* step = static_cast<const longlong2*>(buf);
   const int* E = reinterpret_cast<const int*>(reinterpret_cast<const double*>(step + n) + n);
-  double S = 0.;
-  for (int c = 0; c < n; ++c) {
-    uint64_t b;
-    memcpy(&b, &S, 8);
-    if (E[c] >= 0 && (int)(b >> 52) - 1023 == E[c]) {
-      S += ldexp((double)(b & 1 ? step[c].y : step[c].x), E[c] - 52);  // exact: S stays in its binade
-    } else {
-      const long end = std::min(n3, (long)(c + 1) * NEUTRAL_CHUNK);
-      for (long i = (long)c * NEUTRAL_CHUNK; i < end; ++i) S += 1.0 - x[i];
-    }
-  }
-  return S;
+  return neutral_serial(n3, &step->x, E, [x](long i) { return x[i]; });
 }
 
 }  // namespace sf21

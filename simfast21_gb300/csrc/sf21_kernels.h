@@ -179,7 +179,6 @@ cudaError_t launch_crit_finalize(long n3, float* C, const uint8_t* A, cudaStream
 // The serial double sum of 1 - x (the neutral fraction's): chunks on the GPU
 // into buf (neutral_bytes; n3 a multiple of 16), then, with buf and x on the
 // host, the sum.
-constexpr int NEUTRAL_CHUNK = 4096;
 size_t neutral_bytes(long n3);
 cudaError_t launch_neutral(long n3, const float* x, void* buf, cudaStream_t st);
 double neutral_sum(long n3, const void* buf, const float* x);
