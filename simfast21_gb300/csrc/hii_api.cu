@@ -989,8 +989,9 @@ static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, doubl
   if (!c->d_xhii2) CTX_CUDA(c, dev_malloc(&c->d_xhii2, bf));
   const int ns = (int)c->sets.size();
   const size_t nb = neutral_bytes(c->n3);
-  if (neutral && !c->d_neutral) CTX_CUDA(c, dev_malloc(&c->d_neutral, nb * ns));
-  std::vector<unsigned char> part(neutral ? nb * ns : 0);
+  const bool chunks = neutral && c->n3 > NEUTRAL_HOST;
+  if (chunks && !c->d_neutral) CTX_CUDA(c, dev_malloc(&c->d_neutral, nb * ns));
+  std::vector<unsigned char> part(chunks ? nb * ns : 0);
   float* stage[2] = {c->d_xhii, c->d_xhii2};
   int status = SF21_OK;
   // a copy to pageable memory may keep this thread: it is issued when the next
@@ -1010,7 +1011,7 @@ static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, doubl
     if (e == cudaSuccess && (status = enqueue_radii(c, s, st)) == SF21_OK &&
         (status = enqueue_finish(c, s, c->d_src, stage[b], st)) == SF21_OK) {
       e = cudaEventRecord(c->ev_done[b], st);
-      if (e == cudaSuccess && neutral) e = launch_neutral(c->n3, stage[b], c->d_neutral + s * nb, st);
+      if (e == cudaSuccess && chunks) e = launch_neutral(c->n3, stage[b], c->d_neutral + s * nb, st);
       if (e == cudaSuccess && s >= 1) e = copy_out(s - 1);
       if (e == cudaSuccess && s + 1 == ns) e = copy_out(s);
     }
@@ -1020,7 +1021,7 @@ static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, doubl
     }
   }
   cudaError_t e = cudaSuccess;
-  if (status == SF21_OK && neutral)
+  if (status == SF21_OK && chunks)
     e = cudaMemcpyAsync(part.data(), c->d_neutral, part.size(), cudaMemcpyDeviceToHost, st);
   const cudaError_t ec = cudaStreamSynchronize(c->copy_stream), es = cudaStreamSynchronize(st);
   for (cudaError_t x : {ec, es})
@@ -1032,7 +1033,7 @@ static int run_sets_to_host(sf21_hii_ctx* c, cudaStream_t st, float* xhii, doubl
   if (status == SF21_OK) status = check_device_flag(c);
   if (status == SF21_OK && neutral)
     for (int s = 0; s < ns; ++s)
-      neutral[s] = neutral_sum(c->n3, part.data() + s * nb, xhii + (size_t)s * c->n3) / c->n3;
+      neutral[s] = neutral_sum(c->n3, chunks ? part.data() + s * nb : nullptr, xhii + (size_t)s * c->n3) / c->n3;
   return status;
 }
 

@@ -6,7 +6,6 @@
 // kernels_dt.cu.
 #include <cuda_runtime.h>
 #include <math.h>
-#include <math_constants.h>
 #include <stdint.h>
 
 #include "neutral_sum.h"
@@ -174,61 +173,100 @@ cudaError_t launch_fill0(long n3, uint64_t zeta, const float* src, const float* 
 }
 
 // Neutral fraction (:473-477): the serial double sum of 1 - x from chunks, each
-// a pair of multiples of u (neutral_sum.h).  Pairs compose.  E of a chunk
-// follows from approximate sums; a chunk in which S may leave its binade (about
-// one per binade), starts below 1 or has a term outside [0, 1] is left to the
-// host's serial loop (E = -1).
-// 256^3: 10 ms as a loop on the host, 40 us here.
+// a pair of multiples of u (neutral_sum.h).  Pairs compose.  Everything here is
+// in integers: a term is a multiple of 2^-53 (neutral_units), and while S is in
+// [2^E, 2^(E+1)) an addition rounds it to a multiple of 2^(E+1) of those.  E of
+// a chunk follows from the chunks' sums; a chunk in which S may leave its
+// binade (about one per binade), starts below 1 or has a term outside [0, 1]
+// is left to the host's serial loop (E = -1).
+// A call with host boxes and four sets, neutral fractions included: 16^3 0.52
+// ms with the sums as loops on host threads, 0.99 when one block added the
+// chunks' sums in FP64, each thread all that come before its own, 0.26 so;
+// 64^3 0.81, 1.19, 0.53; 256^3 20.4, 9.0, 8.0.  One pass over the box each,
+// bound by its reads.
 constexpr int NEU_THREADS = 256, NEU_PER = NEUTRAL_CHUNK / NEU_THREADS;  // consecutive terms per thread
 static_assert(NEU_PER == 16, "four float4 per thread");
+constexpr uint64_t NEU_BAD = ~0ull;  // sum of a chunk with a term outside [0, 1]
 
-__device__ __forceinline__ void neutral_terms(const float* __restrict__ x, long n3, double (&t)[NEU_PER]) {
+// false: a term is outside [0, 1]
+__device__ __forceinline__ bool neutral_terms(const float* __restrict__ x, long n3, uint64_t (&t)[NEU_PER]) {
   const long i0 = (long)blockIdx.x * NEUTRAL_CHUNK + (long)threadIdx.x * NEU_PER;
+  bool ok = true;
 #pragma unroll
   for (int k = 0; k < NEU_PER; k += 4) {
     const float4 v = i0 + k < n3 ? __ldg(reinterpret_cast<const float4*>(x + i0 + k)) : make_float4(1.f, 1.f, 1.f, 1.f);
-    t[k] = 1.0 - v.x;
-    t[k + 1] = 1.0 - v.y;
-    t[k + 2] = 1.0 - v.z;
-    t[k + 3] = 1.0 - v.w;
-  }
-}
-
-__global__ void __launch_bounds__(NEU_THREADS) k_neutral_sums(const float* __restrict__ x, long n3, double* __restrict__ sum) {
-  double t[NEU_PER], s = 0.;
-  neutral_terms(x, n3, t);
-  bool bad = false;
+    const float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-  for (int k = 0; k < NEU_PER; ++k) {
-    bad = bad || !(t[k] >= 0.0 && t[k] <= 1.0);
-    s += t[k];
+    for (int j = 0; j < 4; ++j) {
+      ok = ok && f[j] >= 0.0f && f[j] <= 1.0f;
+      t[k + j] = neutral_units(f[j]);
+    }
   }
-  __shared__ double sh[NEU_THREADS];
-  sh[threadIdx.x] = s;
-  bad = __syncthreads_or(bad);
-  for (int o = NEU_THREADS / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) sum[blockIdx.x] = bad ? -1.0 : sh[0];
+  return ok;
 }
 
-// E of every chunk; a chunk with a term outside [0, 1] leaves all that follow to the host
-__global__ void __launch_bounds__(1024) k_neutral_binades(int nchunk, const double* __restrict__ sum, int* __restrict__ E) {
-  __shared__ double sh[1024];
-  const int per = (nchunk + 1023) / 1024, c0 = threadIdx.x * per, c1 = min(nchunk, c0 + per);
-  double s = 0.;
-  for (int c = c0; c < c1; ++c) s += sum[c] < 0.0 ? CUDART_NAN : sum[c];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  double before = 0.;
-  for (int k = 0; k < (int)threadIdx.x; ++k) before += sh[k];
-  for (int c = c0; c < c1; ++c) {
-    const double v = sum[c] < 0.0 ? CUDART_NAN : sum[c];
-    const double lo = before * (1.0 - 1e-9), hi = (before + v) * (1.0 + 1e-9);
-    const int el = (int)(__double_as_longlong(lo) >> 52) - 1023, eh = (int)(__double_as_longlong(hi) >> 52) - 1023;
-    E[c] = lo >= 1.0 && el == eh ? el : -1;  // NaN: the first test fails
-    before += v;
+// sum[chunk]: its terms' sum in units of 2^-32, 256 of them too small at most
+// (a thread's 16 terms are below 2^58 units of 2^-53)
+__global__ void __launch_bounds__(NEU_THREADS)
+k_neutral_sums(const float* __restrict__ x, long n3, uint64_t* __restrict__ sum) {
+  uint64_t t[NEU_PER], s = 0;
+  const bool ok = neutral_terms(x, n3, t);
+#pragma unroll
+  for (int k = 0; k < NEU_PER; ++k) s += t[k];
+  s >>= 21;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  __shared__ uint64_t sh[NEU_THREADS / 32];
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+  const bool good = __syncthreads_and(ok);
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < NEU_THREADS / 32; ++w) s += sh[w];
+    sum[blockIdx.x] = good ? s : NEU_BAD;
+  }
+}
+
+// E of every chunk, from the sums before and after it.  One block scans the
+// chunks, four to a thread: 4096 of them at a time, 8 times at 512^3.
+constexpr int NEU_SCAN = 1024;
+__global__ void __launch_bounds__(NEU_SCAN) k_neutral_binades(int nchunk, const uint64_t* __restrict__ sum, int* __restrict__ E) {
+  __shared__ uint64_t sh[NEU_SCAN / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint64_t carry = 0;
+  for (int c0 = 0; c0 < nchunk; c0 += 4 * NEU_SCAN) {
+    const int c = c0 + 4 * threadIdx.x;
+    uint64_t v[4], t = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[k] = c + k < nchunk ? sum[c + k] : 0;
+      t += v[k] == NEU_BAD ? 0 : v[k];
+    }
+    uint64_t x = t;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) sh[w] = x;
+    __syncthreads();
+    uint64_t y = sh[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t z = __shfl_up_sync(0xffffffffu, y, o);
+      if (lane >= o) y += z;
+    }
+    uint64_t before = carry + x - t;
+    const uint64_t below = __shfl_sync(0xffffffffu, y, w ? w - 1 : 0);
+    if (w) before += below;
+    carry += __shfl_sync(0xffffffffu, y, 31);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (c + k >= nchunk) break;
+      const uint64_t after = before + (v[k] == NEU_BAD ? 0 : v[k]);
+      const int el = 31 - __clzll((long long)before), eh = 31 - __clzll((long long)after);  // in units of 2^-32
+      E[c + k] = el >= 0 && el == eh && v[k] != NEU_BAD ? el : -1;
+      before = after;
+    }
+    __syncthreads();  // sh has been read
   }
 }
 
@@ -236,53 +274,65 @@ __global__ void __launch_bounds__(NEU_THREADS)
 k_neutral_steps(const float* __restrict__ x, long n3, const int* __restrict__ binade, longlong2* __restrict__ step) {
   const int E = binade[blockIdx.x];
   if (E < 0) return;
-  double t[NEU_PER];
+  uint64_t t[NEU_PER];
   neutral_terms(x, n3, t);
   long long d0 = 0, d1 = 0;  // added to an even and an odd S / u
+  const int sh = E + 1;      // u = 2^(E-52)
+  const uint64_t half = 1ull << E;
 #pragma unroll
   for (int k = 0; k < NEU_PER; ++k) {
-    const long long b = __double_as_longlong(t[k]);  // 0 or a normal number <= 1
-    const int sh = E - ((int)(b >> 52) - 1023);
-    const long long m = b ? (b & 0xFFFFFFFFFFFFFLL) | (1LL << 52) : 0;
-    if (sh > 53) continue;  // below u / 2
-    const long long q = m >> sh, rem = m & ((1LL << sh) - 1), half = sh ? 1LL << (sh - 1) : 1;
+    const long long q = (long long)(t[k] >> sh);
+    const uint64_t rem = t[k] & (2 * half - 1);
     const long long up = rem > half;
     const bool tie = rem == half;
     d0 += q + (tie ? (d0 + q) & 1 : up);
     d1 += q + (tie ? (1 + d1 + q) & 1 : up);
   }
-  __shared__ longlong2 sh2[NEU_THREADS];
-  sh2[threadIdx.x] = make_longlong2(d0, d1);
-  for (int o = 1; o < NEU_THREADS; o <<= 1) {  // neighbours in order
-    __syncthreads();
-    if (threadIdx.x % (2 * o) == 0) {
-      const longlong2 f = sh2[threadIdx.x], g = sh2[threadIdx.x + o];
-      sh2[threadIdx.x] = make_longlong2(f.x + (f.x & 1 ? g.y : g.x), f.y + ((1 + f.y) & 1 ? g.y : g.x));
-    }
+  // neighbours in order: within a warp, then the warps
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  auto then = [](longlong2 f, longlong2 g) {
+    return make_longlong2(f.x + (f.x & 1 ? g.y : g.x), f.y + ((1 + f.y) & 1 ? g.y : g.x));
+  };
+  longlong2 f = make_longlong2(d0, d1);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const longlong2 g = make_longlong2(__shfl_down_sync(0xffffffffu, f.x, o), __shfl_down_sync(0xffffffffu, f.y, o));
+    if ((lane & (2 * o - 1)) == 0) f = then(f, g);
   }
-  if (threadIdx.x == 0) step[blockIdx.x] = sh2[0];
+  __shared__ longlong2 sh2[NEU_THREADS / 32];
+  if (lane == 0) sh2[w] = f;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < NEU_THREADS / 32; ++k) f = then(f, sh2[k]);
+    step[blockIdx.x] = f;
+  }
 }
 
 int neutral_chunks(long n3) { return (int)((n3 + NEUTRAL_CHUNK - 1) / NEUTRAL_CHUNK); }
 size_t neutral_bytes(long n3) {  // whole longlong2, so that the sets' buffers can follow one another
-  return ((size_t)neutral_chunks(n3) * (sizeof(longlong2) + sizeof(double) + sizeof(int)) + 15) / 16 * 16;
+  return ((size_t)neutral_chunks(n3) * (sizeof(longlong2) + sizeof(uint64_t) + sizeof(int)) + 15) / 16 * 16;
 }
 cudaError_t launch_neutral(long n3, const float* x, void* buf, cudaStream_t st) {
   const int n = neutral_chunks(n3);
   longlong2* step = static_cast<longlong2*>(buf);
-  double* sum = reinterpret_cast<double*>(step + n);
+  uint64_t* sum = reinterpret_cast<uint64_t*>(step + n);
   int* E = reinterpret_cast<int*>(sum + n);
   k_neutral_sums<<<n, NEU_THREADS, 0, st>>>(x, n3, sum);
-  k_neutral_binades<<<1, 1024, 0, st>>>(n, sum, E);
+  k_neutral_binades<<<1, NEU_SCAN, 0, st>>>(n, sum, E);
   k_neutral_steps<<<n, NEU_THREADS, 0, st>>>(x, n3, E, step);
   return cudaGetLastError();
 }
 
-// The serial sum from the chunks' pairs (buf: launch_neutral's, on the host) and the box x
+// The serial sum from the chunks' pairs (buf: launch_neutral's, on the host; null: none) and the box x
 double neutral_sum(long n3, const void* buf, const float* x) {
+  if (!buf) {
+    double S = 0.;
+    for (long i = 0; i < n3; ++i) S += 1.0 - x[i];
+    return S;
+  }
   const int n = neutral_chunks(n3);
   const longlong2* step = static_cast<const longlong2*>(buf);
-  const int* E = reinterpret_cast<const int*>(reinterpret_cast<const double*>(step + n) + n);
+  const int* E = reinterpret_cast<const int*>(reinterpret_cast<const uint64_t*>(step + n) + n);
   return neutral_serial(n3, &step->x, E, [x](long i) { return x[i]; });
 }
 

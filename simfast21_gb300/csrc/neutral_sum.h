@@ -16,6 +16,36 @@ namespace sf21 {
 
 constexpr int NEUTRAL_CHUNK = 4096;
 
+#if defined(__CUDACC__)
+#define NEU_HD __host__ __device__ __forceinline__
+#else
+#define NEU_HD static inline
+#endif
+
+// 1.0 - x in double, for a float x in [0, 1], as a multiple of 2^-53: doubles
+// of [0, 1] are such multiples from 1/2 up, and below 1/2 the difference is
+// exact, a multiple of 2^-24.  x is rounded to one (ties to even: the
+// difference from 2^53 has the same parity).
+NEU_HD uint64_t neutral_units(float x) {
+  union {
+    float f;
+    uint32_t u;
+  } c;
+  c.f = x;
+  const int ex = (int)((c.u >> 23) & 255);
+  const uint64_t m = (c.u & 0x7FFFFFu) | (ex ? 0x800000u : 0u);
+  uint64_t X = 0;  // x 2^53 = m 2^(ex - 97)
+  if (ex >= 97) {
+    X = m << (ex - 97 < 30 ? ex - 97 : 30);
+  } else if (ex >= 72) {
+    const int s = 97 - ex;
+    const uint64_t rem = m & ((1ull << s) - 1), half = 1ull << (s - 1);
+    X = m >> s;
+    X += rem > half || (rem == half && (X & 1));
+  }
+  return (1ull << 53) - X;
+}
+
 // Exponent of a double that is zero (-1023) or normal and positive.
 inline int neutral_exponent(double s) {
   uint64_t b;

@@ -178,7 +178,10 @@ cudaError_t launch_crit_finalize(long n3, float* C, const uint8_t* A, cudaStream
 
 // The serial double sum of 1 - x (the neutral fraction's): chunks on the GPU
 // into buf (neutral_bytes; n3 a multiple of 16), then, with buf and x on the
-// host, the sum.
+// host, the sum.  Up to NEUTRAL_HOST cells the host adds the terms itself
+// (buf null): a call of four sets takes 0.29 ms so and 0.35 ms by chunks at
+// 24^3, 0.36 and 0.38 at 32^3, 0.41 both ways at 40^3.
+constexpr long NEUTRAL_HOST = 32L * 32 * 32;
 size_t neutral_bytes(long n3);
 cudaError_t launch_neutral(long n3, const float* x, void* buf, cudaStream_t st);
 double neutral_sum(long n3, const void* buf, const float* x);

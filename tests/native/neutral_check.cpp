@@ -2,6 +2,9 @@
 // the serial sum, for a box of one value x everywhere.
 // Usage: neutral_check <n3> <x> ...
 // Prints "<x> <composed> <serial>" in hexadecimal floats.
+//        neutral_check units <n>
+// Prints "units <cases> <mismatches>": neutral_units against 1.0 - x, n floats
+// of each exponent of [0, 1] and those next to the powers of two.
 //
 // The pairs are made by their definition: the serial additions of a chunk to
 // 2^E and to the next double.  The binades come from the exact sums (n times a
@@ -18,6 +21,26 @@ using namespace sf21;
 
 int main(int argc, char** argv) {
   if (argc < 3) return 2;
+  if (!strcmp(argv[1], "units")) {
+    const long n = atol(argv[2]);
+    long cases = 0, bad = 0;
+    uint32_t r = 1;
+    auto check = [&](uint32_t bits) {
+      float x;
+      memcpy(&x, &bits, 4);
+      if (!(x >= 0.0f && x <= 1.0f)) return;
+      ++cases;
+      bad += ldexp((double)neutral_units(x), -53) != 1.0 - x;
+    };
+    for (uint32_t ex = 0; ex <= 127; ++ex) {
+      for (int d = -3; d <= 3; ++d) check((ex << 23) + (uint32_t)d);
+      for (long i = 0; i < n; ++i) check(ex << 23 | ((r = r * 1664525u + 1013904223u) >> 9));
+      for (int k = 0; k < 23; ++k) check(ex << 23 | 1u << k);  // ties among them
+      for (int k = 0; k < 23; ++k) check(ex << 23 | (0x7FFFFFu >> k << k));
+    }
+    printf("units %ld %ld\n", cases, bad);
+    return 0;
+  }
   const long n3 = atol(argv[1]), chunks = (n3 + NEUTRAL_CHUNK - 1) / NEUTRAL_CHUNK;
   for (int a = 2; a < argc; ++a) {
     const float x = strtof(argv[a], nullptr);

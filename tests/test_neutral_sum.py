@@ -31,3 +31,9 @@ def test_composed_sum_is_the_serial_sum(check, N, values):
     assert len(rows) == len(values)
     for x, got, want in rows:
         assert got == want, x
+
+
+def test_terms_are_multiples_of_2_to_the_minus_53(check):
+    """1.0 - x of the float x in [0, 1], in integers."""
+    out = subprocess.run([check, "units", "20000"], capture_output=True, text=True, check=True).stdout.split()
+    assert int(out[1]) > 2000000 and int(out[2]) == 0
