@@ -152,7 +152,7 @@ struct sf21_hii_ctx {
   float2* d_pk = nullptr;
   float* d_pk_w = nullptr;
   float* d_pk_part = nullptr;
-  float2* d_pk_sum = nullptr;
+  double* d_pk_sum = nullptr;
   unsigned long long* d_pk_cnt = nullptr;
   // 21-cm brightness-temperature buffers (allocated on first use)
   float* d_t21 = nullptr;  // xc, xalpha, TK, T_b boxes
@@ -1529,7 +1529,7 @@ static int power_spectrum_device(sf21_hii_ctx* c, const float* box_dev, int flag
   if (!c->d_pk) CTX_CUDA(c, dev_malloc(&c->d_pk, sizeof(float2) * c->n3));
   if (!c->d_pk_w) CTX_CUDA(c, dev_malloc(&c->d_pk_w, sizeof(float) * N));
   if (!c->d_pk_part) CTX_CUDA(c, dev_malloc(&c->d_pk_part, sizeof(float) * (size_t)grid * nk));
-  if (!c->d_pk_sum) CTX_CUDA(c, dev_malloc(&c->d_pk_sum, sizeof(float2) * nk));
+  if (!c->d_pk_sum) CTX_CUDA(c, dev_malloc(&c->d_pk_sum, sizeof(double) * nk));
   if (!c->d_pk_cnt) CTX_CUDA(c, dev_malloc(&c->d_pk_cnt, sizeof(unsigned long long) * nk));
   std::vector<float> wax(N);
   double s1 = 0.;
@@ -1556,19 +1556,18 @@ static int power_spectrum_device(sf21_hii_ctx* c, const float* box_dev, int flag
   }
   CTX_CUDA(c, cudaMemsetAsync(c->d_pk_cnt, 0, sizeof(unsigned long long) * nk, st));
   CTX_CUDA(c, launch_pk_bin(N, c->d_pk, nk, c->d_pk_part, c->d_pk_cnt, st));
-  CTX_CUDA(c, launch_pk_reduce(N, nk, c->d_pk_part, c->d_pk_sum, st));
-  std::vector<float2> sums(nk);
+  CTX_CUDA(c, launch_pk_reduce(N, nk, c->d_pk_part, reinterpret_cast<uint64_t*>(c->d_pk_sum), st));
+  std::vector<double> sums(nk);
   std::vector<unsigned long long> cnt(nk);
-  CTX_CUDA(c, cudaMemcpyAsync(sums.data(), c->d_pk_sum, sizeof(float2) * nk, cudaMemcpyDeviceToHost, st));
+  CTX_CUDA(c, cudaMemcpyAsync(sums.data(), c->d_pk_sum, sizeof(double) * nk, cudaMemcpyDeviceToHost, st));
   CTX_CUDA(c, cudaMemcpyAsync(cnt.data(), c->d_pk_cnt, sizeof(unsigned long long) * nk, cudaMemcpyDeviceToHost, st));
   CTX_CUDA(c, cudaStreamSynchronize(st));
   const double dk = 2.0 * kPI / (N * dl);
   const double dl3 = dl * dl * dl;
   for (int b = 0; b < nk && b < cap; ++b) {
-    const double sum = (double)sums[b].x + (double)sums[b].y;
     const double n = cnt[b] ? (double)cnt[b] : 1.0;
     k[b] = b * dk;
-    P[b] = sum / n / wsum * dl3;
+    P[b] = sums[b] / n / wsum * dl3;
   }
   *nk_out = nk;
   return SF21_OK;

@@ -10,14 +10,15 @@
 //     power = re^2 + im^2 in float as the tool computes it; per-CTA sums in
 //     shared memory, written out per CTA, counts added exactly with integer
 //     atomics;
-//   k_pk_reduce: one warp per bin adds the CTAs' sums as unevaluated pairs of
-//     floats (48 bits), so a few kilobytes go to the host instead of the
-//     14.6 MB of partial sums at 512^3, which took most of the call there.
+//   k_pk_reduce: adds the CTAs' sums in double (softdouble.h), so a few
+//     kilobytes go to the host instead of the 14.6 MB of partial sums at 512^3,
+//     which took most of the call there.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include "sf21_device.cuh"
 #include "sf21_kernels.h"
+#include "softdouble.h"
 
 namespace sf21 {
 
@@ -82,36 +83,39 @@ k_pk_bin(int N, const float2* __restrict__ spec, int nk, float* __restrict__ par
   }
 }
 
-// (hi, lo) += x, the sum kept to twice the float precision (Knuth's two-sum,
-// then renormalised).
-__device__ __forceinline__ void pair_add(float2& s, float x, float xlo) {
-  const float t = __fadd_rn(s.x, x);
-  const float bb = __fsub_rn(t, s.x);
-  const float e = __fadd_rn(__fsub_rn(s.x, __fsub_rn(t, bb)), __fsub_rn(x, bb));
-  const float l = __fadd_rn(__fadd_rn(s.y, xlo), e);
-  s.x = __fadd_rn(t, l);
-  s.y = __fsub_rn(l, __fsub_rn(s.x, t));
-}
-
-// partials: [ncta][nk]; blockIdx.x covers 32 bins, threadIdx.x = bin, the
-// threadIdx.y rows share the CTAs.
-__global__ void __launch_bounds__(1024) k_pk_reduce(int ncta, int nk, const float* __restrict__ partials,
-                                                    float2* __restrict__ sums) {
-  __shared__ float2 sm[32][33];
-  const int b = blockIdx.x * 32 + threadIdx.x;
-  float2 s = make_float2(0.0f, 0.0f);
+// partials: [ncta][nk], not negative; sums[b]: the double sum of bin b's, in
+// the integer routines of softdouble.h, as bits.  A sum with an infinity is
+// infinite, one with a NaN is NaN (those routines take finite operands only).
+// threadIdx.x = bin of the CTA's PKR_BINS, the threadIdx.y rows share the CTAs:
+// a sum of doubles in integers is a chain of 60 instructions, so a bin has 128
+// of them side by side.
+constexpr int PKR_BINS = 8, PKR_ROWS = 128;
+__global__ void __launch_bounds__(PKR_BINS * PKR_ROWS)
+k_pk_reduce(int ncta, int nk, const float* __restrict__ partials, sd_t* __restrict__ sums) {
+  __shared__ sd_t sm[PKR_ROWS][PKR_BINS + 1];
+  const int b = blockIdx.x * PKR_BINS + threadIdx.x;
+  __shared__ int inf[PKR_BINS], nan[PKR_BINS];
+  if (threadIdx.y == 0) inf[threadIdx.x] = nan[threadIdx.x] = 0;
+  __syncthreads();
+  sd_t s = 0;
   if (b < nk)
-    for (int g = threadIdx.y; g < ncta; g += 32) pair_add(s, partials[(long)g * nk + b], 0.0f);
+    for (int g = threadIdx.y; g < ncta; g += PKR_ROWS) {
+      const float v = partials[(long)g * nk + b];
+      if (isfinite(v)) s = sd_add(s, sd_from_float(v));
+      else (isnan(v) ? nan : inf)[threadIdx.x] = 1;
+    }
   sm[threadIdx.y][threadIdx.x] = s;
   __syncthreads();
-  if (threadIdx.y == 0 && b < nk) {
-    for (int g = 1; g < 32; ++g) pair_add(s, sm[g][threadIdx.x].x, sm[g][threadIdx.x].y);
-    sums[b] = s;
+  for (int o = PKR_ROWS / 2; o > 0; o >>= 1) {
+    if (threadIdx.y < o) sm[threadIdx.y][threadIdx.x] = sd_add(sm[threadIdx.y][threadIdx.x], sm[threadIdx.y + o][threadIdx.x]);
+    __syncthreads();
   }
+  if (threadIdx.y == 0 && b < nk)
+    sums[b] = nan[threadIdx.x] ? SD_QNAN : inf[threadIdx.x] ? 0x7FF0000000000000ULL : sm[0][threadIdx.x];
 }
 
-cudaError_t launch_pk_reduce(int N, int nk, const float* partials, float2* sums, cudaStream_t st) {
-  k_pk_reduce<<<(nk + 31) / 32, dim3(32, 32), 0, st>>>(pk_bin_grid(N), nk, partials, sums);
+cudaError_t launch_pk_reduce(int N, int nk, const float* partials, uint64_t* sums, cudaStream_t st) {
+  k_pk_reduce<<<(nk + PKR_BINS - 1) / PKR_BINS, dim3(PKR_BINS, PKR_ROWS), 0, st>>>(pk_bin_grid(N), nk, partials, sums);
   return cudaGetLastError();
 }
 
