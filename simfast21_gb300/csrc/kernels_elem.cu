@@ -80,7 +80,7 @@ k_prologue(long n3, const float* __restrict__ delta, const float* __restrict__ s
     const sd_t one_d = sd_add(SD_ONE, sd_from_float(d));  // 1. + density_map[i]
     // Each quantity takes its fast path (prologue_fast.h), which returns the
     // exact chain's float for all but about one voxel in 2^18 (Rrec: the
-    // quick path for all but one in 2^15, then the fast one); those voxels
+    // quick path for all but one in 2^14, then the fast one); those voxels
     // evaluate the exact chain.
     // fresid = XHI((float)((1+d) * 1.881e-7 * pow(1+z,3) * G_H(z)))      (:220-221)
     float fr;

@@ -29,11 +29,14 @@
 // floor(a b / 2^62) for signed Q.62 values whose product stays below 2^125.
 SD_HD int64_t pf_mulq62(int64_t a, int64_t b) { return (int64_t)(((sd_i128)a * b) >> 62); }
 
-// Float seeds of the Newton iterations (relative error below 2^-21; the
-// iterations and guard bands allow for it, so host and device may differ).
+// Float seeds of the Newton iterations: relative error up to 2^-21.  The
+// iterations and guard bands allow for all of it (checked on the host with
+// seeds at both ends, PF_SEED_ERR), so host and device may differ.
 SD_HD float pf_seed_recip(float x) {
 #ifdef __CUDA_ARCH__
   return __fdividef(1.0f, x);
+#elif defined(PF_SEED_ERR)  // tests: a seed at the edge of its error
+  return 1.0f / x * (1.0f + PF_SEED_ERR);
 #else
   return 1.0f / x;
 #endif
@@ -261,8 +264,11 @@ SD_HD bool rrec_fast(float od, const RrecFast& k, float* out) {
   return pf_round_guard(Fm, eF, 0u, out);
 }
 
-// The same value to relative 2^-41, with a guard band of 2^24 units (2^-40 or
-// more): it declines for about one input in 2^15, which then takes rrec_fast.
+// The same value, with a guard band of 2^25 units (2^-39 or more): it declines
+// for about one input in 2^14, which then takes rrec_fast.  The error is that
+// of 1 / S four times over: the seed's 2^-21 and the rounding of its argument
+// (2^-24) give 2^-41.6 after the Newton step and 2^-39.6 in the fourth power,
+// which leaves a third of the band to the series (2^-44 each, four times over).
 // The series' terms of third and higher order (below 2^-25) are evaluated in
 // float, the squares from 31-bit factors.  tab: rrec_table's 3 x 128 words.
 SD_HD bool rrec_quick(float od, const RrecFast& k, const uint64_t* tab, float* out) {
@@ -311,7 +317,7 @@ SD_HD bool rrec_quick(float od, const RrecFast& k, const uint64_t* tab, float* o
     S >>= 1;
     es += 1;
   }
-  // 1 / S by one Newton step from a float seed: error below 2^-42
+  // 1 / S by one Newton step from a float seed: error below 2^-41.6
   const float yf = pf_seed_recip((float)(uint32_t)(S >> 32) * (1.0f / 1073741824.0f));
   const uint64_t Y0 = (uint64_t)(uint32_t)(yf * 1073741824.0f) << 32;           // Q.62
   const uint64_t t1 = (1ULL << 61) - sd_mulhi64(S, Y0);                         // 2 - S Y0, Q.60
@@ -325,7 +331,7 @@ SD_HD bool rrec_quick(float od, const RrecFast& k, const uint64_t* tab, float* o
   const uint64_t y4 = pf_mulnorm(y2, y2, &e4);
   int eF = e4 + k.cx - 4 * es;
   const uint64_t Fm = pf_mulnorm(y4, k.cm, &eF);
-  return pf_round_guard(Fm, eF, 0u, out, 1ULL << 24);
+  return pf_round_guard(Fm, eF, 0u, out, 1ULL << 25);
 }
 // Word i of the table: 2^62 / c_j, log2 c_j (Q.62), 2^(j/128) (Q.62).
 SD_HD uint64_t rrec_table(int i) {
