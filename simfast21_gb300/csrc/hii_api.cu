@@ -1467,7 +1467,7 @@ static int enqueue_halo_source(sf21_hii_ctx* c, double z, long nhalos, const voi
   if (c->N_halo < c->N) CTX_FAIL(c, SF21_E_ARG, "N_halo < N_smoothed (smooth_box, auxiliary.c:651-654)");
   if (nhalos >= (1L << 28)) CTX_FAIL(c, SF21_E_UNSUPPORTED, "2^28 halos or more (8 CIC entries each, int count)");
   const long nh3 = c->N_halo * c->N_halo * c->N_halo;
-  if (!c->d_fine && !halo_by_tiles(c->N_halo, c->N)) CTX_CUDA(c, dev_malloc(&c->d_fine, sizeof(float) * nh3));
+  if (!c->d_fine && halo_needs_grid(c->N_halo, c->N)) CTX_CUDA(c, dev_malloc(&c->d_fine, sizeof(float) * nh3));
   if (nhalos > c->halo_cap) {
     if (c->d_halos) cudaFree(c->d_halos);
     if (c->d_hscratch) cudaFree(c->d_hscratch);

@@ -278,6 +278,7 @@ struct SmoothArgs {
   sd_divc sm3;     // sm^3 as a divisor
   int post;        // 1: divide by post_div
   sd_divc post_div;
+  float inv_sm3_hi, inv_sm3_lo;  // 1 / sm^3
   float inv_hi, inv_lo;  // 1 / post divisor, where it is of a moderate size (else 0: never sure)
   float zero;            // the average of a block of zeros
 };
@@ -409,6 +410,8 @@ static SmoothArgs smooth_args(long N_halo, long N_smooth, double post_div) {
   a.post = post_div != 0.0;
   memcpy(&b, &post_div, 8);
   a.post_div = sd_divc_prepare(a.post ? b : 0x3FF0000000000000ULL);
+  a.inv_sm3_hi = (float)(1.0 / sm3);
+  a.inv_sm3_lo = (float)(1.0 / sm3 - (double)a.inv_sm3_hi);
   const bool moderate = a.post && post_div > 0x1p-50 && post_div < 0x1p50;
   a.inv_hi = moderate ? (float)(1.0 / post_div) : 0.f;
   a.inv_lo = moderate ? (float)(1.0 / post_div - (double)a.inv_hi) : 0.f;
@@ -430,7 +433,7 @@ static unsigned grid_for(long n) {
 }
 
 // ---------------------------------------------------------------------------
-// Deposit and block average by tiles of the fine grid, for blocks of up to 16
+// Deposit and block average by tiles of the fine grid, for blocks of up to 4
 // cells a side.
 //
 // The entries above are eight per halo, sorted as (cell, double) pairs, and
@@ -446,17 +449,23 @@ static unsigned grid_for(long n) {
 // and the others go again, until none waits.  Within a run the halos keep
 // their order (the sort is stable); when a tile has more of them than the CTA
 // has threads, it takes those below a serial number that leaves no run behind.
-// The block average follows from shared memory; no grid is stored.
+// The block average follows from shared memory, for the blocks that have a
+// contribution, in pairs of floats; no grid is stored.
 //
-// 1200^3 cells, 2 10^7 halos: 14.6 -> 7.6 ms, of which this kernel 6.1 and the
+// 1200^3 cells, 2 10^7 halos: 14.6 -> 7.3 ms, of which this kernel 5.8 and the
 // two sorts 1.0.  It is bound by its instructions (the pairs of floats below)
 // and by the barriers of the rounds: 64 to 256 threads, tiles of 1024 to 8192
 // cells and 24 to 64 KB were within 10 %, a tile of 4096 cells and 96 threads
 // (47 halos in it on average, 60 with those of its neighbours) the fastest.
 constexpr int TILE_THREADS = 96;
-constexpr int TILE_X = 8, TILE_Y = 16, TILE_Z = 32;  // cells, for block sides 1 and 2
 constexpr int TILE_CTAS = 6;
-constexpr int TILE_MAX_SM = 16;
+constexpr int TILE_MAX_SM = 4;  // block sides that have tiles
+// Cells of a tile: whole blocks of sm cells, about 8 x 16 x 32, long in z for
+// the result's rows; 32 KB of shared memory, and a halo is in 1.27 tiles on
+// average
+__host__ __device__ constexpr int tile_x(int sm) { return sm == 3 ? 9 : 8; }
+__host__ __device__ constexpr int tile_y(int sm) { return 16 / sm * sm; }
+__host__ __device__ constexpr int tile_z(int sm) { return 32 / sm * sm; }
 
 struct HaloTiles {
   int N, tx, ty, tz;     // cells of the fine grid and of a tile: whole blocks of sm
@@ -465,15 +474,11 @@ struct HaloTiles {
 };
 
 static HaloTiles halo_tiles(long N_halo, long sm) {
-  // whole blocks of sm cells, about TILE_X x TILE_Y x TILE_Z: long in z for the
-  // result's rows; 32 KB of shared memory (64 KB at sm = 16), and a halo is in
-  // 1.27 tiles on average
   HaloTiles t;
-  auto side = [&](int want) { return (int)(sm * std::max(1L, want / sm)); };
   t.N = (int)N_halo;
-  t.tx = side(TILE_X);
-  t.ty = side(TILE_Y);
-  t.tz = side(TILE_Z);
+  t.tx = tile_x((int)sm);
+  t.ty = tile_y((int)sm);
+  t.tz = tile_z((int)sm);
   t.nx = (t.N + t.tx - 1) / t.tx;
   t.ny = (t.N + t.ty - 1) / t.ty;
   t.nz = (t.N + t.tz - 1) / t.tz;
@@ -538,8 +543,7 @@ __global__ void k_halo_starts(long nh, const uint32_t* __restrict__ keys, long n
 // and where a value is not finite, negative or so small that a low part could
 // be lost, the soft-double chain runs.  (All of it in soft double: 24 000
 // instructions a tile and half of the time waiting for instructions, 33 ms for
-// 1200^3 cells and 2 10^7 halos; 35 doubles a clock and SM on the FP64 unit
-// would be no faster.)
+// 1200^3 cells and 2 10^7 halos.)
 struct FPair {
   float hi, lo;
 };
@@ -562,6 +566,10 @@ __device__ __forceinline__ FPair fp_add(FPair a, float v) {
   const float e = __fadd_rn(__fsub_rn(a.hi, __fsub_rn(s, t)), __fsub_rn(v, t));
   return fp_norm(s, __fadd_rn(e, a.lo));
 }
+__device__ __forceinline__ FPair fp_add2(FPair a, FPair b) {
+  const FPair s = fp_add(a, b.hi);
+  return fp_norm(s.hi, __fadd_rn(s.lo, b.lo));
+}
 // a.hi is the float nearest to every value within 2^-40 of a (and a is of a
 // size at which no low part was lost)
 __device__ __forceinline__ bool fp_sure(FPair a) {
@@ -581,6 +589,21 @@ __device__ __noinline__ float corner_exact(float acc, float4 h, int N, int k) {
   return sd_to_float(sd_add(sd_from_float(acc), w));
 }
 
+// A row of a block
+template <int SM>
+__device__ __forceinline__ void block_row(const float* p, float (&v)[SM]) {
+  if constexpr (SM == 4) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+  } else if constexpr (SM == 2) {
+    const float2 q = *reinterpret_cast<const float2*>(p);
+    v[0] = q.x, v[1] = q.y;
+  } else {
+#pragma unroll
+    for (int k = 0; k < SM; k++) v[k] = p[k];
+  }
+}
+
 // The block average of sm^3 cells in shared memory, rows and planes sy and sx apart
 __device__ __noinline__ float block_exact(const float* v, int sx, int sy, int sm, const SmoothArgs& a) {
   return smooth_value(rows_sum(v, sx, sy, sm), a);
@@ -593,15 +616,14 @@ k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __
   extern __shared__ __align__(16) float tile_fine[];
   __shared__ uint32_t cur[32], take[32];
   __shared__ uint32_t left;  // halos that have not been taken
-  // SM 1 and 2: the tile's sides are constants
-  const int TX = SM ? TILE_X : t.tx, TY = SM ? TILE_Y : t.ty, TZ = SM ? TILE_Z : t.tz;
-  const int cells = (TX * TY * TZ + 3) & ~3;  // whole float4
+  constexpr int TX = tile_x(SM), TY = tile_y(SM), TZ = tile_z(SM);
+  constexpr int cells = (TX * TY * TZ + 3) & ~3;  // whole float4
   uint32_t* slot = reinterpret_cast<uint32_t*>(tile_fine + cells);
   const int tz = blockIdx.x % t.nz, ty = blockIdx.x / t.nz % t.ny, tx = blockIdx.x / t.nz / t.ny;
   const int x0 = tx * TX, y0 = ty * TY, z0 = tz * TZ;
-  const int sm = SM ? SM : (int)a.sm, Ns = (int)a.Ns;
-  const int ox = x0 / sm, oy = y0 / sm, oz = z0 / sm;  // the tile's part of the result
-  const int MX = TX / sm, MY = TY / sm, MZ = TZ / sm;
+  const int Ns = (int)a.Ns;
+  const int ox = x0 / SM, oy = y0 / SM, oz = z0 / SM;  // the tile's part of the result
+  constexpr int MX = TX / SM, MY = TY / SM, MZ = TZ / SM;
   if (ox >= Ns || oy >= Ns || oz >= Ns) return;  // cells beyond the last block
   const int lane = threadIdx.x & 31;
   uint32_t end = 0;  // of the lane's run (warp 0)
@@ -746,7 +768,7 @@ k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __
   __syncthreads();
   const auto where = [&](int o, int* b) {  // block o's cells, and its place in the result (-1: outside)
     const int p = o % MZ, j = o / MZ % MY, i = o / MZ / MY;
-    *b = ((i * sm) * TY + j * sm) * TZ + p * sm;
+    *b = ((i * SM) * TY + j * SM) * TZ + p * SM;
     return ox + i < Ns && oy + j < Ns && oz + p < Ns ? ((long)(ox + i) * Ns + oy + j) * Ns + oz + p : -1L;
   };
   for (int o0 = threadIdx.x - lane; o0 < MX * MY * MZ; o0 += TILE_THREADS) {
@@ -755,17 +777,15 @@ k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __
     long dst = o < MX * MY * MZ ? where(o, &b) : -1;
     bool zero = true;
     if (dst >= 0 && any) {
-      if constexpr (SM == 1) {
-        zero = tile_fine[b] == 0.0f;
-      } else if constexpr (SM == 2) {
+      uint32_t bits = 0;  // (comparisons chained by && wait for one load after the other)
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const float2 v = *reinterpret_cast<const float2*>(tile_fine + b + (k >> 1) * TY * TZ + (k & 1) * TZ);
-          zero = zero && v.x == 0.0f && v.y == 0.0f;
-        }
-      } else {
-        zero = false;
+      for (int r = 0; r < SM * SM; r++) {
+        float v[SM];
+        block_row<SM>(tile_fine + b + (r / SM) * TY * TZ + (r % SM) * TZ, v);
+#pragma unroll
+        for (int k = 0; k < SM; k++) bits |= __float_as_uint(v[k]);
       }
+      zero = bits << 1 == 0;
     }
     if (dst >= 0 && zero) out[dst] = a.zero;
     const uint32_t m = __ballot_sync(0xffffffffu, !zero);
@@ -775,44 +795,84 @@ k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __
     if (!zero) list[at + __popc(m & ((1u << lane) - 1u))] = (uint16_t)o;
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < (int)listed; k += TILE_THREADS) {
-    int b;
-    const long dst = where(list[k], &b);
+  // Side 4: a block's planes to four lanes, since a tile has few blocks then
+  // and the chain of 64 cells would be longer than all the rest
+  constexpr int LANES = SM == 4 ? 4 : 1, PLANES = SM / LANES;
+  for (int k0 = threadIdx.x - lane; k0 < (int)listed * LANES; k0 += TILE_THREADS) {
+    const int k = (k0 + lane) / LANES;
+    int b = 0;
+    const long dst = k < (int)listed ? where(list[k], &b) : -1;
     const float* c = tile_fine + b;
     float v = 0.f;
     bool sure = false;
-    if constexpr (SM == 1 || SM == 2) {
-      FPair q = {c[0], 0.f};
-      if constexpr (SM == 2) {
-        q = fp_add(q, c[1]);
+    FPair part[PLANES];  // each plane's sum: the chains run side by side
 #pragma unroll
-        for (int r = 1; r < 4; r++) {
-          const float2 u = *reinterpret_cast<const float2*>(c + (r >> 1) * TY * TZ + (r & 1) * TZ);
-          q = fp_add(fp_add(q, u.x), u.y);
-        }
-      }
-      // the average is a power of two away from the sum; the quotient by the
-      // post divisor is that of the rounded average
-      if (fp_sure(q)) {
-        v = q.hi * (SM == 1 ? 1.0f : 0.125f);
-        sure = true;
-        if (a.post) {
-          const FPair d = fp_scale({a.inv_hi, a.inv_lo}, v);
-          sure = fp_sure(d);
-          v = d.hi;
-        }
+    for (int y = 0; y < SM; y++) {
+      float u[PLANES][SM];
+#pragma unroll
+      for (int x = 0; x < PLANES; x++) block_row<SM>(c + (lane % LANES + x) * TY * TZ + y * TZ, u[x]);
+#pragma unroll
+      for (int z = 0; z < SM; z++)
+#pragma unroll
+        for (int x = 0; x < PLANES; x++) part[x] = y + z ? fp_add(part[x], u[x][z]) : FPair{u[x][0], 0.f};
+    }
+    FPair q = part[0];
+#pragma unroll
+    for (int x = 1; x < PLANES; x++) q = fp_add2(q, part[x]);
+#pragma unroll
+    for (int o = 1; o < LANES; o <<= 1)
+      q = fp_add2(q, {__shfl_xor_sync(0xffffffffu, q.hi, o), __shfl_xor_sync(0xffffffffu, q.lo, o)});
+    if (dst < 0 || lane % LANES) continue;
+    // the average of 1, 8 or 64 cells is a power of two away from the sum; the
+    // quotient by the post divisor is that of the rounded average
+    if constexpr (SM == 3) q = fp_mul(q, {a.inv_sm3_hi, a.inv_sm3_lo});
+    if (fp_sure(q)) {
+      v = SM == 3 ? q.hi : q.hi * (1.0f / (SM * SM * SM));
+      sure = true;
+      if (a.post) {
+        const FPair d = fp_scale({a.inv_hi, a.inv_lo}, v);
+        sure = fp_sure(d);
+        v = d.hi;
       }
     }
-    if (!sure) v = block_exact(c, TY * TZ, TZ, sm, a);
+    if (!sure) v = block_exact(c, TY * TZ, TZ, SM, a);
     out[dst] = v;
   }
 }
 
-// The tiles take every block side that fits shared memory; larger blocks (few
-// smoothed cells for many fine ones) and grids beyond 2048 keep the fine grid.
-bool halo_by_tiles(long N_halo, long N_smooth) {
+// Which deposit takes a catalogue (fine: the fine grid in memory, tiles: the
+// kernel above; ms a call).
+//
+// Block sides up to 4 have tiles.  0.0001, 0.001 and 0.01 halos per cell:
+//   480 -> 160   fine 0.39, 0.48, 1.05   tiles 0.25, 0.36, 0.53
+//   480 -> 120   fine 0.36, 0.44, 1.02   tiles 0.24, 0.40, 0.67
+//   1200 -> 300  fine 2.69, 3.84, 12.3   tiles 1.59, 3.87, 8.32
+// From 5 up a tile has too few blocks for its threads (with the blocks' cells in
+// a loop: 480 -> 96, fine 0.36, 0.44, 1.04, tiles 0.40, 0.90, 1.51; 480 -> 30,
+// fine 1.27, 1.49, 2.83, tiles 4.2, 7.6, 18.9).
+//
+// Where the tiles are fewer than two an SM (up to about 100^3 cells), they wait
+// for the rounds of their halos, and from 70 sm halos a tile the sort of the
+// contributions is done first:
+//   48^3, side 1   0.01 per cell: fine 0.11, tiles 0.08;  0.1: 0.17, 0.22;  1: 0.27, 0.73
+//   72^3, side 3   0.02:          0.18, 0.15;             0.1: 0.20, 0.21;  2: 1.13, 1.28
+//   108^3, side 1  0.02:          0.19, 0.18;             0.1: 0.25, 0.25;  2: 3.30, 1.62
+// Grids beyond 2048 keep the fine grid.
+static bool has_tiles(long N_halo, long N_smooth) {
   const long sm = block_side(N_halo, N_smooth);
   return sm >= 1 && sm <= TILE_MAX_SM && N_halo <= 2048;
+}
+constexpr long FEW_TILES = 300;
+static bool few_tiles(long N_halo, long N_smooth) {
+  return halo_tiles(N_halo, block_side(N_halo, N_smooth)).keys() / 8 < FEW_TILES;
+}
+static bool by_tiles(long nh, long N_halo, long N_smooth) {
+  if (!has_tiles(N_halo, N_smooth)) return false;
+  const long sm = block_side(N_halo, N_smooth), tiles = halo_tiles(N_halo, sm).keys() / 8;
+  return tiles >= FEW_TILES || nh < 70 * sm * tiles;
+}
+bool halo_needs_grid(long N_halo, long N_smooth) {
+  return !has_tiles(N_halo, N_smooth) || few_tiles(N_halo, N_smooth);
 }
 
 size_t halo_scratch_bytes(long nh, long N_halo, long N_smooth) {
@@ -820,13 +880,15 @@ size_t halo_scratch_bytes(long nh, long N_halo, long N_smooth) {
   cub::DeviceRadixSort::SortKeys(nullptr, key_tmp, (uint32_t*)nullptr, (uint32_t*)nullptr, (int)nh);
   cub::DeviceSelect::Unique(nullptr, uniq_tmp, (uint32_t*)nullptr, (uint32_t*)nullptr, (int*)nullptr, (int)nh);
   size_t tmp = std::max(key_tmp, uniq_tmp);
-  if (halo_by_tiles(N_halo, N_smooth)) {
+  size_t bytes = 0;
+  if (has_tiles(N_halo, N_smooth)) {
     size_t pairs = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, pairs, (uint32_t*)nullptr, (uint32_t*)nullptr, (uint32_t*)nullptr,
                                     (uint32_t*)nullptr, (int)nh);
     // records | keys and indices, twice | masses and weights | starts | CUB temporary storage
-    return (size_t)nh * 40 + 4 * (size_t)(halo_tiles(N_halo, block_side(N_halo, N_smooth)).keys() + 1) +
-           std::max(tmp, pairs) + 4096;
+    bytes = (size_t)nh * 40 + 4 * (size_t)(halo_tiles(N_halo, block_side(N_halo, N_smooth)).keys() + 1) +
+            std::max(tmp, pairs) + 4096;
+    if (!few_tiles(N_halo, N_smooth)) return bytes;
   }
   const long ne = 8 * nh;
   size_t t64 = 0, t32 = 0;
@@ -836,7 +898,7 @@ size_t halo_scratch_bytes(long nh, long N_halo, long N_smooth) {
                                   (sd_t*)nullptr, (int)ne);
   tmp = std::max(tmp, std::max(t64, t32));
   // k0 | k1 (8 B each) | v0 | v1 (8 B each) | CUB temporary storage
-  return (size_t)ne * 32 + tmp + 4096;
+  return std::max(bytes, (size_t)ne * 32 + tmp + 4096);
 }
 
 static uint64_t bits_of(double d) {
@@ -912,16 +974,17 @@ static cudaError_t source_by_tiles(long nh, const HaloRec* halos, const RionCons
   }
   if (a.sm == 1) return tiles_launch<1>(t, start, i1, rec, out, a, st);
   if (a.sm == 2) return tiles_launch<2>(t, start, i1, rec, out, a, st);
-  return tiles_launch<0>(t, start, i1, rec, out, a, st);
+  if (a.sm == 3) return tiles_launch<3>(t, start, i1, rec, out, a, st);
+  return tiles_launch<4>(t, start, i1, rec, out, a, st);
 }
 
-// fine: N_halo^3 floats, not used when halo_by_tiles
+// fine: N_halo^3 floats, used only if halo_needs_grid
 cudaError_t launch_halo_source(long nh, const void* halos_dev, double z, long N_halo, long N_smooth, float* fine,
                                float* out, void* scratch, size_t scratch_bytes, cudaStream_t st, double qion,
                                double post_div) {
   const RionConst rk = rion_const(z, qion);
   const HaloRec* hrec = (const HaloRec*)halos_dev;
-  if (halo_by_tiles(N_halo, N_smooth))
+  if (by_tiles(nh, N_halo, N_smooth))
     return source_by_tiles(nh, hrec, rk, N_halo, N_smooth, out, scratch, scratch_bytes, post_div, st);
   const long ne = 8 * nh;
   const long Nh3 = N_halo * N_halo * N_halo;

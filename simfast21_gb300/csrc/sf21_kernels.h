@@ -191,7 +191,7 @@ double neutral_sum(long n3, const void* buf, const float* x);
 // {float Mass, x, y, z}; fine: N_halo^3 floats; out: N_smooth^3 floats.
 // qion != 0: the weight is Rion / qion (sfr, get_SFR.c:119-121); post_div != 0:
 // each smoothed cell is then divided by it (get_SFR.c:129-131).
-bool halo_by_tiles(long N_halo, long N_smooth);  // launch_halo_source needs no fine grid
+bool halo_needs_grid(long N_halo, long N_smooth);  // some catalogue goes through launch_halo_source's fine grid
 size_t halo_scratch_bytes(long nh, long N_halo, long N_smooth);
 cudaError_t launch_halo_source(long nh, const void* halos_dev, double z, long N_halo, long N_smooth, float* fine,
                                float* out, void* scratch, size_t scratch_bytes, cudaStream_t st, double qion = 0.0,

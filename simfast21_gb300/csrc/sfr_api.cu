@@ -90,7 +90,7 @@ extern "C" int sf21_sfr_create(const sf21_sfr_config* cfg, sf21_sfr_ctx** out) {
   } while (0)
   SCREATE(cudaSetDevice(cfg->device));
   SCREATE(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
-  if (!halo_by_tiles(cfg->N_halo, cfg->N_smoothed)) SCREATE(dev_malloc(&c->d_fine, sizeof(float) * c->n3_halo));
+  if (halo_needs_grid(cfg->N_halo, cfg->N_smoothed)) SCREATE(dev_malloc(&c->d_fine, sizeof(float) * c->n3_halo));
   SCREATE(dev_malloc(&c->d_out, sizeof(float) * c->n3));
 #undef SCREATE
   *out = c;
