@@ -916,6 +916,13 @@ static int check_run_args(sf21_hii_ctx* c, int kind, const void* delta, const vo
 static int enqueue_run(sf21_hii_ctx* c, double z, int kind, const float* delta_dev, const float* src_dev,
                        float* xhii_dev, cudaStream_t st) {
   int rc;
+  // every set's finish reads the source: where an output box covers it, it is copied first
+  const size_t bf = sizeof(float) * c->n3;
+  const uintptr_t s0 = (uintptr_t)src_dev, x0 = (uintptr_t)xhii_dev;
+  if (s0 < x0 + bf * c->sets.size() && x0 < s0 + bf) {
+    CTX_CUDA(c, cudaMemcpyAsync(c->d_src, src_dev, bf, cudaMemcpyDeviceToDevice, st));
+    src_dev = c->d_src;
+  }
   if ((rc = enqueue_front(c, z, kind, delta_dev, src_dev, st))) return rc;
   for (int s = 0; s < (int)c->sets.size(); ++s) {
     if ((rc = enqueue_radii(c, s, st))) return rc;

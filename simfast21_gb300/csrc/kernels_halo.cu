@@ -452,8 +452,7 @@ static unsigned grid_for(long n) {
 // The block average follows from shared memory, for the blocks that have a
 // contribution, in pairs of floats; no grid is stored.
 //
-// 1200^3 cells, 2 10^7 halos: 14.6 -> 7.3 ms, of which this kernel 5.8 and the
-// two sorts 1.0.  It is bound by its instructions (the pairs of floats below)
+// 1200^3 cells, 2 10^7 halos: 14.6 -> 7.3 ms, of which the two sorts take 1.0.  It is bound by its instructions (the pairs of floats below)
 // and by the barriers of the rounds: 64 to 256 threads, tiles of 1024 to 8192
 // cells and 24 to 64 KB were within 10 %, a tile of 4096 cells and 96 threads
 // (47 halos in it on average, 60 with those of its neighbours) the fastest.
