@@ -58,8 +58,14 @@ typedef struct {
   int device;        /* CUDA device ordinal                                 */
   int nsets;         /* parameter sets sharing each forward transform (>=1) */
   const sf21_hii_set *sets;
-  int kmax;          /* radii per spectrum read (0 = automatic: the
-                        autotuner picks 8, 6 or 4; else fixed, <= 8)       */
+  int kmax;          /* radii per batch, and work boxes of 8 N^3 bytes (<= 8;
+                        larger values are taken as 8).  The passes over
+                        pairs of radii take pairs only: one radius less when
+                        it is odd.  1 = the passes for single radii.  0 =
+                        automatic: 8 boxes, the radii of a batch (8, 6 or 4)
+                        tuned; N <= 80 with the pair passes: up to 64 radii
+                        in one launch of each pass, in work boxes of 104 MB
+                        at most in all                                     */
   int path;          /* radius pipeline: 0 = tuned at create (times one batch
                         of each available one at each candidate batch size
                         and keeps the least time per radius; the timings
@@ -70,11 +76,15 @@ typedef struct {
                         thread-block clusters (N 64..512), 3 = three axis
                         passes with the ky pass TMA-pipelined and
                         persistent, 4 = ky and kx passes TMA-pipelined
-                        (3 and 4: N 64..1024), 5-7 = the same over
+                        (3 and 4: N 64..1024), 5 = three axis passes over
+                        pairs of radii (kmax = 1: over single radii in
+                        column-block-major boxes), 6 and 7 = 3 and 4 over
                         column-block-major work boxes, 8 = column-block-
                         major c-axis pass + one persistent launch running
                         the ky and kx passes slab by slab through L2
-                        (N 64..512) */
+                        (N 64..512).  Sides that are not powers of two: 0 or
+                        1, the pair passes where the side has them and kmax
+                        is not 1, else three axis passes */
   int graph;         /* 0 = sf21_hii_run_z_device captures its per-redshift
                         schedule as a CUDA graph and replays it while z, the
                         kind, the buffers and the stream stay the same;
@@ -239,8 +249,9 @@ int sf21_hii_vjp_device(sf21_hii_ctx *ctx, double z, int src_kind, const float *
 int sf21_hii_path(const sf21_hii_ctx *ctx, double *ms_tuned, int cap);
 
 /* Radii per spectrum read (batch size K) in use: kmax when the config fixed
- * it, else the autotuner's choice among kmax (<= 8), 6 and 4 (least time per
- * radius together with the pipeline).  No reference counterpart. */
+ * it, else the autotuner's choice among 8, 6 and 4 (least time per radius
+ * together with the pipeline); see sf21_hii_config.kmax for the radii that a
+ * launch takes.  No reference counterpart. */
 int sf21_hii_batch_radii(const sf21_hii_ctx *ctx);
 
 /* Synchronises the context's stream and reports SF21_E_TIMEOUT if a bounded

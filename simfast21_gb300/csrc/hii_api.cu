@@ -391,8 +391,11 @@ static int prologue_args(sf21_hii_ctx* c, double z, int kind, PrologueArgs* pa) 
   return SF21_OK;
 }
 
-// The passes over radius pairs read slot K of a batch with an odd number K of
-// radii: the last radius again, with the next work box.
+// The passes over radius pairs take an even number of radii at a time: all the
+// work boxes (kmax of them when the caller asks for an odd number) but one.
+static int pair_radii(int K) { return K & ~1; }
+// They read slot K of a batch with an odd number K of radii (the last batch of
+// a set): the last radius again, with the next work box.
 static void pad_pair(const sf21_hii_ctx* c, Batch& bt) {
   if ((bt.K & 1) && bt.K < (int)c->d_work.size()) {
     bt.r[bt.K] = bt.r[bt.K - 1];
@@ -489,12 +492,12 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
   CREATE_CUDA(dev_malloc(&c->d_spec, box_c));
   CREATE_CUDA(dev_malloc(&c->d_rc, c->n3));
   // passes over pairs of radii (pipeline 5, and the one of the sides that are
-  // not powers of two): an even number of boxes.  Sides that are not powers
-  // of two take one radius at a time when only one box is asked for.
+  // not powers of two).  One radius at a time goes through the passes for
+  // single radii, which need one box only.
   const PairOps* po = pair_ops((int)N);
   if (po) CREATE_CUDA(po->setup());
   c->nat = po;
-  if (c->gen ? (po && K > 1) : (cfg->path == 0 || cfg->path == 5)) c->pair = po;
+  if (K > 1 && (c->gen || cfg->path == 0 || cfg->path == 5)) c->pair = po;
   // Small boxes take more radii to a launch, several to a grid row, while the
   // boxes of all of them are well inside the L2: a launch takes 1.5 us and
   // fills a part of the device.  64^3, 43 radii: 111 us with 8 to a launch,
@@ -502,7 +505,7 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
   c->K_launch = K;
   if (c->pair && cfg->kmax <= 0)
     c->K_launch = (int)std::max<long>(K, std::min<long>(po->launch_radii, (104L << 20) / (long)box_c / KMAX * KMAX));
-  const int Kw = c->pair ? c->K_launch + (c->K_launch & 1) : K;
+  const int Kw = c->K_launch;
   c->d_work.assign(Kw, nullptr);
   CREATE_CUDA(dev_malloc(&c->d_work_base, box_c * Kw));
   for (int k = 0; k < Kw; ++k) c->d_work[k] = c->d_work_base + (size_t)k * c->n3;
@@ -604,10 +607,10 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
           bt.r[k].ridx = k;
           bt.r[k].work = c->d_work[k];
         }
-        pad_pair(c, bt);
         for (int p = 1; p <= NPATH; ++p) {
           if (!available(p)) continue;
           c->path = p;
+          bt.K = use_pairs(c) ? pair_radii(Kc) : Kc;
           for (int rep = 0; rep < 4; ++rep) {
             CREATE_CUDA(cudaEventRecord(t0, c->stream));
             if (enqueue_batch(c, bt, c->stream) != SF21_OK) {
@@ -621,6 +624,7 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
             CREATE_CUDA(cudaEventSynchronize(t1));
             float ms = 0.f;
             CREATE_CUDA(cudaEventElapsedTime(&ms, t0, t1));
+            ms *= (float)Kc / bt.K;  // of Kc radii
             if (rep > 0 && ms < ms_p[p]) ms_p[p] = ms;  // the first run warms up
           }
         }
@@ -803,11 +807,14 @@ static int enqueue_batch(sf21_hii_ctx* c, const Batch& bt, cudaStream_t st) {
     span(c, KD_ICA, e2, e3);
     return SF21_OK;
   }
-  if (c->path >= 6) {  // column-block-major work boxes, TMA-pipelined passes
+  if (c->path >= 5) {  // column-block-major work boxes, one radius or TMA-pipelined passes
     int e0 = mark(c, st);
     CTX_CUDA(c, launch_rows_filter_cb(N, c->d_spec, bt, c->d_tw, st));
     int e1 = mark(c, st);
-    CTX_CUDA(c, launch_pipe(N, 0, 1, c->pmaps, bt, c->d_work_base, c->d_rc, c->d_alpha, c->d_tw, c->d_err,
+    if (c->path == 5)
+      CTX_CUDA(c, launch_cols_b_cb(N, bt, c->d_tw, st));
+    else
+      CTX_CUDA(c, launch_pipe(N, 0, 1, c->pmaps, bt, c->d_work_base, c->d_rc, c->d_alpha, c->d_tw, c->d_err,
                               c->nsm, st, c->wait_limit));
     int e2 = mark(c, st);
     if (c->path == 7)
@@ -861,7 +868,7 @@ static int enqueue_radii(sf21_hii_ctx* c, int set, cudaStream_t st) {
   c->rc_clear = false;
   if (c->path == 8) CTX_CUDA(c, cudaMemsetAsync(c->d_rc32, 0xFF, sizeof(unsigned int) * c->n3, st));
   const int nr = (int)s.R.size();
-  const int per = use_pairs(c) && c->K_launch > c->K ? c->K_launch : c->K;
+  const int per = !use_pairs(c) ? c->K : c->K_launch > c->K ? c->K_launch : pair_radii(c->K);
   for (int k0 = 0; k0 < nr; k0 += per) {
     Batch bt;
     memset(&bt, 0, sizeof(bt));
@@ -1292,11 +1299,14 @@ static int enqueue_recompute(sf21_hii_ctx* c, const Batch& bt, cudaStream_t st) 
   return SF21_OK;
 }
 
+// radii per batch of the criterion and the VJP
+static int adj_radii(const sf21_hii_ctx* c) { return c->pair ? pair_radii(c->K) : c->K; }
+
 static Batch make_batch(const sf21_hii_ctx* c, int set, int k0, int nr) {
   const SetInfo& s = c->sets[set];
   Batch bt;
   memset(&bt, 0, sizeof(bt));
-  bt.K = nr - k0 < c->K ? nr - k0 : c->K;
+  bt.K = std::min(nr - k0, adj_radii(c));
   bt.set = set;
   bt.zmul = (float)s.fesc;
   for (int k = 0; k < bt.K; ++k) {
@@ -1321,7 +1331,7 @@ extern "C" int sf21_hii_criterion_device(sf21_hii_ctx* c, double z, int kind, co
   const int N = (int)c->N;
   CTX_CUDA(c, launch_crit_init(c->n3, c->d_C, c->d_A, st));
   const int nr = c->sets[set].n_fft;  // radii of the FFT branch (R >= 2 dx)
-  for (int k0 = 0; k0 < nr; k0 += c->K) {
+  for (int k0 = 0; k0 < nr; k0 += adj_radii(c)) {
     Batch bt = make_batch(c, set, k0, nr);
     if ((rc = enqueue_recompute(c, bt, st))) return rc;
     int e0 = mark(c, st);
@@ -1366,7 +1376,7 @@ extern "C" int sf21_hii_vjp_device(sf21_hii_ctx* c, double z, int kind, const fl
   Batch none;
   memset(&none, 0, sizeof(none));
   const int nr = c->sets[set].n_fft;
-  for (int k0 = 0; k0 < nr; k0 += c->K) {
+  for (int k0 = 0; k0 < nr; k0 += adj_radii(c)) {
     Batch bt = make_batch(c, set, k0, nr);
     if ((rc = enqueue_recompute(c, bt, st))) return rc;
     int e0 = mark(c, st);

@@ -85,6 +85,59 @@ k_rows_filter_cb(const float2* __restrict__ spec, Batch bt, const float2* __rest
                      (int)(row / N), (int)(row % N), j);
 }
 
+// b-axis inverse pass in place: tile (a, column block) = one contiguous run
+// of N CW values per radius.  One CTA per tile (blockIdx.x = cb N + a) walks
+// the K radii with two register sets in turn, the loads of radius k + 1 in
+// flight during the transform of radius k.  (A persistent form with
+// prefetch across tiles, as in the a-axis pass below, measured 5 % slower
+// here: this pass is at the HBM roofline and the hardware's dynamic tile
+// order keeps the concurrent tiles' accesses closer together.)
+//
+// A CTA takes the whole column block: with 16 columns a warp covers 16
+// lines x 2 threads, whose shared-memory exchanges of the line FFT are free of
+// bank conflicts.  (Half blocks of 8 columns, two CTAs per SM, measured
+// slower even with a conflict-free exchange padding.)
+template <int N>
+__global__ void __launch_bounds__(KGeom<N>::THREADS, KGeom<N>::PER_SM)
+k_cols_b_cb(Batch bt, const float2* __restrict__ gtw) {
+  using G = CbGeom<N>;
+  using X = KGeom<N>;
+  extern __shared__ float2 dsm[];
+  float2* stw = dsm;
+  float2* sbuf = dsm + N;
+  for (int t = threadIdx.x; t < N; t += blockDim.x) stw[t] = gtw[t];
+  const int col = threadIdx.x % X::KW;
+  const int j = threadIdx.x / X::KW;
+  const long off = (long)blockIdx.x * N * G::CW + col;  // element (b = 0) of this column
+  auto load = [&](float2 (&v)[8], int k) {
+    const float2* box = bt.r[k].work + off;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v[r] = box[(j + r * (N / 8)) * G::CW];
+  };
+  auto store = [&](const float2 (&v)[8], int k) {
+    float2* box = bt.r[k].work + off;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) box[(j + r * (N / 8)) * G::CW] = v[r];
+  };
+  float2* s0 = sbuf + col * X::LS;
+  float2* s1 = sbuf + (X::KW + col) * X::LS;
+  float2 va[8], vb[8];
+  load(va, 0);
+  __syncthreads();  // twiddles
+  for (int k = 0; k < bt.K; k += 2) {
+    if (k + 1 < bt.K) load(vb, k + 1);
+    if (FftPP<N>::CALL_SYNC && k > 0) __syncthreads();
+    fft_line_pp<N, true>(va, s0, s1, stw, j);
+    store(va, k);
+    if (k + 1 < bt.K) {
+      if (k + 2 < bt.K) load(va, k + 2);
+      if (FftPP<N>::CALL_SYNC) __syncthreads();
+      fft_line_pp<N, true>(vb, s0, s1, stw, j);
+      store(vb, k + 1);
+    }
+  }
+}
+
 // a-axis inverse pass of the K radii + centre test + first-hit update
 // (get_HIIbubbles.c:335-352; centre test: is_centre).  Persistent (5 %
 // faster here than one CTA per tile): CTA i
@@ -179,6 +232,9 @@ template <int N>
 struct CbLaunch {
   using G = CbGeom<N>;
   static cudaError_t setup() {
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute(k_cols_b_cb<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)KGeom<N>::SMEM)))
+      return e;
     return cudaFuncSetAttribute(k_cols_a_test_cb<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)KGeom<N>::SMEM);
   }
@@ -189,6 +245,11 @@ struct CbLaunch {
   static int grid(int nsm) {
     const int ntiles = N * G::NBLK;
     return ntiles < nsm * KGeom<N>::PER_SM ? ntiles : nsm * KGeom<N>::PER_SM;
+  }
+  static cudaError_t cols_b(const Batch& bt, const float2* tw, cudaStream_t st) {
+    using X = KGeom<N>;
+    k_cols_b_cb<N><<<(unsigned)(N * G::NBLK), X::THREADS, X::SMEM, st>>>(bt, tw);
+    return cudaGetLastError();
   }
   static cudaError_t cols_a_test(const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw, int nsm,
                                  cudaStream_t st) {
@@ -213,6 +274,9 @@ struct CbLaunch {
 cudaError_t cb_setup(int N) { SF21_CB_DISPATCH(N, LL::setup()); }
 cudaError_t launch_rows_filter_cb(int N, const float2* spec, const Batch& bt, const float2* tw, cudaStream_t st) {
   SF21_CB_DISPATCH(N, LL::rows(spec, bt, tw, st));
+}
+cudaError_t launch_cols_b_cb(int N, const Batch& bt, const float2* tw, cudaStream_t st) {
+  SF21_CB_DISPATCH(N, LL::cols_b(bt, tw, st));
 }
 cudaError_t launch_cols_a_test_cb(int N, const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw, int nsm,
                                   cudaStream_t st) {

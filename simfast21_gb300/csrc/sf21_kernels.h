@@ -102,9 +102,11 @@ cudaError_t launch_pipe(int N, int mode, int layout, const PipeMaps& pm, const B
                         uint32_t spin_limit = 0);
 
 // Radius pipeline over column-block-major work boxes (kernels_cb.cu):
-// c-axis filter pass, a-axis pass + centre test (the b axis is launch_pipe's).
+// c-axis filter pass, in-place b-axis pass (one radius at a time: kmax = 1; else
+// the pair passes' or launch_pipe's), a-axis pass + centre test.
 cudaError_t cb_setup(int N);
 cudaError_t launch_rows_filter_cb(int N, const float2* spec, const Batch& bt, const float2* tw, cudaStream_t st);
+cudaError_t launch_cols_b_cb(int N, const Batch& bt, const float2* tw, cudaStream_t st);
 cudaError_t launch_cols_a_test_cb(int N, const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw, int nsm,
                                   cudaStream_t st);
 
