@@ -222,7 +222,7 @@ static std::string tune_cache_path() {
 
 // Revision of the pipelines' kernels: timings stored for other kernels are
 // not reused.
-constexpr int kTuneRev = 2;
+constexpr int kTuneRev = 3;
 
 static std::string tune_key(int device, long N, int K) {
   cudaDeviceProp pr;
@@ -571,12 +571,14 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
   // each candidate K (the cap, and 6 and 4 below it unless the caller fixed
   // kmax) one K-radius batch of every available pipeline is timed (or the
   // timings are read from the per-device cache); the (pipeline, K) with the
-  // least time per radius wins.
+  // least time per radius wins.  Boxes whose radii go to one launch of each pair
+  // pass (K_launch above) have no choice to make: one batch of another pipeline
+  // is no measure of it.
   auto available = [&](int p) {
     return !((p == 2 && !can_plane) || ((p == 3 || p == 4 || p == 6 || p == 7) && !can_pipe) ||
              (p == 8 && !can_fused));
   };
-  if (want == 0 && (can_plane || can_pipe || can_fused)) {
+  if (want == 0 && c->K_launch <= K && (can_plane || can_pipe || can_fused)) {
     std::vector<int> kcands = {K};
     if (cfg->kmax <= 0)
       for (int kc : {6, 4})
@@ -651,12 +653,8 @@ extern "C" int sf21_hii_create(const sf21_hii_config* cfg, sf21_hii_ctx** out) {
     }
     if (t0) cudaEventDestroy(t0);
     if (t1) cudaEventDestroy(t1);
-    if (c->K_launch <= K) {
-      c->path = best_path;
-      c->K = best_K;
-    } else {
-      c->path = 5;  // the timings are of one batch to a launch
-    }
+    c->path = best_path;
+    c->K = best_K;
     if (best_per_radius < 1e29)
       for (int p = 0; p <= NPATH; ++p) c->tune_ms[p] = best_ms[p];
   }
