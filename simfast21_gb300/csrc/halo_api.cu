@@ -661,7 +661,9 @@ extern "C" int sf21_halo_create(const sf21_halo_config* cfg, sf21_halo_ctx** out
   }
   HCREATE(dev_malloc(&c->d_tw, sizeof(float2) * N));
   HCREATE(cudaMemcpy(c->d_tw, tw.data(), sizeof(float2) * N, cudaMemcpyHostToDevice));
-  // sides with pair lines: the filter bank takes two transforms at a time
+  // sides with pair lines: the filter bank takes two transforms at a time.  Not
+  // 600, whose pair line has the roundings of the HII stage's 25 x 24 lines: the
+  // catalogues would not keep the bits of kernels_gen.cu's.
   c->pair = N == 600 ? nullptr : pair_ops(N);
   if (c->pair) {
     HCREATE(c->pair->setup());
@@ -1067,7 +1069,7 @@ static int run_filter_bank(sf21_halo_ctx* c, const std::vector<MassPlan>& plan, 
       HCTX_CUDA(c, c->pair->hf_rows(c->d_spec, hb, c->d_twp, c->nsm, st));
       HCTX_CUDA(c, c->pair->cols_b(bt, true, c->d_twp, c->nsm, st));
       HCTX_CUDA(c, c->pair->hf_cols_a(hb, c->d_twp, c->nsm, st));
-    } else {  // a 2-3-5 side without pair lines (every power of two has them)
+    } else {  // a 2-3-5 side without pair lines, or 600
       HCTX_CUDA(c, launch_gen_hf_rows_filter(c->gp, c->d_spec, hb, c->d_tw, st));
       HCTX_CUDA(c, launch_gen_hf_cols(c->gp, hb, 1, false, c->d_tw, st));
       HCTX_CUDA(c, launch_gen_hf_cols(c->gp, hb, 0, true, c->d_tw, st));

@@ -180,13 +180,13 @@ struct sf21_hii_ctx {
 };
 
 // Kernel kinds reported by sf21_hii_profile_read, in this order.
-static const char* kKindNames[] = {"prologue", "alpha", "fwd_rows", "fwd_cols_b", "fwd_cols_a",
+static const char* kKindNames[] = {"prologue", "fwd_rows", "fwd_cols_b", "fwd_cols_a",
                                    "inv_rows_filter", "inv_cols_b", "inv_cols_a_test", "dt_a",
                                    "dt_b", "dt_c_finish", "inv_plane_filter", "crit_cols_a",
                                    "adj_cols_a", "adj_cols_b_fwd", "adj_rows_acc", "adj_final",
-                                   "finish_prep", "inv_cols_ba_fused"};
-enum { KD_PRO, KD_ALPHA, KD_FROWS, KD_FCB, KD_FCA, KD_IROWS, KD_ICB, KD_ICA, KD_DTR, KD_DTB, KD_DTA, KD_PLANE,
-       KD_CRIT, KD_ADJA, KD_ADJB, KD_ADJR, KD_ADJF, KD_PREP, KD_FUSED, KD_COUNT };
+                                   "inv_cols_ba_fused"};
+enum { KD_PRO, KD_FROWS, KD_FCB, KD_FCA, KD_IROWS, KD_ICB, KD_ICA, KD_DTR, KD_DTB, KD_DTA, KD_PLANE,
+       KD_CRIT, KD_ADJA, KD_ADJB, KD_ADJR, KD_ADJF, KD_FUSED, KD_COUNT };
 
 // Records an event on st when timing is on; returns its index (or -1).
 static int mark(sf21_hii_ctx* c, cudaStream_t st) {
@@ -701,27 +701,23 @@ const PairOps* pair_ops(int N) {
 }
 }  // namespace sf21
 
-// ---- transform passes: register kernels (power-of-two sides) or shared-memory
-// kernels (other sides), same arguments ------------------------------------
+// ---- transform passes -----------------------------------------------------
+// One natural-layout box: pair lines where the side has them (every power of
+// two and 600 among others), else the shared-memory kernels.
 static cudaError_t x_fwd_rows(sf21_hii_ctx* c, const float2* in, float2* out, const float* alpha, cudaStream_t st) {
-  Batch none;
-  memset(&none, 0, sizeof(none));
   if (c->nat) return c->nat->nat_rows(in, nullptr, nullptr, out, (int)c->N, false, alpha, pair_tw(c), c->nsm, st);
-  if (c->gen && gen600_supported((int)c->N)) return launch_gen600_rows(0, in, out, none, alpha, c->d_tw, false, st);
-  return c->gen ? launch_gen_fwd_rows(c->gp, in, out, alpha, c->d_tw, st)
-                : launch_fwd_rows((int)c->N, in, out, alpha, c->d_tw, st);
+  return launch_gen_fwd_rows(c->gp, in, out, alpha, c->d_tw, st);
 }
 static cudaError_t x_inv_rows_plain(sf21_hii_ctx* c, float2* box, cudaStream_t st) {
-  Batch none;
-  memset(&none, 0, sizeof(none));
   if (c->nat) return c->nat->nat_rows(box, nullptr, nullptr, box, (int)c->N, true, nullptr, pair_tw(c), c->nsm, st);
-  if (c->gen && gen600_supported((int)c->N)) return launch_gen600_rows(1, box, box, none, nullptr, c->d_tw, false, st);
-  return c->gen ? launch_gen_inv_rows_plain(c->gp, box, c->d_tw, st) : launch_inv_rows_plain((int)c->N, box, c->d_tw, st);
+  return launch_gen_inv_rows_plain(c->gp, box, c->d_tw, st);
 }
+// A batch's boxes, one radius at a time: register kernels (powers of two, 600)
+// or shared-memory kernels.
 // cb: the radius pipeline's batch in the column-block-major layout (N = 600 only)
 static cudaError_t x_inv_rows_filter(sf21_hii_ctx* c, const float2* spec, const Batch& bt, cudaStream_t st,
                                      bool cb = false) {
-  if (c->gen && gen600_supported((int)c->N)) return launch_gen600_rows(2, spec, nullptr, bt, nullptr, c->d_tw, cb, st);
+  if (c->gen && gen600_supported((int)c->N)) return launch_gen600_rows(spec, bt, c->d_tw, cb, st);
   return c->gen ? launch_gen_inv_rows_filter(c->gp, spec, bt, c->d_tw, st)
                 : launch_inv_rows_filter((int)c->N, spec, bt, c->d_tw, st);
 }
@@ -731,7 +727,7 @@ static cudaError_t x_cols(sf21_hii_ctx* c, float2* box, const Batch& bt, int nbo
   if (box && c->nat) return c->nat->nat_cols(box, axis, inverse, (int)c->N, pair_tw(c), st);
   if (!c->gen) return launch_cols((int)c->N, box, bt, nbox, axis, inverse, c->d_tw, st);
   if (!box && nbox != bt.K) return cudaErrorInvalidValue;
-  if (gen600_supported((int)c->N)) return launch_gen600_cols(box, bt, axis, inverse, cb, c->d_tw, st);
+  if (gen600_supported((int)c->N)) return launch_gen600_cols(bt, axis, inverse, cb, c->d_tw, st);
   return launch_gen_cols(c->gp, box, bt, axis, inverse, c->d_tw, st);
 }
 static cudaError_t x_cols_a_test(sf21_hii_ctx* c, const Batch& bt, cudaStream_t st) {

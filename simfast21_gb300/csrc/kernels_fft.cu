@@ -11,9 +11,9 @@
 // centre test.
 //
 // Passes:
-//   c-axis (contiguous rows): coalesced row loads straight into registers;
-//     the inverse variant reads the spectrum once and emits K filtered,
-//     c-transformed work boxes (one per radius of the batch);
+//   c-axis (contiguous rows), inverse: coalesced row loads straight into
+//     registers; reads the spectrum once and emits K filtered, c-transformed
+//     work boxes (one per radius of the batch);
 //   b- and a-axis (strided): a tile of N rows x CW contiguous columns, each
 //     column a line of the FFT;
 //   the a-axis inverse pass ends in the centre test (:335-352, :437-438) and
@@ -25,36 +25,6 @@
 #include "sf21_kernels.h"
 
 namespace sf21 {
-
-// ---------------------------------------------------------------------------
-// Forward c-axis pass of the packed prologue output: z = (rec0, ion * alpha).
-template <int N>
-__global__ void __launch_bounds__(RowGeom<N>::THREADS)
-k_fwd_rows(const float2* __restrict__ in, float2* __restrict__ out,
-           const float* __restrict__ alpha_ptr, const float2* __restrict__ gtw) {
-  using G = RowGeom<N>;
-  using L = LineGeom<N>;
-  __shared__ float2 stw[N];
-  __shared__ float2 sbuf[G::ROWS * L::LS];
-  load_twiddles<N>(stw, gtw);
-  const int row_in_cta = threadIdx.x / G::T;
-  const int j = threadIdx.x % G::T;
-  const long row = (long)blockIdx.x * G::ROWS + row_in_cta;
-  const float alpha = alpha_ptr ? fabsf(*alpha_ptr) : 1.0f;
-  float2 v[8];
-  const float2* src = in + row * N;
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    float2 x = src[j + r * (N / 8)];
-    x.y *= alpha;
-    v[r] = x;
-  }
-  __syncthreads();
-  fft_line<N, false>(v, sbuf + row_in_cta * L::LS, stw, j);
-  float2* dst = out + row * N;
-#pragma unroll
-  for (int r = 0; r < 8; ++r) dst[j + r * (N / 8)] = v[r];
-}
 
 // ---------------------------------------------------------------------------
 // Inverse c-axis pass with the k-space top-hat filter of K radii
@@ -98,28 +68,6 @@ k_inv_rows_filter(const float2* __restrict__ spec, Batch bt, const float2* __res
 #pragma unroll
     for (int r = 0; r < 8; ++r) dst[j + r * (N / 8)] = v[r];
   }
-}
-
-// Unfiltered inverse c-axis pass in place (plain form and tests).
-template <int N>
-__global__ void __launch_bounds__(RowGeom<N>::THREADS)
-k_inv_rows_plain(float2* __restrict__ box, const float2* __restrict__ gtw) {
-  using G = RowGeom<N>;
-  using L = LineGeom<N>;
-  __shared__ float2 stw[N];
-  __shared__ float2 sbuf[G::ROWS * L::LS];
-  load_twiddles<N>(stw, gtw);
-  const int row_in_cta = threadIdx.x / G::T;
-  const int j = threadIdx.x % G::T;
-  const long row = (long)blockIdx.x * G::ROWS + row_in_cta;
-  float2 v[8];
-  float2* p = box + row * N;
-#pragma unroll
-  for (int r = 0; r < 8; ++r) v[r] = p[j + r * (N / 8)];
-  __syncthreads();
-  fft_line<N, true>(v, sbuf + row_in_cta * L::LS, stw, j);
-#pragma unroll
-  for (int r = 0; r < 8; ++r) p[j + r * (N / 8)] = v[r];
 }
 
 // ---------------------------------------------------------------------------
@@ -209,14 +157,6 @@ struct Launch {
   static constexpr size_t smem_cols() { return (N + ColGeom<N>::CW * LineGeom<N>::LS) * sizeof(float2); }
   static unsigned grid_rows() { return (unsigned)((long)N * N / RowGeom<N>::ROWS); }
   static unsigned grid_cols() { return (unsigned)((long)N * (N / ColGeom<N>::CW)); }
-  static cudaError_t fwd_rows(const float2* in, float2* out, const float* alpha, const float2* tw, cudaStream_t st) {
-    k_fwd_rows<N><<<grid_rows(), RowGeom<N>::THREADS, 0, st>>>(in, out, alpha, tw);
-    return cudaGetLastError();
-  }
-  static cudaError_t inv_rows_plain(float2* box, const float2* tw, cudaStream_t st) {
-    k_inv_rows_plain<N><<<grid_rows(), RowGeom<N>::THREADS, 0, st>>>(box, tw);
-    return cudaGetLastError();
-  }
   static cudaError_t inv_rows_filter(const float2* spec, const Batch& bt, const float2* tw, cudaStream_t st) {
     k_inv_rows_filter<N><<<grid_rows(), RowGeom<N>::THREADS, 0, st>>>(spec, bt, tw);
     return cudaGetLastError();
@@ -257,13 +197,6 @@ struct Launch {
   }
 
 cudaError_t fft_setup(int N) { SF21_DISPATCH_N(N, LL::setup()); }
-cudaError_t launch_fwd_rows(int N, const float2* in, float2* out, const float* alpha, const float2* tw,
-                            cudaStream_t st) {
-  SF21_DISPATCH_N(N, LL::fwd_rows(in, out, alpha, tw, st));
-}
-cudaError_t launch_inv_rows_plain(int N, float2* box, const float2* tw, cudaStream_t st) {
-  SF21_DISPATCH_N(N, LL::inv_rows_plain(box, tw, st));
-}
 cudaError_t launch_inv_rows_filter(int N, const float2* spec, const Batch& bt, const float2* tw, cudaStream_t st) {
   SF21_DISPATCH_N(N, LL::inv_rows_filter(spec, bt, tw, st));
 }

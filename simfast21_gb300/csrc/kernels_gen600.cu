@@ -115,7 +115,7 @@ __device__ __forceinline__ void dft24(float2 (&u)[24], const float2* tw) {
   for (int q1 = 0; q1 < 8; ++q1) dft3<INV>(u[3 * q1], u[3 * q1 + 1], u[3 * q1 + 2]);
 }
 
-// EPI 0: transform in place (box0, or the batch's K boxes); EPI 1: inverse,
+// EPI 0: transform of the batch's K boxes in place; EPI 1: inverse,
 // centre test and first-hit update of the batch's K boxes (the transform is
 // not stored).  AXIS 1: lines along b; AXIS 0: along a.  LAYOUT 0: natural
 // boxes (a N^2 + b N + c: a-axis rows N^2 apart, 600 rows of a tile on 600
@@ -123,7 +123,7 @@ __device__ __forceinline__ void dft24(float2 (&u)[24], const float2* tw) {
 // ((c / 8) N + a) N + b) 8 + c mod 8, where a b-axis tile is one contiguous
 // run and an a-axis tile stays inside one 23 MB slab.
 template <bool INV, int EPI, int AXIS, int LAYOUT>
-__global__ void __launch_bounds__(g600::THREADS, 3) k_gen600_cols(float2* box0, Batch bt, uint8_t* rc,
+__global__ void __launch_bounds__(g600::THREADS, 3) k_gen600_cols(Batch bt, uint8_t* rc,
                                                                const float* __restrict__ alpha_ptr,
                                                                const float2* __restrict__ gtw) {
   using namespace g600;
@@ -139,7 +139,6 @@ __global__ void __launch_bounds__(g600::THREADS, 3) k_gen600_cols(float2* box0, 
   const long cbk = c0 / CW;
   const long base = LAYOUT == 1 ? (AXIS == 1 ? (cbk * N + outer) * N * CW : (cbk * N * N + outer) * CW) + col
                                 : (AXIS == 1 ? (long)outer * N * N : (long)outer * N) + c0 + col;
-  const int nbox = box0 ? 1 : bt.K;
   float alpha = 1.0f;
   if (EPI == 1) alpha = *alpha_ptr;
   // EPI 1: first hits of this thread's 24 outputs (rows 25 k1 + r), over the
@@ -147,8 +146,8 @@ __global__ void __launch_bounds__(g600::THREADS, 3) k_gen600_cols(float2* box0, 
   // one, its radius index is byte e of hbyte (24 bytes in 6 words)
   uint32_t hmask = 0u;
   uint32_t hbyte[6] = {0u, 0u, 0u, 0u, 0u, 0u};
-  for (int k = 0; k < nbox; ++k) {
-    float2* box = box0 ? box0 : bt.r[k].work;
+  for (int k = 0; k < bt.K; ++k) {
+    float2* box = bt.r[k].work;
     __syncthreads();  // twiddles (k = 0); the previous box's step 2 is done with the exchange
     if (r < N1) {
       float2 y[25];
@@ -213,12 +212,10 @@ bool gen600_supported(int N) { return N == g600::N; }
 // (for fixed k1, 25 consecutive values: coalesced stores).  The exchange is
 // the warp's own shared-memory block (stride 25 float2 per k2: the reads by
 // k2 meet distinct banks), so a row needs no CTA barrier.
-// MODE 0: forward, imaginary part times |alpha| (the packed prologue box);
-// MODE 1: inverse in place; MODE 2: inverse of the spectrum row times the
-// top-hat filter of each of the batch's K radii, into the K work boxes.
-// In MODE 2 the window takes one value per |k_c| (c and N - c share it): all
-// 32 lanes evaluate the row's N/2 + 1 values once per radius into a
-// shared-memory row, instead of 24 lanes evaluating 25 each.  Same
+// Inverse of the spectrum row times the top-hat filter of each of the batch's K
+// radii, into the K work boxes.  The window takes one value per |k_c| (c and
+// N - c share it): all 32 lanes evaluate the row's N/2 + 1 values once per
+// radius into a shared-memory row, instead of 24 lanes evaluating 25 each.  Same
 // expression, same bits.
 namespace g600 {
 constexpr int RW = 8;                      // rows (warps) per CTA
@@ -230,12 +227,11 @@ constexpr int NW = (N / 2 + 32) / 32;      // window values per lane
 constexpr size_t RSMEM = (size_t)(N + RW * (XS + N + WS)) * sizeof(float2);
 }  // namespace g600
 
-template <int MODE, int LAYOUT>
-__global__ void __launch_bounds__(g600::RTHREADS, 2) k_gen600_rows(const float2* in, float2* out, Batch bt,
-                                                                  const float* __restrict__ alpha_ptr,
+template <int LAYOUT>
+__global__ void __launch_bounds__(g600::RTHREADS, 2) k_gen600_rows(const float2* __restrict__ spec, Batch bt,
                                                                   const float2* __restrict__ gtw) {
   using namespace g600;
-  constexpr bool INV = MODE != 0;
+  constexpr bool INV = true;
   extern __shared__ float2 gsm[];
   float2* tw = gsm;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -245,12 +241,9 @@ __global__ void __launch_bounds__(g600::RTHREADS, 2) k_gen600_rows(const float2*
   for (int t = threadIdx.x; t < N; t += RTHREADS) tw[t] = gtw[t];
   __syncthreads();
   const long row = (long)blockIdx.x * RW + w;
-  const float2* src = in + row * N;
-  const int nout = MODE == 2 ? bt.K : 1;
-  float alpha = 1.0f;
-  if (MODE == 0 && alpha_ptr) alpha = fabsf(*alpha_ptr);
-  float kmag[NW];  // MODE 2: |k| at |k_c| = lane + 32 i (<= N/2) of this row
-  if (MODE == 2) {
+  const float2* src = spec + row * N;
+  float kmag[NW];  // |k| at |k_c| = lane + 32 i (<= N/2) of this row
+  {
     const int a = (int)(row / N), b = (int)(row % N);
     const int ka = kfreq(a, N), kb = kfreq(b, N);
     const int kab = ka * ka + kb * kb;
@@ -261,8 +254,8 @@ __global__ void __launch_bounds__(g600::RTHREADS, 2) k_gen600_rows(const float2*
     }
     for (int c = lane; c < N; c += 32) zrow[c] = src[c];
   }
-  for (int k = 0; k < nout; ++k) {
-    if (MODE == 2) {  // the window of radius k at every |k_c|
+  for (int k = 0; k < bt.K; ++k) {
+    {  // the window of radius k at every |k_c|
       const float dkR = bt.r[k].dkR;
 #pragma unroll
       for (int i = 0; i < NW; ++i) {
@@ -276,13 +269,7 @@ __global__ void __launch_bounds__(g600::RTHREADS, 2) k_gen600_rows(const float2*
 #pragma unroll
       for (int n2 = 0; n2 < 25; ++n2) {
         const int c = lane + N1 * n2;
-        if (MODE == 2) {
-          y[n2] = filter_mul(zrow[c], wrow[c <= N / 2 ? c : N - c]);
-        } else {
-          float2 v = src[c];
-          if (MODE == 0) v.y *= alpha;
-          y[n2] = v;
-        }
+        y[n2] = filter_mul(zrow[c], wrow[c <= N / 2 ? c : N - c]);
       }
       dft25<INV>(y, tw);
 #pragma unroll
@@ -302,13 +289,13 @@ __global__ void __launch_bounds__(g600::RTHREADS, 2) k_gen600_rows(const float2*
       for (int n1 = 0; n1 < 24; ++n1) u[n1] = ex[lane * N2 + n1];
       dft24<INV>(u, tw);
       if (LAYOUT == 0) {
-        float2* dst = (MODE == 2 ? bt.r[k].work : out) + row * N + lane;
+        float2* dst = bt.r[k].work + row * N + lane;
 #pragma unroll
         for (int q1 = 0; q1 < 8; ++q1)
 #pragma unroll
           for (int q2 = 0; q2 < 3; ++q2) dst[25 * (q1 + 8 * q2)] = u[3 * q1 + q2];
       } else {  // column-block major: (a, b, c) at ((c / 8) N^2 + a N + b) 8 + c mod 8, row = a N + b
-        float2* dst = (MODE == 2 ? bt.r[k].work : out) + row * CW;
+        float2* dst = bt.r[k].work + row * CW;
 #pragma unroll
         for (int q1 = 0; q1 < 8; ++q1)
 #pragma unroll
@@ -333,51 +320,32 @@ cudaError_t gen600_setup() {
   if ((e = g600_attr<true, 0, 0, 0>()) || (e = g600_attr<true, 0, 1, 0>()) || (e = g600_attr<false, 0, 0, 0>()) ||
       (e = g600_attr<false, 0, 1, 0>()) || (e = g600_attr<true, 0, 1, 1>()) || (e = g600_attr<true, 1, 0, 1>()))
     return e;
-  for (auto f : {k_gen600_rows<0, 0>, k_gen600_rows<1, 0>, k_gen600_rows<2, 0>, k_gen600_rows<2, 1>})
+  for (auto f : {k_gen600_rows<0>, k_gen600_rows<1>})
     if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g600::RSMEM))) return e;
   return cudaSuccess;
 }
 
-cudaError_t launch_gen600_rows(int mode, const float2* in, float2* out, const Batch& bt, const float* alpha,
-                               const float2* tw, bool cb, cudaStream_t st) {
+cudaError_t launch_gen600_rows(const float2* spec, const Batch& bt, const float2* tw, bool cb, cudaStream_t st) {
   const unsigned grid = (unsigned)((long)g600::N * g600::N / g600::RW);
-  const int T = g600::RTHREADS;
-  const size_t S = g600::RSMEM;
-  if (mode == 0)
-    k_gen600_rows<0, 0><<<grid, T, S, st>>>(in, out, bt, alpha, tw);
-  else if (mode == 1)
-    k_gen600_rows<1, 0><<<grid, T, S, st>>>(in, out, bt, nullptr, tw);
-  else if (cb)
-    k_gen600_rows<2, 1><<<grid, T, S, st>>>(in, nullptr, bt, nullptr, tw);
-  else
-    k_gen600_rows<2, 0><<<grid, T, S, st>>>(in, nullptr, bt, nullptr, tw);
+  auto f = cb ? k_gen600_rows<1> : k_gen600_rows<0>;
+  f<<<grid, g600::RTHREADS, g600::RSMEM, st>>>(spec, bt, tw);
   return cudaGetLastError();
 }
 
-cudaError_t launch_gen600_cols(float2* box0, const Batch& bt, int axis, bool inverse, bool cb, const float2* tw,
-                               cudaStream_t st) {
+cudaError_t launch_gen600_cols(const Batch& bt, int axis, bool inverse, bool cb, const float2* tw, cudaStream_t st) {
   const unsigned grid = (unsigned)(g600::N * (g600::N / g600::CW));
-  const int T = g600::THREADS;
-  const size_t S = g600::SMEM;
-  if (cb) {  // the radius batch's b-axis inverse
-    if (box0 || axis != 1 || !inverse) return cudaErrorInvalidValue;
-    k_gen600_cols<true, 0, 1, 1><<<grid, T, S, st>>>(nullptr, bt, nullptr, nullptr, tw);
-  } else if (inverse && axis == 1) {
-    k_gen600_cols<true, 0, 1, 0><<<grid, T, S, st>>>(box0, bt, nullptr, nullptr, tw);
-  } else if (inverse) {
-    k_gen600_cols<true, 0, 0, 0><<<grid, T, S, st>>>(box0, bt, nullptr, nullptr, tw);
-  } else if (axis == 1) {
-    k_gen600_cols<false, 0, 1, 0><<<grid, T, S, st>>>(box0, bt, nullptr, nullptr, tw);
-  } else {
-    k_gen600_cols<false, 0, 0, 0><<<grid, T, S, st>>>(box0, bt, nullptr, nullptr, tw);
-  }
+  if (cb && (axis != 1 || !inverse)) return cudaErrorInvalidValue;  // the radius batch's b-axis inverse
+  auto f = cb ? k_gen600_cols<true, 0, 1, 1>
+           : inverse ? (axis == 1 ? k_gen600_cols<true, 0, 1, 0> : k_gen600_cols<true, 0, 0, 0>)
+                     : (axis == 1 ? k_gen600_cols<false, 0, 1, 0> : k_gen600_cols<false, 0, 0, 0>);
+  f<<<grid, g600::THREADS, g600::SMEM, st>>>(bt, nullptr, nullptr, tw);
   return cudaGetLastError();
 }
 
 cudaError_t launch_gen600_cols_a_test(const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw,
                                       cudaStream_t st) {
   const unsigned grid = (unsigned)(g600::N * (g600::N / g600::CW));
-  k_gen600_cols<true, 1, 0, 1><<<grid, g600::THREADS, g600::SMEM, st>>>(nullptr, bt, rc, alpha, tw);
+  k_gen600_cols<true, 1, 0, 1><<<grid, g600::THREADS, g600::SMEM, st>>>(bt, rc, alpha, tw);
   return cudaGetLastError();
 }
 

@@ -38,11 +38,6 @@ struct PrologueArgs {
 };
 
 cudaError_t fft_setup(int N);
-// c-axis forward of the packed box (imag part times *alpha), in -> out
-cudaError_t launch_fwd_rows(int N, const float2* in, float2* out, const float* alpha, const float2* tw,
-                            cudaStream_t st);
-// c-axis inverse in place, no filter
-cudaError_t launch_inv_rows_plain(int N, float2* box, const float2* tw, cudaStream_t st);
 // c-axis inverse with the top-hat filter of the batch's K radii: spec -> bt.r[k].work
 cudaError_t launch_inv_rows_filter(int N, const float2* spec, const Batch& bt, const float2* tw, cudaStream_t st);
 // strided axis (1 = b, 0 = a) in place, of `box` (nbox = 1) or of the batch's work boxes
@@ -327,21 +322,18 @@ struct GenPlan {
   int nst;        // stages
   int radix[16];  // radix of each stage (8, 4, 2, 3 or 5)
 };
-// Register-resident passes for N = 600 (kernels_gen600.cu): 600 = 24 x 25,
-// one shared-memory exchange per line; twiddles: the plain table of the
-// shared-memory family.  cb: the radius batch's work boxes in the
-// column-block-major layout ((c / 8) N + a) N + b) 8 + c mod 8 (rows mode 2
-// writes it, the b-axis inverse and the a-axis test pass read it); otherwise
-// natural boxes.  launch_gen600_cols_a_test reads the batch in that layout.
+// Register-resident passes of single radii for N = 600 (kernels_gen600.cu): 600
+// = 24 x 25, one shared-memory exchange per line; twiddles: the plain table of
+// the shared-memory family.  cb: the batch's work boxes in the column-block-
+// major layout ((c / 8) N + a) N + b) 8 + c mod 8 (the rows write it, the b-axis
+// inverse and the a-axis test pass read it); otherwise natural boxes.
 bool gen600_supported(int N);
 cudaError_t gen600_setup();
-cudaError_t launch_gen600_cols(float2* box0, const Batch& bt, int axis, bool inverse, bool cb, const float2* tw,
-                               cudaStream_t st);
-// rows: mode 0 forward (in -> out, imaginary part times |*alpha|), 1 inverse
-// in place (in == out), 2 inverse of the spectrum times the batch's filters
-// (in = spectrum -> bt.r[k].work)
-cudaError_t launch_gen600_rows(int mode, const float2* in, float2* out, const Batch& bt, const float* alpha,
-                               const float2* tw, bool cb, cudaStream_t st);
+// b (1) or a (0) axis of the batch's boxes, in place
+cudaError_t launch_gen600_cols(const Batch& bt, int axis, bool inverse, bool cb, const float2* tw, cudaStream_t st);
+// c axis, inverse, of the spectrum times the batch's filters -> bt.r[k].work
+cudaError_t launch_gen600_rows(const float2* spec, const Batch& bt, const float2* tw, bool cb, cudaStream_t st);
+// a axis of the batch in the cb layout + centre test + first-hit update
 cudaError_t launch_gen600_cols_a_test(const Batch& bt, uint8_t* rc, const float* alpha, const float2* tw,
                                       cudaStream_t st);
 bool gen_supported(int N);
