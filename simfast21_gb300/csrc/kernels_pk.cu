@@ -87,9 +87,9 @@ k_pk_bin(int N, const float2* __restrict__ spec, int nk, float* __restrict__ par
 // the integer routines of softdouble.h, as bits.  A sum with an infinity is
 // infinite, one with a NaN is NaN (those routines take finite operands only).
 // threadIdx.x = bin of the CTA's PKR_BINS, the threadIdx.y rows share the CTAs:
-// a sum of doubles in integers is a chain of 60 instructions, so a bin has 128
-// of them side by side.
-constexpr int PKR_BINS = 8, PKR_ROWS = 128;
+// a sum of doubles in integers is a chain of 60 instructions, so a bin has 512
+// of them side by side (512^3, 8192 partial sums a bin: 24 us; 60 with 128).
+constexpr int PKR_BINS = 2, PKR_ROWS = 512;
 __global__ void __launch_bounds__(PKR_BINS * PKR_ROWS)
 k_pk_reduce(int ncta, int nk, const float* __restrict__ partials, sd_t* __restrict__ sums) {
   __shared__ sd_t sm[PKR_ROWS][PKR_BINS + 1];
