@@ -22,11 +22,13 @@
 #include <unistd.h>
 #include <stdlib.h>
 
-#include <atomic>
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <future>
 #include <string>
 #include <system_error>
+#include <thread>
 #include <vector>
 
 #include "../../include/sf21_hii.h"
@@ -1643,15 +1645,38 @@ auto beside(F f) -> std::future<decltype(f())> {
     return std::async(std::launch::deferred, f);
   }
 }
-// Maps the pages of [p, p + n) writable, contents as they are; nothing where the kernel cannot
-void map_pages(void* p, size_t n) {
+// Maps the pages of [p, p + n) writable on a thread, contents as they are, from p on; nothing where the
+// kernel cannot
+class PageMapper {
+ public:
+  static constexpr size_t kStep = 8 << 20;
+  PageMapper(void* p, size_t n) {
+    done_ = beside([this, p, n] {
 #ifndef MADV_POPULATE_WRITE
 #define MADV_POPULATE_WRITE 23
 #endif
-  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), a = ((uintptr_t)p + page - 1) / page * page,
-                  e = ((uintptr_t)p + n) / page * page;
-  if (a < e) madvise((void*)a, e - a, MADV_POPULATE_WRITE);
-}
+      const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), p0 = (uintptr_t)p, a = (p0 + page - 1) / page * page,
+                      e = (p0 + n) / page * page;
+      for (uintptr_t q = a; q < e; q += kStep) {
+        if (madvise((void*)q, std::min<size_t>(kStep, e - q), MADV_POPULATE_WRITE)) break;
+        mapped_.store(std::min(q + kStep, e) - p0, std::memory_order_release);
+      }
+    });
+  }
+  // the mapped bytes, once there are `bytes` of them or no more to come (then n)
+  size_t wait(size_t bytes, size_t n) {
+    for (;;) {
+      const bool done = !done_.valid() || done_.wait_for(std::chrono::seconds(0)) != std::future_status::timeout;
+      const size_t m = done ? n : mapped_.load(std::memory_order_acquire);
+      if (m >= bytes) return m;
+      std::this_thread::yield();
+    }
+  }
+
+ private:
+  std::atomic<size_t> mapped_{0};
+  std::future<void> done_;
+};
 }  // namespace
 
 extern "C" int sf21_t21_run_z(sf21_hii_ctx* c, const sf21_t21_cosmo* cosmo, double z, const float* delta,
@@ -1680,7 +1705,7 @@ extern "C" int sf21_t21_run_z(sf21_hii_ctx* c, const sf21_t21_cosmo* cosmo, doub
   const T21Cosmo cs{cosmo->omega_m, cosmo->omega_b, cosmo->omega_lambda, c->hubble};
   // (and the output's pages: a caller's new array takes 2.6 ms of page faults at 256^3)
   auto growth = beside([cs, z] { return cs.growth(z); });
-  const auto pages = beside([tb, bf] { map_pages(tb, bf); });
+  PageMapper pages(tb, bf);
   CTX_CUDA(c, cudaMemcpyAsync(c->d_delta, delta, bf, cudaMemcpyHostToDevice, st));
   CTX_CUDA(c, cudaMemcpyAsync(c->d_xhii, xhii, bf, cudaMemcpyHostToDevice, st));
   if (spin) {
@@ -1712,7 +1737,14 @@ extern "C" int sf21_t21_run_z(sf21_hii_ctx* c, const sf21_t21_cosmo* cosmo, doub
   CTX_CUDA(c, launch_t21_finish(n3, c->d_pk, c->d_delta, c->d_xhii, spin ? d_xc : nullptr, spin ? d_xa : nullptr,
                                 spin ? d_tk : nullptr, ta, d_tb, c->d_t21_part, st));
   std::vector<float> part(2 * (size_t)nb);
-  CTX_CUDA(c, cudaMemcpyAsync(tb, d_tb, bf, cudaMemcpyDeviceToHost, st));
+  // the box behind its pages: a copy that meets unmapped ones takes up to ten times as long, and mapping them
+  // beside it or by eight threads at once holds both up (512^3, new output: pinned boxes 22.6 ms without a
+  // mapper, 25 with one that the copy does not wait for, 16.7 so; unpinned 28.3, 23.8, 16.6)
+  for (size_t o = 0; o < bf;) {
+    const size_t upto = pages.wait(std::min(bf, o + PageMapper::kStep), bf);
+    CTX_CUDA(c, cudaMemcpyAsync((char*)tb + o, (char*)d_tb + o, upto - o, cudaMemcpyDeviceToHost, st));
+    o = upto;
+  }
   CTX_CUDA(c, cudaMemcpyAsync(part.data(), c->d_t21_part, sizeof(float) * part.size(), cudaMemcpyDeviceToHost, st));
   CTX_CUDA(c, cudaStreamSynchronize(st));
   double s_tb = 0., s_ts = 0.;
