@@ -275,7 +275,7 @@ PIPELINES = {
     2: ("plane", "cluster plane pass + kx pass"),
     3: ("tma_ky", "three axis passes, ky pass TMA-pipelined"),
     4: ("tma_ky_kx", "three axis passes, ky and kx passes TMA-pipelined"),
-    5: ("cb_three_pass", "column-block-major work boxes, three axis passes"),
+    5: ("pairs_three_pass", "three axis passes over pairs of radii"),
     6: ("cb_tma_ky", "column-block-major work boxes, ky pass TMA-pipelined"),
     7: ("cb_tma_ky_kx", "column-block-major work boxes, ky and kx passes TMA-pipelined"),
     8: ("cb_fused_l2", "column-block-major work boxes, c-axis pass + one persistent ky/kx launch through L2"),
@@ -592,10 +592,10 @@ def run_ours(args, w, rank, world):
     }.get(dom, None)
     achieved = alg / (per_launch_ms / 1e3) / 1e9 if alg else None
     # DRAM traffic per launch (dram__bytes_read + dram__bytes_write) from the
-    # ncu capture of the same kernels at 512^3, K = 8, per voxel*radius
-    # (profiles/radius_kernels_cb_single512.md), scaled to this launch's radii
-    traffic_b = {"inv_cols_b": 15.94, "inv_cols_a_test": 8.00, "inv_rows_filter": 8.94}.get(dom)
-    traffic = traffic_b * n3 * K_avg if (traffic_b and path >= 5) else None
+    # ncu capture of the same kernels at 512^3 per voxel*radius
+    # (profiles/kernels_256.md), for this launch's radii
+    traffic_b = {"inv_cols_b": 15.77, "inv_cols_a_test": 8.00, "inv_rows_filter": 7.80 + 8.02 / K_avg}.get(dom)
+    traffic = traffic_b * n3 * K_avg if (traffic_b and path == 5) else None
     # whole radius pipeline against the 16 B per voxel*radius algorithmic traffic
     pipe_ms = sum(kinds.get(k, (0, 0))[0] for k in ("inv_rows_filter", "inv_cols_b", "inv_cols_a_test",
                                                      "inv_plane_filter", "inv_cols_ba_fused"))
@@ -722,7 +722,7 @@ def run_ours(args, w, rank, world):
             "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": hbm,
                          "unit": "GB/s", "frac": (achieved / hbm) if achieved else None,
                          "peak_source": peak_kind, "traffic": traffic,
-                         "traffic_source": "ncu capture, 512^3 K=8, scaled per launch" if traffic else None,
+                         "traffic_source": "ncu capture, 512^3, per voxel and radius" if traffic else None,
                          "pipeline_16B_per_voxel_radius_gbs": pipe_gbs,
                          "pipeline_frac": (pipe_gbs / hbm) if pipe_gbs else None,
                          "step_16B_per_voxel_radius_frac": value / world * 16.0 / (hbm * 1e9)},

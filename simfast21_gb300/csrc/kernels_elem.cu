@@ -182,8 +182,7 @@ cudaError_t launch_fill0(long n3, uint64_t zeta, const float* src, const float* 
 // A call with host boxes and four sets, neutral fractions included: 16^3 0.52
 // ms with the sums as loops on host threads, 0.99 when one block added the
 // chunks' sums in FP64, each thread all that come before its own, 0.26 so;
-// 64^3 0.81, 1.19, 0.53; 256^3 20.4, 9.0, 8.0.  One pass over the box each,
-// bound by its reads.
+// 64^3 0.81, 1.19, 0.53; 256^3 20.4, 9.0, 8.0.
 constexpr int NEU_THREADS = 256, NEU_PER = NEUTRAL_CHUNK / NEU_THREADS;  // consecutive terms per thread
 static_assert(NEU_PER == 16, "four float4 per thread");
 constexpr uint64_t NEU_BAD = ~0ull;  // sum of a chunk with a term outside [0, 1]

@@ -7,8 +7,8 @@
 //     index(a, b, c) = ((c / 8) N + a) N + b) 8 + c mod 8,
 // one slab of 8 N^2 values per column block: a b-axis tile (fixed a, one
 // block) is one contiguous run, an a-axis tile (fixed b) reads 128-byte runs
-// inside one slab.  A batch with an odd number of radii carries its last
-// radius twice (the centre test of a radius is idempotent).
+// inside one slab.  A batch with an odd number of radii (the last one of a set)
+// carries its last radius twice (the centre test of a radius is idempotent).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -853,9 +853,10 @@ k_pair_nat_cols(float2* box, int nblk, const float2* __restrict__ plain) {
 // tiles want few exchanges as long as two or more CTAs fit an SM (two groups at
 // 256: kx 0.40, three 0.47; at 512 0.53 and 0.53, but ky 0.86 and 0.74), rows
 // want many threads (512: three groups 0.56, two 0.80), and threads per line
-// that fill whole warps (400: 40 threads 0.58, 50 threads 0.76).  Sides whose
-// radices have no such cut (720, 1000, 1080, 1152, 1200, 1280) stay with the
-// shared-memory lines of kernels_gen.cu; 600 follows kernels_gen600.cu.
+// that fill whole warps (400: 40 threads 0.58, 50 threads 0.76).  600 follows
+// kernels_gen600.cu.  720, 1000, 1080, 1152, 1200 and 1280 have no line here yet,
+// though their radices have such cuts (1200 = 25 x 6 x 8): they stay with the
+// shared-memory lines of kernels_gen.cu.
 template <int N> struct PairSide;
 #define SF21_SIDE(N_, CT, CREGS, RT, RW_, RREGS, COLS, ROWS)          \
   template <> struct PairSide<N_> {                                  \

@@ -181,10 +181,11 @@ class FilterBank:
 
     def path(self):
         """(pipeline in use: 1 = three axis passes, 2 = plane clusters,
-        3 = TMA-pipelined ky pass, 4 = TMA-pipelined ky and kx passes, and over
-        column-block-major work boxes 5 = three axis passes, 6 = TMA ky pass,
-        7 = TMA ky and kx passes, 8 = c-axis pass + one persistent ky/kx
-        launch through L2; {pipeline: tuned ms of one batch})."""
+        3 = TMA-pipelined ky pass, 4 = TMA-pipelined ky and kx passes, 5 = three
+        axis passes over pairs of radii, and over column-block-major work boxes
+        6 = TMA ky pass, 7 = TMA ky and kx passes, 8 = c-axis pass + one
+        persistent ky/kx launch through L2; {pipeline: tuned ms of one batch,
+        0 where it was not timed})."""
         ms = (ctypes.c_double * NPATH)()
         p = self._lib.sf21_hii_path(self._h, ms, NPATH)
         return p, {i + 1: ms[i] for i in range(NPATH)}
