@@ -446,18 +446,21 @@ static unsigned grid_for(long n) {
 // tile's cells are in shared memory, so a chain never leaves the CTA, and its
 // order is made there: every waiting contribution puts its serial number
 // 8 i + corner into its cell's slot by atomicMin, the smallest one is added,
-// and the others go again, until none waits.  Within a run the halos keep
-// their order (the sort is stable); when a tile has more of them than the CTA
-// has threads, it takes those below a serial number that leaves no run behind.
+// and the others go again, until none waits (in a crowd: tile_crowd).  Within a
+// run the halos keep their order (the sort is stable); when a tile has more of
+// them than the CTA has threads, it takes those below a serial number that
+// leaves no run behind.
 // The block average follows from shared memory, for the blocks that have a
 // contribution, in pairs of floats; no grid is stored.
 //
-// 1200^3 cells, 2 10^7 halos: 14.6 -> 7.3 ms, of which the two sorts take 1.0.  It is bound by its instructions (the pairs of floats below)
-// and by the barriers of the rounds: 64 to 256 threads, tiles of 1024 to 8192
+// 1200^3 cells, 2 10^7 halos: 14.6 -> 7.4 ms, of which the two sorts take 1.0.
+// It is bound by its instructions (the pairs of floats below) and by the
+// barriers of the rounds: 64 to 256 threads, tiles of 1024 to 8192
 // cells and 24 to 64 KB were within 10 %, a tile of 4096 cells and 96 threads
 // (47 halos in it on average, 60 with those of its neighbours) the fastest.
 constexpr int TILE_THREADS = 96;
 constexpr int TILE_CTAS = 6;
+constexpr int TILE_ROUNDS = 24;  // more of them for 96 halos: a crowd (24 and tile_crowd for 96 take about the same)
 constexpr int TILE_MAX_SM = 4;  // block sides that have tiles
 // Cells of a tile: whole blocks of sm cells, about 8 x 16 x 32, long in z for
 // the result's rows; 32 KB of shared memory, and a halo is in 1.27 tiles on
@@ -580,6 +583,19 @@ __device__ __forceinline__ FPair fp_one_minus(float f) {  // exact for f in [0, 
   return {h, __fsub_rn(__fsub_rn(1.0f, h), f)};
 }
 
+// The weight of the corner (a, b, c) of a halo of mass weight m at the
+// fractions fx, fy, fz, by the factors of Cic (the upper ones are floats); true
+// where the pair holds
+__device__ __forceinline__ bool cic_pair(float m, float fx, float fy, float fz, int a, int b, int c, FPair* w) {
+  const float fx1 = __fsub_rn(1.0f, fx);
+  const float yp = __fsub_rn(1.0f, __fsub_rn(1.0f, fy)), zp = __fsub_rn(1.0f, __fsub_rn(1.0f, fz));
+  const FPair X = a ? FPair{__fsub_rn(1.0f, fx1), 0.f} : fp_one_minus(fx);
+  const FPair Y = b ? FPair{yp, 0.f} : fp_one_minus(a ? yp : fy);
+  const FPair Z = c ? FPair{zp, 0.f} : fp_one_minus(a || b ? zp : fz);
+  *w = fp_scale(fp_mul(fp_mul(X, Y), Z), m);
+  return fx >= 0.f && fx < 1.f && fy >= 0.f && fy < 1.f && fz >= 0.f && fz < 1.f && m >= 0x1p-50f && m < 0x1p60f;
+}
+
 // acc + the contribution of corner k of a halo, as the reference adds it
 __device__ __noinline__ float corner_exact(float acc, float4 h, int N, int k) {
   const Cic q = cic_of(h.y, h.z, h.w, N);
@@ -608,6 +624,110 @@ __device__ __noinline__ float block_exact(const float* v, int sx, int sy, int sm
   return smooth_value(rows_sum(v, sx, sy, sm), a);
 }
 
+// How many of each of a tile's runs go now (warp 0; lane = run, which stands at
+// cur[run] and ends at end): take = their numbers, summed up to each run
+__device__ __forceinline__ void tile_take(uint32_t more, uint32_t end, const uint32_t* __restrict__ idx,
+                                          const uint32_t* cur, uint32_t* take) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t b = cur[lane], n = end - b;
+  uint32_t m = n;
+  if (more > TILE_THREADS) {
+    // a share of the threads in proportion to what is left, one at least
+    // (27 runs: 69 + 27 = 96), then only what lies below the first entry
+    // that some run would keep back
+    const uint32_t share = n ? 1 + (uint32_t)((unsigned long long)n * (TILE_THREADS - 27) / more) : 0;
+    m = min(n, share);
+    const uint32_t limit = __reduce_min_sync(0xffffffffu, m < n ? idx[b + m] : 0xffffffffu);
+    uint32_t lo = 0, hi = m;
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (idx[b + mid] < limit)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    m = lo;
+  }
+  uint32_t incl = m;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  take[lane] = incl;
+}
+// The halo of this thread, one of the taken
+__device__ __forceinline__ uint32_t tile_taken(const uint32_t* __restrict__ idx, const uint32_t* cur, const uint32_t* take) {
+  int r = 0;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1)
+    if (take[r + s - 1] <= threadIdx.x) r += s;
+  return idx[cur[r] + threadIdx.x - (r ? take[r - 1] : 0)];
+}
+
+// The rest of a tile that has a crowd, many halos in a cell: the contributions
+// of 96 halos at a time are worked out by all threads, and eight lanes, one to
+// a corner, add them halo by halo in the catalogue's order.  A round of
+// k_halo_tiles adds one of a cell's contributions, and the posts to a slot are
+// served in turn: 1.3 us a round.  10^6 halos, 97 532 of them in one cell of
+// 480^3: 123 ms by rounds alone, 44 by the fine grid, 20 so.  A function of its
+// own, so that the tiles without a crowd (all of them, as a rule) keep their
+// registers.  (The cells of a halo differ: N > 1.)
+__device__ __noinline__ void tile_crowd(int N, int tx, int ty, int tz, const uint32_t* __restrict__ idx,
+                                        const float4* __restrict__ rec, int x0, int y0, int z0, uint32_t more,
+                                        uint32_t end, uint32_t* cur, uint32_t* take, uint32_t* work, float* fine) {
+  uint32_t* halo = work;                                           // [TILE_THREADS], in the catalogue's order
+  int* cells = reinterpret_cast<int*>(work + TILE_THREADS);        // [8 TILE_THREADS]: 2 cell + (the pair holds), or -1
+  float2* pairs = reinterpret_cast<float2*>(cells + 8 * TILE_THREADS);
+  const int lane = threadIdx.x & 31;
+  while (more) {
+    if (threadIdx.x < 32) tile_take(more, end, idx, cur, take);
+    __syncthreads();
+    const uint32_t taken = take[31], i = threadIdx.x < taken ? tile_taken(idx, cur, take) : ~0u;
+    cells[threadIdx.x] = (int)i;
+    __syncthreads();
+    int rank = 0;
+    for (int k = 0; k < TILE_THREADS; k++) rank += (uint32_t)cells[k] < i;
+    if (threadIdx.x < taken) halo[rank] = i;
+    __syncthreads();
+    for (int e = threadIdx.x; e < 8 * (int)taken; e += TILE_THREADS) {
+      const float4 h = rec[halo[e >> 3]];
+      const int a = e >> 2 & 1, b = e >> 1 & 1, c = e & 1;
+      float fx, fy, fz;
+      const int lx = (int)wrap_cell(cic_cell(h.y, &fx) + a, N) - x0;
+      const int ly = (int)wrap_cell(cic_cell(h.z, &fy) + b, N) - y0;
+      const int lz = (int)wrap_cell(cic_cell(h.w, &fz) + c, N) - z0;
+      const bool in = (unsigned)lx < (unsigned)tx && (unsigned)ly < (unsigned)ty && (unsigned)lz < (unsigned)tz;
+      FPair w;
+      const bool plain = cic_pair(h.x, fx, fy, fz, a, b, c, &w);
+      cells[e] = in ? 2 * ((lx * ty + ly) * tz + lz) + plain : -1;
+      pairs[e] = make_float2(w.hi, w.lo);
+    }
+    __syncthreads();
+    if (threadIdx.x < 8) {
+      int c = cells[threadIdx.x];
+      float2 w = pairs[threadIdx.x];
+      for (int r = 0; r < (int)taken; r++) {
+        const int c1 = c, e = 8 * min(r + 1, (int)taken - 1) + threadIdx.x;
+        const FPair w1 = {w.x, w.y};
+        c = cells[e];
+        w = pairs[e];
+        if (c1 >= 0) {
+          const FPair v = fp_add(w1, fine[c1 >> 1]);
+          if ((c1 & 1) && fp_sure(v))
+            fine[c1 >> 1] = v.hi;
+          else if (!(c1 & 1) || w1.hi != 0.0f)
+            fine[c1 >> 1] = corner_exact(fine[c1 >> 1], rec[halo[r]], N, threadIdx.x);
+        }
+        __syncwarp(0xffu);
+      }
+    }
+    if (threadIdx.x < 32) cur[lane] += take[lane] - (lane ? take[lane - 1] : 0);
+    more -= taken;
+    __syncthreads();
+  }
+}
+
 template <int SM>
 __global__ void __launch_bounds__(TILE_THREADS, TILE_CTAS)
 k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __restrict__ idx,
@@ -615,6 +735,8 @@ k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __
   extern __shared__ __align__(16) float tile_fine[];
   __shared__ uint32_t cur[32], take[32];
   __shared__ uint32_t left;  // halos that have not been taken
+  __shared__ int rounds;     // of the batch
+  __shared__ bool crowd;
   constexpr int TX = tile_x(SM), TY = tile_y(SM), TZ = tile_z(SM);
   constexpr int cells = (TX * TY * TZ + 3) & ~3;  // whole float4
   uint32_t* slot = reinterpret_cast<uint32_t*>(tile_fine + cells);
@@ -638,7 +760,7 @@ k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __
     }
     cur[lane] = b;
     const uint32_t n = __reduce_add_sync(0xffffffffu, end - b);
-    if (lane == 0) left = n;
+    if (lane == 0) left = n, rounds = 0;
   }
   __syncthreads();
   uint32_t more = left;
@@ -649,34 +771,7 @@ k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __
       *reinterpret_cast<uint4*>(slot + k) = make_uint4(~0u, ~0u, ~0u, ~0u);
     }
   while (more) {
-    if (threadIdx.x < 32) {  // how many of each run now
-      const uint32_t b = cur[lane], n = end - b;
-      uint32_t m = n;
-      if (more > TILE_THREADS) {
-        // a share of the threads in proportion to what is left, one at least
-        // (27 runs: 69 + 27 = 96), then only what lies below the first entry
-        // that some run would keep back
-        const uint32_t share = n ? 1 + (uint32_t)((unsigned long long)n * (TILE_THREADS - 27) / more) : 0;
-        m = min(n, share);
-        const uint32_t limit = __reduce_min_sync(0xffffffffu, m < n ? idx[b + m] : 0xffffffffu);
-        uint32_t lo = 0, hi = m;
-        while (lo < hi) {
-          const uint32_t mid = (lo + hi) >> 1;
-          if (idx[b + mid] < limit)
-            lo = mid + 1;
-          else
-            hi = mid;
-        }
-        m = lo;
-      }
-      uint32_t incl = m;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-      }
-      take[lane] = incl;
-    }
+    if (threadIdx.x < 32) tile_take(more, end, idx, cur, take);
     __syncthreads();
     const uint32_t taken = take[31];
     uint32_t wait = 0;  // bit k = 4 a + 2 b + c: that corner's contribution waits
@@ -687,11 +782,7 @@ k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __
     FPair w[8];
     bool plain = false;  // the pairs hold
     if (threadIdx.x < taken) {
-      int r = 0;
-#pragma unroll
-      for (int s = 16; s > 0; s >>= 1)
-        if (take[r + s - 1] <= threadIdx.x) r += s;
-      const uint32_t i = idx[cur[r] + threadIdx.x - (r ? take[r - 1] : 0)];
+      const uint32_t i = tile_taken(idx, cur, take);
       h = rec[i];
       order = 8 * i;
       float fx, fy, fz;
@@ -723,6 +814,7 @@ k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __
       }
     }
     do {
+      if (threadIdx.x == 0) rounds++;
       if (wait) {
 #pragma unroll
         for (int k = 0; k < 8; k++)
@@ -754,10 +846,18 @@ k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __
     } while (__syncthreads_or(wait != 0));
     if (threadIdx.x < 32) {
       cur[lane] += take[lane] - (lane ? take[lane - 1] : 0);
-      if (lane == 0) left = more - taken;
+      if (lane == 0) {
+        left = more - taken;
+        crowd = rounds > TILE_ROUNDS;
+        rounds = 0;
+      }
     }
     __syncthreads();
     more = left;
+    if (crowd && more && t.N > 1) {
+      tile_crowd(t.N, TX, TY, TZ, idx, rec, x0, y0, z0, more, end, cur, take, slot, tile_fine);
+      break;
+    }
   }
   // Blocks without a contribution first (most of them, at a halo per hundred
   // cells); the others into a list, so that whole warps work on them
