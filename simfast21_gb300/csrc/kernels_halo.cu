@@ -951,11 +951,20 @@ k_halo_tiles(HaloTiles t, const uint32_t* __restrict__ start, const uint32_t* __
 // fine 1.27, 1.49, 2.83, tiles 4.2, 7.6, 18.9).
 //
 // Where the tiles are fewer than two an SM (up to about 100^3 cells), they wait
-// for the rounds of their halos, and from 70 sm halos a tile the sort of the
-// contributions is done first:
-//   48^3, side 1   0.01 per cell: fine 0.11, tiles 0.08;  0.1: 0.17, 0.22;  1: 0.27, 0.73
-//   72^3, side 3   0.02:          0.18, 0.15;             0.1: 0.20, 0.21;  2: 1.13, 1.28
-//   108^3, side 1  0.02:          0.19, 0.18;             0.1: 0.25, 0.25;  2: 3.30, 1.62
+// for the rounds of their halos, and many halos a tile go faster through the
+// sort of the contributions, the sooner the fewer the tiles are (us a call among
+// others, by halos a tile):
+//   48^3, side 1, 36 tiles    140: fine 65, tiles 65;  250: 66, 75
+//   64^3, side 1, 64 tiles    140: 67, 64;  200: 68, 70;  300: 70, 77
+//   96^3, side 1, 216 tiles   140: 78, 69;  250: 85, 81
+//   64^3, side 2, 64 tiles    150: 66, 62;  250: 69, 70
+//   72^3, side 3, 120 tiles   250: 77, 73
+//   96^3, side 4, 216 tiles   350: 98, 82
+// so the line lies at 95 halos a tile and one more for every tile, half as much
+// again for sides above 1 (less to average and store).  Up to 2000 halos the
+// tiles are ahead in any case: eight contributions a halo are long enough for
+// the larger form of the sort then, the halos are not (32^3, 8 tiles, 200 a
+// tile: 40, 35).
 // Grids beyond 2048 keep the fine grid.
 static bool has_tiles(long N_halo, long N_smooth) {
   const long sm = block_side(N_halo, N_smooth);
@@ -968,7 +977,7 @@ static bool few_tiles(long N_halo, long N_smooth) {
 static bool by_tiles(long nh, long N_halo, long N_smooth) {
   if (!has_tiles(N_halo, N_smooth)) return false;
   const long sm = block_side(N_halo, N_smooth), tiles = halo_tiles(N_halo, sm).keys() / 8;
-  return tiles >= FEW_TILES || nh < 70 * sm * tiles;
+  return tiles >= FEW_TILES || nh < 2000 || 2 * nh < (sm > 1 ? 3 : 2) * (95 + tiles) * tiles;
 }
 bool halo_needs_grid(long N_halo, long N_smooth) {
   return !has_tiles(N_halo, N_smooth) || few_tiles(N_halo, N_smooth);
