@@ -10,7 +10,7 @@
 //     power = re^2 + im^2 in float as the tool computes it; per-CTA sums in
 //     shared memory, written out per CTA, counts added exactly with integer
 //     atomics;
-//   k_pk_reduce: adds the CTAs' sums in double (softdouble.h), so a few
+//   k_pk_reduce: adds the CTAs' sums exactly, in integers, so a few
 //     kilobytes go to the host instead of the 14.6 MB of partial sums at 512^3,
 //     which took most of the call there.
 #include <cuda_runtime.h>
@@ -83,35 +83,84 @@ k_pk_bin(int N, const float2* __restrict__ spec, int nk, float* __restrict__ par
   }
 }
 
-// partials: [ncta][nk], not negative; sums[b]: the double sum of bin b's, in
-// the integer routines of softdouble.h, as bits.  A sum with an infinity is
-// infinite, one with a NaN is NaN (those routines take finite operands only).
-// threadIdx.x = bin of the CTA's PKR_BINS, the threadIdx.y rows share the CTAs:
-// a sum of doubles in integers is a chain of 60 instructions, so a bin has 512
-// of them side by side (512^3, 8192 partial sums a bin: 24 us; 60 with 128).
-constexpr int PKR_BINS = 2, PKR_ROWS = 512;
-__global__ void __launch_bounds__(PKR_BINS * PKR_ROWS)
-k_pk_reduce(int ncta, int nk, const float* __restrict__ partials, sd_t* __restrict__ sums) {
-  __shared__ sd_t sm[PKR_ROWS][PKR_BINS + 1];
-  const int b = blockIdx.x * PKR_BINS + threadIdx.x;
-  __shared__ int inf[PKR_BINS], nan[PKR_BINS];
-  if (threadIdx.y == 0) inf[threadIdx.x] = nan[threadIdx.x] = 0;
-  __syncthreads();
-  sd_t s = 0;
-  if (b < nk)
-    for (int g = threadIdx.y; g < ncta; g += PKR_ROWS) {
-      const float v = partials[(long)g * nk + b];
-      if (isfinite(v)) s = sd_add(s, sd_from_float(v));
-      else (isnan(v) ? nan : inf)[threadIdx.x] = 1;
-    }
-  sm[threadIdx.y][threadIdx.x] = s;
-  __syncthreads();
-  for (int o = PKR_ROWS / 2; o > 0; o >>= 1) {
-    if (threadIdx.y < o) sm[threadIdx.y][threadIdx.x] = sd_add(sm[threadIdx.y][threadIdx.x], sm[threadIdx.y + o][threadIdx.x]);
-    __syncthreads();
+// partials: [ncta][nk], not negative; sums[b]: bin b's sum, rounded to double
+// once, as bits.  Terms are 128-bit integers in units of 2^-103 of the largest
+// one's exponent (2^16 CTAs at most: 120 bits), which a first pass over the
+// partials finds: sums of integers are two instructions a term and shuffles
+// after that.  (Chains and a tree of soft doubles made a call 6 us longer at
+// 64^3, 128 partial sums a bin, 73 us for 67, and 12 at 512^3, 8192 a bin.)  A
+// sum with an infinity is infinite, one with a NaN is NaN.
+// threadIdx.x = bin of the CTA's PKR_BINS, the threadIdx.y rows share the CTAs.
+constexpr int PKR_BINS = 4, PKR_ROWS = 256, PKR_WARPS = PKR_BINS * PKR_ROWS / 32;
+static_assert(PKR_WARPS == 32, "the last step is one warp, four sums to a lane");
+
+__device__ __forceinline__ sd_u128 pk_lanes(sd_u128 v) {  // over the warp's lanes of one bin
+#pragma unroll
+  for (int o = PKR_BINS; o < 32; o <<= 1)
+    v += (sd_u128)__shfl_xor_sync(0xffffffffu, (unsigned long long)(v >> 64), o) << 64 |
+         __shfl_xor_sync(0xffffffffu, (unsigned long long)v, o);
+  return v;
+}
+
+// v 2^e as a double's bits, to nearest even (its exponent is a normal one)
+__device__ __forceinline__ uint64_t pk_double(sd_u128 v, int e) {
+  if (!v) return 0;
+  const uint64_t hi = (uint64_t)(v >> 64);
+  const int top = hi ? 127 - __clzll((long long)hi) : 63 - __clzll((long long)(uint64_t)v);
+  uint64_t q;
+  if (top <= 52) {
+    q = (uint64_t)v << (52 - top);
+  } else {
+    const int s = top - 52;
+    const sd_u128 rem = v & (((sd_u128)1 << s) - 1), half = (sd_u128)1 << (s - 1);
+    q = (uint64_t)(v >> s);
+    q += rem > half || (rem == half && (q & 1));
   }
-  if (threadIdx.y == 0 && b < nk)
-    sums[b] = nan[threadIdx.x] ? SD_QNAN : inf[threadIdx.x] ? 0x7FF0000000000000ULL : sm[0][threadIdx.x];
+  return ((uint64_t)(top + e + 1022) << 52) + q;  // q has bit 52 (or is 2^53: the next exponent)
+}
+
+__global__ void __launch_bounds__(PKR_BINS * PKR_ROWS)
+k_pk_reduce(int ncta, int nk, const float* __restrict__ partials, uint64_t* __restrict__ sums) {
+  __shared__ uint32_t most[PKR_BINS];
+  __shared__ unsigned long long part[PKR_WARPS][PKR_BINS][2];
+  const int x = threadIdx.x, b = blockIdx.x * PKR_BINS + x, tid = threadIdx.y * PKR_BINS + x;
+  const int lane = tid & 31, w = tid >> 5;
+  if (tid < PKR_BINS) most[tid] = 0;
+  __syncthreads();
+  const int g0 = b < nk ? threadIdx.y : ncta;
+  uint32_t m = 0;  // of the bits: floats that are not negative are in their order, infinity and NaNs above them
+#pragma unroll 8
+  for (int g = g0; g < ncta; g += PKR_ROWS) m = max(m, __float_as_uint(partials[(long)g * nk + b]) & 0x7FFFFFFFu);
+#pragma unroll
+  for (int o = PKR_BINS; o < 32; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (lane < PKR_BINS) atomicMax(&most[x], m);
+  __syncthreads();
+  m = most[x];
+  const int E = max((int)(m >> 23), 1);
+  sd_u128 s = 0;
+  if (m < 0x7F800000u) {
+#pragma unroll 8
+    for (int g = g0; g < ncta; g += PKR_ROWS) {
+      const uint32_t u = __float_as_uint(partials[(long)g * nk + b]) & 0x7FFFFFFFu;
+      const int e = max((int)(u >> 23), 1);
+      const uint32_t f = (u & 0x7FFFFFu) | (u >> 23 ? 0x800000u : 0u);  // value f 2^(e - 150)
+      s += (sd_u128)f << 80 >> min(E - e, 127);
+    }
+  }
+  s = pk_lanes(s);
+  if (lane < PKR_BINS) {
+    part[w][x][0] = (unsigned long long)(s >> 64);
+    part[w][x][1] = (unsigned long long)s;
+  }
+  __syncthreads();
+  if (w == 0) {
+    s = 0;
+#pragma unroll
+    for (int k = lane / PKR_BINS; k < PKR_WARPS; k += 32 / PKR_BINS) s += (sd_u128)part[k][x][0] << 64 | part[k][x][1];
+    s = pk_lanes(s);
+    if (lane < PKR_BINS && b < nk)
+      sums[b] = m > 0x7F800000u ? SD_QNAN : m == 0x7F800000u ? 0x7FF0000000000000ULL : pk_double(s, E - 230);
+  }
 }
 
 cudaError_t launch_pk_reduce(int N, int nk, const float* partials, uint64_t* sums, cudaStream_t st) {

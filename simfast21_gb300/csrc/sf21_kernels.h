@@ -209,7 +209,7 @@ int pk_bin_grid(int N);
 cudaError_t launch_pk_pack(int N, const float* box, const float* wax, float2* out, cudaStream_t st);
 cudaError_t launch_pk_bin(int N, const float2* spec, int nk, float* partials, unsigned long long* counts,
                           cudaStream_t st);
-// sums[b] = bits of the double sum of the CTAs' sums of bin b
+// sums[b] = bits of the CTAs' sums of bin b, added and rounded to double
 cudaError_t launch_pk_reduce(int N, int nk, const float* partials, uint64_t* sums, cudaStream_t st);
 
 // 21-cm brightness temperature (kernels_t21.cu).
